@@ -1488,12 +1488,11 @@ int inqb_orthonormalize(inqb_ctx* ctx, void* psi, int M, int ld, void* stream) {
   INQB_CHECK_CTX(ctx);
   INQB_TRY(check_block(ctx, psi, M, ld));
   INQB_GUARD(ctx);
-  DevBuf S, X, info;
-  INQB_TRY(S.ensure(sizeof(double2) * (size_t)M * M));
-  INQB_TRY(X.ensure(sizeof(double2) * (size_t)M * M));
-  INQB_TRY(info.ensure(sizeof(int)));
-  return launch_orthonormalize(ctx->precision, psi, ld, M, ctx->N, ctx->dV, S.as<double2>(), X.as<double2>(),
-                               info.as<int>(), stream);
+  const size_t MM = (size_t)M * M;
+  INQB_TRY(ctx->d_orth.ensure(sizeof(double2) * (2 * MM + 1)));
+  double2* S = ctx->d_orth.as<double2>();
+  return launch_orthonormalize(ctx->precision, psi, ld, M, ctx->N, ctx->dV, S, S + MM,
+                               reinterpret_cast<int*>(S + 2 * MM), stream);
 }
 
 int inqb_overlap_block(inqb_ctx* ctx, const void* a, int Ma, int lda, const void* b, int Mb, int ldb, double* S,
@@ -1512,10 +1511,10 @@ int inqb_cholesky_inverse(inqb_ctx* ctx, double* S, int M, int lds, void* stream
   if (!S || M <= 0 || lds < M) return fail(INQB_ERR_INVALID, "cholesky inverse: need S, M > 0 and lds >= M");
   if (((uintptr_t)S) % 16 != 0) return fail(INQB_ERR_INVALID, "cholesky inverse: S must be 16-byte aligned");
   INQB_GUARD(ctx);
-  DevBuf X, info;
-  INQB_TRY(X.ensure(sizeof(double2) * (size_t)M * M));
-  INQB_TRY(info.ensure(sizeof(int)));
-  return launch_cholesky_inverse(reinterpret_cast<double2*>(S), M, lds, X.as<double2>(), info.as<int>(), stream);
+  const size_t MM = (size_t)M * M;
+  INQB_TRY(ctx->d_orth.ensure(sizeof(double2) * (MM + 1)));
+  double2* X = ctx->d_orth.as<double2>();
+  return launch_cholesky_inverse(reinterpret_cast<double2*>(S), M, lds, X, reinterpret_cast<int*>(X + MM), stream);
 }
 
 int inqb_rotate_block(inqb_ctx* ctx, const void* a, int Ma, int lda, const double* R, int ldr, int Mo, void* out,

@@ -1,7 +1,7 @@
 // Observables and FP64 orbital linear algebra on the device:
 //   density   rho[p] = sum_m occ[m] |psi[p][m]|^2       (src/observables/density.hpp:23-33)
 //   dipole    dV sum_p r_p rho[p]                         (src/observables/dipole.hpp:23-40)
-//   overlap   S = dV psi^H psi, FP64 accumulation         (src/operations/overlap.hpp:41)
+//   overlap   S = dV psi^H psi, FP64 arithmetic            (src/operations/overlap.hpp:41)
 //   cholesky  S = U^H U, U upper                          (src/matrix/cholesky.hpp:28-89)
 //   rotate    psi <- psi U^-1                             (src/operations/rotate.hpp:147-157)
 // Input orbitals may be complex64 (mixed) or complex128; every sum is FP64.
@@ -77,152 +77,382 @@ __global__ void k_dipole(const double* __restrict__ rho, long N, LatticeView g, 
   }
 }
 
-// S[i][j] += dV sum_{p in chunk} conj(a[p][i]) b[p][j] ; 32x32 tile per CTA.  The
-// square overlap passes the same block twice; an orbital-sharded caller passes two
-// blocks (one block of operations::overlap's set-parallel branch).
-template <typename T>
-__global__ void __launch_bounds__(1024) k_overlap(const cplx<T>* __restrict__ pa, long lda, int Ma,
-                                                  const cplx<T>* __restrict__ pb_, long ldb, int Mb, long N,
-                                                  long chunk, double dV, double2* __restrict__ S, long lds) {
-  constexpr int TP = 32;  // points staged per round
-  __shared__ double2 a[TP][33], b[TP][33];
-  const int ti = threadIdx.y, tj = threadIdx.x;
-  const int i0 = blockIdx.y * 32, j0 = blockIdx.x * 32;
-  const long p0 = (long)blockIdx.z * chunk, p1 = min(N, p0 + chunk);
-  double re = 0.0, im = 0.0;
-  for (long pb = p0; pb < p1; pb += TP) {
-    // thread (ti, tj) loads point pb+ti, orbital i0+tj of a / j0+tj of b
-    const long p = pb + ti;
-    double2 va = make_double2(0, 0), vb = make_double2(0, 0);
-    if (p < p1) {
-      if (i0 + tj < Ma) {
-        cplx<T> v = pa[p * lda + i0 + tj];
-        va = make_double2(v.x, v.y);
-      }
-      if (j0 + tj < Mb) {
-        cplx<T> v = pb_[p * ldb + j0 + tj];
-        vb = make_double2(v.x, v.y);
-      }
+// ---------------------------------------------------------------- overlap
+// 256 threads as a 16 x 16 grid, a warp 4 x 8 of it: a warp's 16-byte shared loads then
+// touch 64 bytes of the row operand and 128 of the column operand, one wavefront each (as
+// 2 x 16 the column operand took two or more, and the loads bound the kernel at 59% of the
+// FP64 rate).
+__device__ __forceinline__ int grid_row() { return (threadIdx.x / 32) % 4 * 4 + threadIdx.x % 32 / 8; }
+__device__ __forceinline__ int grid_col() { return threadIdx.x / 128 * 8 + threadIdx.x % 8; }
+
+// S[i][j] += dV sum_{p in slab} conj(a[p][i]) b[p][j], FP64 products and sums.  256
+// threads as 16 x 16, TM x TM outputs a thread (outputs ti + 16 a, tj + 16 b), so a CTA
+// holds a (16 TM)^2 tile in registers over its slab of points; KP points are staged at a
+// time, the next ones fetched into registers meanwhile.  The pass is bound by the FP64
+// units: a thread's TM^2 complex products take 4 TM^2 DFMA for 2 TM 16-byte shared loads.
+// The square overlap (upper) computes the tiles on and above the diagonal only, which is
+// all the Cholesky factorisation reads.
+template <int TM>
+struct OverlapCfg {
+  static constexpr int KP = TM == 4 ? 8 : TM == 2 ? 16 : 32;
+  static constexpr int CTAS = TM == 4 ? 2 : 4;  // per SM
+};
+
+template <typename T, int TM>
+__global__ void __launch_bounds__(256, OverlapCfg<TM>::CTAS)
+    k_overlap(const cplx<T>* __restrict__ pa, long lda, int Ma, const cplx<T>* __restrict__ pb, long ldb, int Mb,
+              long N, long slab, double dV, double2* __restrict__ S, long lds, int upper) {
+  constexpr int TILE = 16 * TM, KP = OverlapCfg<TM>::KP, PER = TILE * KP / 256;
+  __shared__ double2 sa[KP][TILE], sb[KP][TILE];
+  const int tiles_j = (Mb + TILE - 1) / TILE;
+  int bi, bj;
+  if (upper) {  // tile blockIdx.x of the rows (0, 0..), (1, 1..), ...
+    int t = blockIdx.x;
+    bi = 0;
+    while (t >= tiles_j - bi) t -= tiles_j - bi++;
+    bj = bi + t;
+  } else {
+    bi = blockIdx.x / tiles_j;
+    bj = blockIdx.x % tiles_j;
+  }
+  const int i0 = bi * TILE, j0 = bj * TILE;
+  const bool diag = upper && bi == bj;  // one block serves both sides
+  const int ti = grid_row(), tj = grid_col();
+  const long p0 = (long)blockIdx.y * slab, p1 = min(N, p0 + slab);
+  double re[TM][TM], im[TM][TM];
+#pragma unroll
+  for (int a = 0; a < TM; ++a)
+#pragma unroll
+    for (int b = 0; b < TM; ++b) re[a][b] = im[a][b] = 0.0;
+  cplx<T> va[PER], vb[PER];
+  auto fetch = [&](long pc) {
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int e = threadIdx.x + 256 * u, q = e / TILE, j = e % TILE;
+      const long p = pc + q;
+      va[u] = (p < p1 && i0 + j < Ma) ? pa[p * lda + i0 + j] : mk<T>(0, 0);
+      if (!diag) vb[u] = (p < p1 && j0 + j < Mb) ? pb[p * ldb + j0 + j] : mk<T>(0, 0);
     }
-    a[ti][tj] = va;
-    b[ti][tj] = vb;
+  };
+  fetch(p0);
+  const double2(*sbv)[TILE] = diag ? sa : sb;
+  for (long pc = p0; pc < p1; pc += KP) {
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int e = threadIdx.x + 256 * u, q = e / TILE, j = e % TILE;
+      sa[q][j] = make_double2(va[u].x, va[u].y);
+      if (!diag) sb[q][j] = make_double2(vb[u].x, vb[u].y);
+    }
     __syncthreads();
-#pragma unroll 8
-    for (int q = 0; q < TP; q++) {
-      const double2 x = a[q][ti], y = b[q][tj];
-      re += x.x * y.x + x.y * y.y;
-      im += x.x * y.y - x.y * y.x;
+    if (pc + KP < p1) fetch(pc + KP);
+#pragma unroll 4
+    for (int q = 0; q < KP; ++q) {
+      double2 x[TM], y[TM];
+#pragma unroll
+      for (int a = 0; a < TM; ++a) x[a] = sa[q][ti + 16 * a];
+#pragma unroll
+      for (int b = 0; b < TM; ++b) y[b] = sbv[q][tj + 16 * b];
+      // a tile on the diagonal needs its 16-wide blocks a <= b only
+#pragma unroll
+      for (int a = 0; a < TM; ++a)
+#pragma unroll
+        for (int b = 0; b < TM; ++b) {
+          if (a > b && diag) continue;
+          re[a][b] = fma(x[a].x, y[b].x, fma(x[a].y, y[b].y, re[a][b]));
+          im[a][b] = fma(x[a].x, y[b].y, fma(-x[a].y, y[b].x, im[a][b]));
+        }
     }
     __syncthreads();
   }
-  if (i0 + ti < Ma && j0 + tj < Mb) {
-    atomicAdd(&S[(long)(i0 + ti) * lds + j0 + tj].x, dV * re);
-    atomicAdd(&S[(long)(i0 + ti) * lds + j0 + tj].y, dV * im);
+#pragma unroll
+  for (int a = 0; a < TM; ++a)
+#pragma unroll
+    for (int b = 0; b < TM; ++b) {
+      const int i = i0 + ti + 16 * a, j = j0 + tj + 16 * b;
+      if (i < Ma && j < Mb && !(upper && i > j)) {
+        atomicAdd(&S[(long)i * lds + j].x, dV * re[a][b]);
+        atomicAdd(&S[(long)i * lds + j].y, dV * im[a][b]);
+      }
+    }
+}
+
+// ---------------------------------------------------------------- Cholesky factor and its inverse
+// S = U^H U by blocks of kNB, one launch per block row: launch k (k = -1 first) finishes
+// block row k and updates the trailing blocks, and the CTA of the next diagonal block also
+// factors it, so the serial part (32 pivots in shared memory) runs inside the same launch.
+//   S[k][k] holds W_k = U_kk^-1 after its factorisation, U[k][j] (in X) = W_k^H S[k][j];
+//   trailing S[i][j] -= U[k][i]^H U[k][j], each CTA forming both panels itself.
+// The factorisation leaves a pivot row unscaled until the end (D[i][j] -= conj(D[k][i])
+// D[k][j] / d_k reads the row as it is), so a pivot costs one barrier.
+constexpr int kNB = 32;
+
+// thread (r, c0): row r = tid / 8, columns c0 + 8 m for m < 4, c0 = tid % 8
+struct Quad {
+  double2 v[4];
+};
+__device__ __forceinline__ Quad quad_zero() {
+  Quad q;
+#pragma unroll
+  for (int m = 0; m < 4; ++m) q.v[m] = make_double2(0.0, 0.0);
+  return q;
+}
+__device__ __forceinline__ void quad_store(double2 (*d)[kNB], const Quad& q) {
+  const int r = threadIdx.x / 8, c0 = threadIdx.x % 8;
+#pragma unroll
+  for (int m = 0; m < 4; ++m) d[r][c0 + 8 * m] = q.v[m];
+}
+// block (bi, bj) of an M x M matrix; outside the matrix: the identity (one) or zero
+__device__ __forceinline__ Quad quad_load(const double2* A, long lda, int M, int bi, int bj, bool one) {
+  const int r = threadIdx.x / 8, c0 = threadIdx.x % 8;
+  Quad q;
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const int i = bi * kNB + r, j = bj * kNB + c0 + 8 * m;
+    q.v[m] = (i < M && j < M) ? A[(long)i * lda + j] : make_double2(one && i == j ? 1.0 : 0.0, 0.0);
+  }
+  return q;
+}
+__device__ __forceinline__ void quad_write(double2* A, long lda, int M, int bi, int bj, const Quad& q) {
+  const int r = threadIdx.x / 8, c0 = threadIdx.x % 8;
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const int i = bi * kNB + r, j = bj * kNB + c0 + 8 * m;
+    if (i < M && j < M) A[(long)i * lda + j] = q.v[m];
+  }
+}
+// acc += s A^H B (ADJ) or s A B of two blocks in shared memory
+template <bool ADJ>
+__device__ __forceinline__ void quad_mul(Quad& acc, double s, const double2 (*A)[kNB], const double2 (*B)[kNB]) {
+  const int r = threadIdx.x / 8, c0 = threadIdx.x % 8;
+#pragma unroll 4
+  for (int q = 0; q < kNB; ++q) {
+    double2 a = ADJ ? A[q][r] : A[r][q];
+    a = make_double2(s * a.x, ADJ ? -s * a.y : s * a.y);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const double2 b = B[q][c0 + 8 * m];
+      acc.v[m].x = fma(a.x, b.x, fma(-a.y, b.y, acc.v[m].x));
+      acc.v[m].y = fma(a.x, b.y, fma(a.y, b.x, acc.v[m].y));
+    }
   }
 }
 
-// In-place Cholesky of the Hermitian S (upper triangle used): on exit the upper
-// triangle holds U with S = U^H U.  One CTA; info[0] = first failing pivot + 1.
-__global__ void __launch_bounds__(1024) k_cholesky(double2* __restrict__ S, int M, long lds, int* __restrict__ info) {
-  __shared__ int bad;
-  if (threadIdx.x == 0) bad = 0;
-  __syncthreads();
-  for (int k = 0; k < M; k++) {
-    __syncthreads();
-    const double d = S[(long)k * lds + k].x;
+// Factor the block in D (upper triangle) and write U_kk to U, W_k = U_kk^-1 (zero below
+// the diagonal) to S; info gets the first failing pivot + 1.  W is scratch.
+__device__ void chol_diag(double2 (*D)[kNB], double2 (*W)[kNB], double2* S, long lds, double2* U, int M, int k,
+                          int* info) {
+  const int r = threadIdx.x / 8, c0 = threadIdx.x % 8;
+  const int first = *info;  // a failed pivot of an earlier block stays the first
+  for (int p = 0; p < kNB; ++p) {
+    const double d = D[p][p].x;
     if (!(d > 0.0)) {
-      if (threadIdx.x == 0) {
-        bad = 1;
-        info[0] = k + 1;
-      }
-      __syncthreads();
+      if (threadIdx.x == 0 && first == 0) *info = k * kNB + p + 1;
       return;
     }
-    const double u = sqrt(d);
-    __syncthreads();
-    for (int j = k + threadIdx.x; j < M; j += blockDim.x) {
-      double2 v = S[(long)k * lds + j];
-      S[(long)k * lds + j] = j == k ? make_double2(u, 0.0) : make_double2(v.x / u, v.y / u);
-    }
-    __syncthreads();
-    // trailing update: S[i][j] -= conj(U[k][i]) U[k][j], k < i <= j
-    const int n = M - k - 1;
-    for (long t = threadIdx.x; t < (long)n * n; t += blockDim.x) {
-      const int i = k + 1 + (int)(t / n), j = k + 1 + (int)(t % n);
-      if (j < i) continue;
-      const double2 ui = S[(long)k * lds + i], uj = S[(long)k * lds + j];
-      double2 s = S[(long)i * lds + j];
-      s.x -= ui.x * uj.x + ui.y * uj.y;
-      s.y -= ui.x * uj.y - ui.y * uj.x;
-      S[(long)i * lds + j] = s;
-    }
-  }
-  (void)bad;
-}
-
-// X = U^-1 (upper triangular), one thread per column j, back substitution.
-__global__ void k_triangular_inverse(const double2* __restrict__ U, int M, long ldu, double2* __restrict__ X) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= M) return;
-  for (int i = 0; i < M; i++) X[(long)i * M + j] = make_double2(0, 0);
-  for (int i = j; i >= 0; i--) {
-    double2 s = make_double2(i == j ? 1.0 : 0.0, 0.0);
-    for (int k = i + 1; k <= j; k++) {
-      const double2 u = U[(long)i * ldu + k], x = X[(long)k * M + j];
-      s.x -= u.x * x.x - u.y * x.y;
-      s.y -= u.x * x.y + u.y * x.x;
-    }
-    const double uii = U[(long)i * ldu + i].x;
-    X[(long)i * M + j] = make_double2(s.x / uii, s.y / uii);
-  }
-}
-
-// psi[p][:] <- psi[p][:] X  (X upper triangular), FP64 arithmetic, in place.
-template <typename T>
-__global__ void k_rotate_upper(cplx<T>* __restrict__ psi, long ld, int M, long N, const double2* __restrict__ X) {
-  extern __shared__ double2 row[];
-  for (long p = blockIdx.x; p < N; p += gridDim.x) {
-    __syncthreads();
-    for (int m = threadIdx.x; m < M; m += blockDim.x) {
-      const cplx<T> v = psi[p * ld + m];
-      row[m] = make_double2(v.x, v.y);
-    }
-    __syncthreads();
-    for (int j = threadIdx.x; j < M; j += blockDim.x) {
-      double re = 0.0, im = 0.0;
-      for (int i = 0; i <= j; i++) {
-        const double2 a = row[i], x = X[(long)i * M + j];
-        re += a.x * x.x - a.y * x.y;
-        im += a.x * x.y + a.y * x.x;
+    if (r > p) {
+      const double2 x = D[p][r];
+      const double2 f = make_double2(x.x / d, -x.y / d);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const int c = c0 + 8 * m;
+        if (c < r) continue;
+        const double2 y = D[p][c];
+        D[r][c].x -= f.x * y.x - f.y * y.y;
+        D[r][c].y -= f.x * y.y + f.y * y.x;
       }
-      psi[p * ld + j] = mk<T>((T)re, (T)im);
     }
+    __syncthreads();
+  }
+  // U[r][c] = D[r][c] / sqrt(d_r); W starts as the identity
+  const double d = D[r][r].x, u = sqrt(d);
+  Quad q;
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const int c = c0 + 8 * m;
+    const double2 y = D[r][c];
+    q.v[m] = c > r ? make_double2(y.x / u, y.y / u) : make_double2(c == r ? u : 0.0, 0.0);
+    W[r][c] = make_double2(c == r ? 1.0 : 0.0, 0.0);
+  }
+  __syncthreads();
+  quad_store(D, q);
+  quad_write(U, M, M, k, k, q);
+  __syncthreads();
+  // rows from the last up: W[q] / U[q][q] is final, then W[r] -= U[r][q] W[q] / U[q][q]
+  for (int p = kNB - 1; p > 0; --p) {
+    if (r < p) {
+      const double inv = 1.0 / D[p][p].x;
+      const double2 f = make_double2(D[r][p].x * inv, D[r][p].y * inv);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const int c = c0 + 8 * m;
+        if (c < p) continue;
+        const double2 y = W[p][c];
+        W[r][c].x -= f.x * y.x - f.y * y.y;
+        W[r][c].y -= f.x * y.y + f.y * y.x;
+      }
+    }
+    __syncthreads();
+  }
+  const double inv = 1.0 / D[r][r].x;
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const double2 y = W[r][c0 + 8 * m];
+    q.v[m] = make_double2(y.x * inv, y.y * inv);
+  }
+  quad_write(S, lds, M, k, k, q);
+}
+
+__global__ void __launch_bounds__(256)
+    k_chol_step(double2* S, long lds, double2* U, int M, int k, int* info) {
+  __shared__ double2 A[kNB][kNB], B[kNB][kNB], W[kNB][kNB];
+  if (k < 0) {
+    quad_store(A, quad_load(S, lds, M, 0, 0, true));
+    __syncthreads();
+    chol_diag(A, W, S, lds, U, M, 0, info);
+    return;
+  }
+  const int nb = (M + kNB - 1) / kNB;
+  int t = blockIdx.x, i = k + 1;
+  while (t >= nb - i) t -= nb - i++;
+  const int j = i + t;
+  // panels U[k][i], U[k][j] = W_k^H S[k][i], W_k^H S[k][j]
+  quad_store(W, quad_load(S, lds, M, k, k, false));
+  quad_store(A, quad_load(S, lds, M, k, i, false));
+  quad_store(B, quad_load(S, lds, M, k, j, false));
+  __syncthreads();
+  Quad pi = quad_zero(), pj = quad_zero();
+  quad_mul<true>(pi, 1.0, W, A);
+  if (i != j) quad_mul<true>(pj, 1.0, W, B);
+  __syncthreads();
+  if (i == j) {
+    pj = pi;
+    quad_write(U, M, M, k, j, pj);
+  }
+  quad_store(A, pi);
+  quad_store(B, pj);
+  __syncthreads();
+  Quad s = quad_load(S, lds, M, i, j, i == j);
+  quad_mul<true>(s, -1.0, A, B);
+  if (i == k + 1 && j == k + 1) {
+    __syncthreads();
+    quad_store(A, s);
+    __syncthreads();
+    chol_diag(A, W, S, lds, U, M, i, info);
+  } else {
+    quad_write(S, lds, M, i, j, s);
   }
 }
 
-// out[p][j] = sum_{i < Ma} a[p][i] R[i][j], j < Mo: one block of operations::rotate's
-// set-parallel branch (src/operations/rotate.hpp:100-125), FP64 arithmetic, a row of a
-// staged in shared memory per point.
-template <typename T>
-__global__ void k_rotate_block(const cplx<T>* __restrict__ a, long lda, int Ma, const double2* __restrict__ R,
-                               long ldr, int Mo, cplx<T>* __restrict__ out, long ldo, long N) {
-  extern __shared__ double2 row[];
-  for (long p = blockIdx.x; p < N; p += gridDim.x) {
-    __syncthreads();
-    for (int m = threadIdx.x; m < Ma; m += blockDim.x) {
-      const cplx<T> v = a[p * lda + m];
-      row[m] = make_double2(v.x, v.y);
+// X = U^-1 in place of S: CTA j solves block column j from the diagonal up,
+// X[i][j] = -W_i sum_{i < q <= j} U[i][q] X[q][j], and zeroes it below the diagonal.
+__global__ void __launch_bounds__(256) k_chol_inverse(double2* S, long lds, const double2* __restrict__ U, int M) {
+  __shared__ double2 A[kNB][kNB], B[kNB][kNB];
+  const int j = blockIdx.x, nb = (M + kNB - 1) / kNB;
+  for (int i = j + 1; i < nb; ++i) quad_write(S, lds, M, i, j, quad_zero());
+  for (int i = j - 1; i >= 0; --i) {
+    Quad acc = quad_zero();
+    for (int q = i + 1; q <= j; ++q) {
+      __syncthreads();
+      quad_store(A, quad_load(U, M, M, i, q, false));
+      quad_store(B, quad_load(S, lds, M, q, j, false));
+      __syncthreads();
+      quad_mul<false>(acc, 1.0, A, B);
     }
     __syncthreads();
-    for (int j = threadIdx.x; j < Mo; j += blockDim.x) {
-      double re = 0.0, im = 0.0;
-      for (int i = 0; i < Ma; i++) {
-        const double2 x = row[i], r = R[(long)i * ldr + j];
-        re += x.x * r.x - x.y * r.y;
-        im += x.x * r.y + x.y * r.x;
+    quad_store(A, quad_load(S, lds, M, i, i, false));
+    quad_store(B, acc);
+    __syncthreads();
+    Quad x = quad_zero();
+    quad_mul<false>(x, -1.0, A, B);
+    quad_write(S, lds, M, i, j, x);
+  }
+}
+
+// ---------------------------------------------------------------- rotation
+// out[p][j] = sum_i a[p][i] R[i][j], FP64 arithmetic.  A CTA owns 64 points and (16 TN)
+// columns at a time, 256 threads as 16 x 16 with 4 x TN outputs each; eight orbitals i are
+// staged at a time, the next ones fetched into registers meanwhile.
+// UPPER: R is upper triangular and out may be a.  The CTA walks its columns from the last
+// block down: a block of outputs reads only the input columns up to itself, so it may
+// overwrite its own input columns once they are read.
+template <typename T, int TN, bool UPPER>
+__global__ void __launch_bounds__(256, TN == 4 ? 2 : 3)
+    k_rotate(const cplx<T>* a, long lda, int Ma, const double2* __restrict__ R, long ldr, int Mo, cplx<T>* out,
+             long ldo, long N) {
+  constexpr int TP = 4, PTS = 16 * TP, COLS = 16 * TN, KP = 8;
+  constexpr int PA = PTS * KP / 256, PB = (COLS * KP + 255) / 256;
+  __shared__ double2 sa[KP][PTS + 1];  // [i][point]; the odd row spreads the transposing stores
+  __shared__ double2 sr[KP][COLS];
+  const int tp = grid_row(), tj = grid_col();
+  const long p0 = (long)blockIdx.x * PTS;
+  const int nblk = (Mo + COLS - 1) / COLS;
+  const int b_hi = UPPER ? nblk - 1 : (int)blockIdx.y, b_lo = UPPER ? 0 : (int)blockIdx.y;
+  for (int jb = b_hi; jb >= b_lo; --jb) {
+    const int j0 = jb * COLS;
+    const int kend = UPPER ? min(Ma, j0 + COLS) : Ma;
+    double re[TP][TN], im[TP][TN];
+#pragma unroll
+    for (int u = 0; u < TP; ++u)
+#pragma unroll
+      for (int v = 0; v < TN; ++v) re[u][v] = im[u][v] = 0.0;
+    cplx<T> va[PA];
+    double2 vr[PB];
+    auto fetch = [&](int k0) {
+#pragma unroll
+      for (int u = 0; u < PA; ++u) {
+        const int e = threadIdx.x + 256 * u, i = k0 + e % KP;
+        const long p = p0 + e / KP;
+        va[u] = (p < N && i < kend) ? a[p * lda + i] : mk<T>(0, 0);
       }
-      out[p * ldo + j] = mk<T>((T)re, (T)im);
+#pragma unroll
+      for (int u = 0; u < PB; ++u) {
+        const int e = threadIdx.x + 256 * u, i = k0 + e / COLS, j = j0 + e % COLS;
+        vr[u] = (e < KP * COLS && i < kend && j < Mo) ? R[(long)i * ldr + j] : make_double2(0.0, 0.0);
+      }
+    };
+    fetch(0);
+    for (int k0 = 0; k0 < kend; k0 += KP) {
+#pragma unroll
+      for (int u = 0; u < PA; ++u) {
+        const int e = threadIdx.x + 256 * u;
+        sa[e % KP][e / KP] = make_double2(va[u].x, va[u].y);
+      }
+#pragma unroll
+      for (int u = 0; u < PB; ++u) {
+        const int e = threadIdx.x + 256 * u;
+        if (e < KP * COLS) sr[e / COLS][e % COLS] = vr[u];
+      }
+      __syncthreads();
+      if (k0 + KP < kend) fetch(k0 + KP);
+      const int vmin = UPPER ? max(0, (k0 - j0) / 16) : 0;
+#pragma unroll 4
+      for (int q = 0; q < KP; ++q) {
+        double2 x[TP], y[TN];
+#pragma unroll
+        for (int u = 0; u < TP; ++u) x[u] = sa[q][tp + 16 * u];
+#pragma unroll
+        for (int v = 0; v < TN; ++v) y[v] = sr[q][tj + 16 * v];
+        // UPPER: R[i][j] = 0 for the 16-wide column blocks left of row i
+#pragma unroll
+        for (int v = 0; v < TN; ++v) {
+          if (UPPER && v < vmin) continue;
+#pragma unroll
+          for (int u = 0; u < TP; ++u) {
+            re[u][v] = fma(x[u].x, y[v].x, fma(-x[u].y, y[v].y, re[u][v]));
+            im[u][v] = fma(x[u].x, y[v].y, fma(x[u].y, y[v].x, im[u][v]));
+          }
+        }
+      }
+      __syncthreads();
     }
+#pragma unroll
+    for (int u = 0; u < TP; ++u)
+#pragma unroll
+      for (int v = 0; v < TN; ++v) {
+        const long p = p0 + tp + 16 * u;
+        const int j = j0 + tj + 16 * v;
+        if (p < N && j < Mo) out[p * ldo + j] = mk<T>((T)re[u][v], (T)im[u][v]);
+      }
   }
 }
 
@@ -307,19 +537,43 @@ int launch_dipole(const double* rho, long N, const double lat[3][3], const int n
   return INQB_OK;
 }
 
-template <typename T>
-static int orthonormalize_impl(void* psi, long ld, int M, long N, double dV, double2* S, double2* X, int* info,
-                               cudaStream_t st) {
-  INQB_CUDA_TRY(cudaMemsetAsync(S, 0, sizeof(double2) * (size_t)M * M, st));
-  INQB_CUDA_TRY(cudaMemsetAsync(info, 0, sizeof(int), st));
-  const int tiles = (M + 31) / 32;
-  long nchunks = std::max<long>(1, std::min<long>(N / 1024, (148L * 8) / (tiles * tiles) + 1));
-  const long chunk = (N + nchunks - 1) / nchunks;
-  nchunks = (N + chunk - 1) / chunk;
-  k_overlap<T><<<dim3(tiles, tiles, (unsigned)nchunks), dim3(32, 32), 0, st>>>(
-      (const cplx<T>*)psi, ld, M, (const cplx<T>*)psi, ld, M, N, chunk, dV, S, M);
+// tiles of the output at TM outputs a side per thread; slabs of points so that the CTAs
+// fill the GPU (at least 512 points a slab)
+template <typename T, int TM>
+static int overlap_launch(const void* a, long lda, int Ma, const void* b, long ldb, int Mb, long N, double dV,
+                          double2* S, long lds, bool upper, cudaStream_t st) {
+  constexpr int TILE = 16 * TM, KP = OverlapCfg<TM>::KP;
+  const long ti = (Ma + TILE - 1) / TILE, tj = (Mb + TILE - 1) / TILE;
+  const long tiles = upper ? ti * (ti + 1) / 2 : ti * tj;
+  long slabs = std::max<long>(1, std::min<long>(N / 512, 148L * OverlapCfg<TM>::CTAS / tiles));
+  const long slab = ((N + slabs - 1) / slabs + KP - 1) / KP * KP;
+  slabs = (N + slab - 1) / slab;
+  k_overlap<T, TM><<<dim3((unsigned)tiles, (unsigned)slabs), 256, 0, st>>>(
+      (const cplx<T>*)a, lda, Ma, (const cplx<T>*)b, ldb, Mb, N, slab, dV, S, lds, upper);
   INQB_CUDA_TRY(cudaGetLastError());
-  k_cholesky<<<1, 1024, 0, st>>>(S, M, M, info);
+  return INQB_OK;
+}
+
+// the tile follows the larger block: a 16- or 32-wide tile where a 64-wide one would be
+// mostly padding
+template <typename T>
+static int overlap_any(const void* a, long lda, int Ma, const void* b, long ldb, int Mb, long N, double dV,
+                       double2* S, long lds, bool upper, cudaStream_t st) {
+  const int M = std::max(Ma, Mb);
+  if (M <= 16) return overlap_launch<T, 1>(a, lda, Ma, b, ldb, Mb, N, dV, S, lds, upper, st);
+  if (M <= 32) return overlap_launch<T, 2>(a, lda, Ma, b, ldb, Mb, N, dV, S, lds, upper, st);
+  return overlap_launch<T, 4>(a, lda, Ma, b, ldb, Mb, N, dV, S, lds, upper, st);
+}
+
+// S (upper triangle of a Hermitian matrix) <- U^-1; X: M x M scratch (receives U)
+static int cholesky_inverse_launch(double2* S, int M, long lds, double2* X, int* info, cudaStream_t st) {
+  const int nb = (M + kNB - 1) / kNB;
+  INQB_CUDA_TRY(cudaMemsetAsync(info, 0, sizeof(int), st));
+  for (int k = -1; k + 1 < nb; k++) {
+    const int n = nb - 1 - k;
+    k_chol_step<<<k < 0 ? 1 : n * (n + 1) / 2, 256, 0, st>>>(S, lds, X, M, k, info);
+  }
+  k_chol_inverse<<<nb, 256, 0, st>>>(S, lds, X, M);
   INQB_CUDA_TRY(cudaGetLastError());
   int h_info = 0;
   INQB_CUDA_TRY(cudaMemcpyAsync(&h_info, info, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -327,11 +581,33 @@ static int orthonormalize_impl(void* psi, long ld, int M, long N, double dV, dou
   if (h_info != 0)
     return fail(INQB_ERR_NOT_POSITIVE_DEFINITE,
                 "overlap matrix is not positive definite at pivot " + std::to_string(h_info - 1));
-  k_triangular_inverse<<<(M + 127) / 128, 128, 0, st>>>(S, M, M, X);
+  return INQB_OK;
+}
+
+template <typename T, int TN, bool UPPER>
+static int rotate_launch(const void* a, long lda, int Ma, const double2* R, long ldr, int Mo, void* out, long ldo,
+                         long N, cudaStream_t st) {
+  const dim3 grid((unsigned)((N + 63) / 64), UPPER ? 1u : (unsigned)((Mo + 16 * TN - 1) / (16 * TN)));
+  k_rotate<T, TN, UPPER><<<grid, 256, 0, st>>>((const cplx<T>*)a, lda, Ma, R, ldr, Mo, (cplx<T>*)out, ldo, N);
   INQB_CUDA_TRY(cudaGetLastError());
-  const int blocks = (int)std::min<long>(N, 148L * 16);
-  k_rotate_upper<T><<<blocks, 128, sizeof(double2) * M, st>>>((cplx<T>*)psi, ld, M, N, X);
-  INQB_CUDA_TRY(cudaGetLastError());
+  return INQB_OK;
+}
+
+template <typename T, bool UPPER>
+static int rotate_any(const void* a, long lda, int Ma, const double2* R, long ldr, int Mo, void* out, long ldo, long N,
+                      cudaStream_t st) {
+  if (Mo <= 16) return rotate_launch<T, 1, UPPER>(a, lda, Ma, R, ldr, Mo, out, ldo, N, st);
+  if (Mo <= 32) return rotate_launch<T, 2, UPPER>(a, lda, Ma, R, ldr, Mo, out, ldo, N, st);
+  return rotate_launch<T, 4, UPPER>(a, lda, Ma, R, ldr, Mo, out, ldo, N, st);
+}
+
+template <typename T>
+static int orthonormalize_impl(void* psi, long ld, int M, long N, double dV, double2* S, double2* X, int* info,
+                               cudaStream_t st) {
+  INQB_CUDA_TRY(cudaMemsetAsync(S, 0, sizeof(double2) * (size_t)M * M, st));
+  INQB_TRY(overlap_any<T>(psi, ld, M, psi, ld, M, N, dV, S, M, true, st));
+  INQB_TRY(cholesky_inverse_launch(S, M, M, X, info, st));
+  INQB_TRY((rotate_any<T, true>(psi, ld, M, S, M, M, psi, ld, N, st)));
   INQB_CUDA_TRY(cudaStreamSynchronize(st));
   return INQB_OK;
 }
@@ -351,15 +627,7 @@ template <typename T>
 static int overlap_block_impl(const void* a, long lda, int Ma, const void* b, long ldb, int Mb, long N, double dV,
                               double2* S, long lds, cudaStream_t st) {
   INQB_CUDA_TRY(cudaMemset2DAsync(S, sizeof(double2) * lds, 0, sizeof(double2) * Mb, Ma, st));
-  const int ti = (Ma + 31) / 32, tj = (Mb + 31) / 32;
-  long nchunks = std::max<long>(1, std::min<long>(N / 1024, (148L * 8) / (ti * tj) + 1));
-  const long chunk = (N + nchunks - 1) / nchunks;
-  nchunks = (N + chunk - 1) / chunk;
-  k_overlap<T><<<dim3(tj, ti, (unsigned)nchunks), dim3(32, 32), 0, st>>>((const cplx<T>*)a, lda, Ma,
-                                                                          (const cplx<T>*)b, ldb, Mb, N, chunk, dV,
-                                                                          S, lds);
-  INQB_CUDA_TRY(cudaGetLastError());
-  return INQB_OK;
+  return overlap_any<T>(a, lda, Ma, b, ldb, Mb, N, dV, S, lds, false, st);
 }
 
 int launch_overlap_block(int precision, const void* a, long lda, int Ma, const void* b, long ldb, int Mb, long N,
@@ -370,39 +638,14 @@ int launch_overlap_block(int precision, const void* a, long lda, int Ma, const v
 }
 
 int launch_cholesky_inverse(double2* S, int M, long lds, double2* X, int* info, void* stream) {
-  cudaStream_t st = (cudaStream_t)stream;
-  INQB_CUDA_TRY(cudaMemsetAsync(info, 0, sizeof(int), st));
-  k_cholesky<<<1, 1024, 0, st>>>(S, M, lds, info);
-  INQB_CUDA_TRY(cudaGetLastError());
-  int h_info = 0;
-  INQB_CUDA_TRY(cudaMemcpyAsync(&h_info, info, sizeof(int), cudaMemcpyDeviceToHost, st));
-  INQB_CUDA_TRY(cudaStreamSynchronize(st));
-  if (h_info != 0)
-    return fail(INQB_ERR_NOT_POSITIVE_DEFINITE,
-                "overlap matrix is not positive definite at pivot " + std::to_string(h_info - 1));
-  k_triangular_inverse<<<(M + 127) / 128, 128, 0, st>>>(S, M, lds, X);
-  INQB_CUDA_TRY(cudaGetLastError());
-  INQB_CUDA_TRY(cudaMemcpy2DAsync(S, sizeof(double2) * lds, X, sizeof(double2) * M, sizeof(double2) * M, M,
-                                  cudaMemcpyDeviceToDevice, st));
-  INQB_CUDA_TRY(cudaStreamSynchronize(st));
-  return INQB_OK;
-}
-
-template <typename T>
-static int rotate_block_impl(const void* a, long lda, int Ma, const double2* R, long ldr, int Mo, void* out,
-                             long ldo, long N, cudaStream_t st) {
-  const int blocks = (int)std::min<long>(N, 148L * 16);
-  k_rotate_block<T><<<blocks, 128, sizeof(double2) * Ma, st>>>((const cplx<T>*)a, lda, Ma, R, ldr, Mo,
-                                                               (cplx<T>*)out, ldo, N);
-  INQB_CUDA_TRY(cudaGetLastError());
-  return INQB_OK;
+  return cholesky_inverse_launch(S, M, lds, X, info, (cudaStream_t)stream);
 }
 
 int launch_rotate_block(int precision, const void* a, long lda, int Ma, const double2* R, long ldr, int Mo,
                         void* out, long ldo, long N, void* stream) {
   return precision == INQB_FP64
-             ? rotate_block_impl<double>(a, lda, Ma, R, ldr, Mo, out, ldo, N, (cudaStream_t)stream)
-             : rotate_block_impl<float>(a, lda, Ma, R, ldr, Mo, out, ldo, N, (cudaStream_t)stream);
+             ? rotate_any<double, false>(a, lda, Ma, R, ldr, Mo, out, ldo, N, (cudaStream_t)stream)
+             : rotate_any<float, false>(a, lda, Ma, R, ldr, Mo, out, ldo, N, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------- orthonormalisation without allocation

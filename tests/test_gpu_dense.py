@@ -1,0 +1,74 @@
+"""The dense orbital kernels at the edges of their tiles: the overlap and rotation tiles
+(16, 32 and 64 wide) and the blocks of 32 of the Cholesky factor and its inverse, against
+numpy.
+
+Tolerances: a sum of n rounded FP64 products is within about sqrt(n) 1.1e-16 of its
+2-norm; the factor's condition number (below 10 for these sets) multiplies it once."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [1, 15, 16, 17, 31, 32, 33, 63, 64, 65, 100, 129]
+
+
+def _ham(pb, n=16, precision="fp64"):
+    return pb.KSHamiltonian(np.eye(3) * 6.0, (n, n, n), precision)
+
+
+def _block(h, M, ld, seed, dtype):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn((h.N, ld, 2), generator=g, device="cuda", dtype=torch.float64)
+    return torch.view_as_complex(x).to(dtype)[:, :M]
+
+
+@pytest.mark.parametrize("M", SIZES)
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-13), ("mixed", 1e-6)])
+def test_orthonormalize_edges(pb, M, precision, tol):
+    h = _ham(pb, precision=precision)
+    x = _block(h, M, M + 3, M, h.dtype)
+    pad = x.as_strided((h.N, 3), (M + 3, 1), M).clone()
+    ref = x.to(torch.complex128)
+    u = torch.linalg.cholesky(h.volume_element * (ref.conj().T @ ref), upper=True)
+    ref = torch.linalg.solve_triangular(u, ref, upper=True, left=False)
+    h.orthonormalize_(x)
+    assert float((x - ref).norm() / ref.norm()) < tol
+    assert torch.equal(x.as_strided((h.N, 3), (M + 3, 1), M), pad)  # past the block: untouched
+
+
+@pytest.mark.parametrize("Ma,Mb", [(1, 1), (5, 33), (33, 5), (17, 64), (65, 100)])
+def test_overlap_and_rotate_blocks(pb, Ma, Mb):
+    h = _ham(pb)
+    a, b = _block(h, Ma, Ma + 1, 1, h.dtype), _block(h, Mb, Mb, 2, h.dtype)
+    S = h.overlap_block(a, b)
+    ref = h.volume_element * (a.conj().T @ b)
+    assert float((S - ref).norm() / ref.norm()) < 1e-13
+    got = h.rotate_block(a, S)
+    assert float((got - a @ S).norm() / (a @ S).norm()) < 1e-14
+
+
+@pytest.mark.parametrize("M", SIZES)
+def test_cholesky_inverse_edges(pb, M):
+    h = _ham(pb)
+    x = _block(h, M, M, 7, torch.complex128)
+    S = (x.conj().T @ x) / h.N + 0.1 * torch.eye(M, device="cuda")
+    big = torch.full((M, M + 2), 5.0 + 1.0j, dtype=torch.complex128, device="cuda")
+    big[:, :M] = S
+    ref = torch.linalg.inv(torch.linalg.cholesky(S, upper=True))
+    got = h.cholesky_inverse_(big[:, :M])
+    assert float((got - ref).norm() / ref.norm()) < 1e-13
+    assert float(torch.tril(got, -1).abs().sum()) == 0.0
+    assert torch.all(big[:, M:] == 5.0 + 1.0j)
+
+
+@pytest.mark.parametrize("M,zero", [(40, 0), (40, 31), (40, 32), (100, 97)])
+def test_cholesky_reports_the_first_failing_pivot(pb, M, zero):
+    h = _ham(pb)
+    x = _block(h, M, M, 3, torch.complex128).clone()
+    x[:, zero] = 0  # an exact zero pivot
+    keep = x.clone()
+    with pytest.raises(pb.InqbError) as e:
+        h.orthonormalize_(x)
+    assert f"pivot {zero}" in str(e.value)
+    assert torch.equal(x, keep)
