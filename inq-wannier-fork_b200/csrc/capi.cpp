@@ -364,7 +364,7 @@ struct MlwfWork {
   void* partial = nullptr;   // per-slab Gram partial sums
   int2* pairs = nullptr;     // [2 np - 1][np]
   double* delta = nullptr;   // [2 np - 1][np]
-  double* change = nullptr;  // [1]
+  double* change = nullptr;  // [2]: the sweep's trace change; sweeps run
 };
 
 int mlwf_work(inqb_ctx* ctx, int M, bool with_gram, MlwfWork& w) {
@@ -379,7 +379,7 @@ int mlwf_work(inqb_ctx* ctx, int M, bool with_gram, MlwfWork& w) {
   const size_t oa = take(sizeof(double2) * 6 * MM), ou = take(sizeof(double2) * MM),
                od = take(sizeof(double2) * 6 * M), os = take(sizeof(double) * 3 * M),
                op = take(partial_bytes), opr = take(sizeof(int2) * steps * np),
-               ode = take(sizeof(double) * steps * np), oc = take(sizeof(double));
+               ode = take(sizeof(double) * steps * np), oc = take(2 * sizeof(double));
   INQB_TRY(ctx->d_mlwf.ensure(off));
   char* b = static_cast<char*>(ctx->d_mlwf.ptr);
   w.a = reinterpret_cast<double2*>(b + oa);
@@ -394,8 +394,7 @@ int mlwf_work(inqb_ctx* ctx, int M, bool with_gram, MlwfWork& w) {
 }
 
 // One JADE sweep (2 np - 1 rotation steps and the trace-change sum) as a CUDA graph:
-// captured once per call on a private stream, launched once per sweep (the sweep's
-// pair schedule is copied to the same buffer before each launch).
+// captured once per call on a private stream, launched once per sweep.
 struct SweepGraph {
   cudaStream_t cap = nullptr;
   cudaGraph_t graph = nullptr;
@@ -420,51 +419,68 @@ struct SweepGraph {
   }
 };
 
-// jade_complex on device arrays a [6][M][M] (rotated in place), u, adiag.  The pair
-// schedule of each sweep is made on the host (the reference's round-robin shift) and
-// copied before the sweep; the sweep's trace change is read back once per sweep.
-int jade_dev(int M, double2* a, double2* u, double2* adiag, int maxsweep, double tol, const MlwfWork& w, int* sweeps,
-             void* stream) {
-  const int np = (M + 1) / 2, steps = 2 * np - 1;
-  cudaStream_t st = (cudaStream_t)stream;
-  INQB_TRY(launch_identity(u, M, stream));
+// The pairs of one sweep's rotation steps, [2 np - 1][np].  The reference's shift returns
+// to its start after them, so every sweep takes the same pairs.
+std::vector<int2> jade_schedule(int np) {
+  const int steps = 2 * np - 1;
+  std::vector<int2> sched((size_t)steps * np);
   std::vector<int> top(np), bot(np);
   for (int i = 0; i < np; i++) {
     top[i] = i;
     bot[np - i - 1] = np + i;
   }
-  std::vector<int2> sched((size_t)steps * np);
-  SweepGraph graph;
-  int nsweep = 0;
-  for (;;) {
-    ++nsweep;
-    for (int s = 0; s < steps; s++) {
-      for (int i = 0; i < np; i++) sched[(size_t)s * np + i] = make_int2(top[i], bot[i]);
-      // the reference's shift: bot[j] <- bot[j+1], top[j+1] <- top[j] as one parallel
-      // move, then the ends, then one swap (jade_complex.hpp:296-322)
-      const int top_back = top[np - 1], bot_front = bot[0];
-      std::vector<int> t2 = top, b2 = bot;
-      for (int j = 0; j + 1 < np; j++) {
-        b2[j] = bot[j + 1];
-        t2[j + 1] = top[j];
-      }
-      b2[np - 1] = top_back;
-      t2[0] = bot_front;
-      if (np > 1)
-        std::swap(t2[0], t2[1]);
-      else
-        std::swap(t2[0], b2[0]);
-      top.swap(t2);
-      bot.swap(b2);
+  for (int s = 0; s < steps; s++) {
+    for (int i = 0; i < np; i++) sched[(size_t)s * np + i] = make_int2(top[i], bot[i]);
+    // the reference's shift: bot[j] <- bot[j+1], top[j+1] <- top[j] as one parallel
+    // move, then the ends, then one swap (jade_complex.hpp:296-322)
+    const int top_back = top[np - 1], bot_front = bot[0];
+    std::vector<int> t2 = top, b2 = bot;
+    for (int j = 0; j + 1 < np; j++) {
+      b2[j] = bot[j + 1];
+      t2[j + 1] = top[j];
     }
-    INQB_CUDA_TRY(cudaMemcpyAsync(w.pairs, sched.data(), sizeof(int2) * sched.size(), cudaMemcpyHostToDevice, st));
-    if (!graph.exec) INQB_TRY(graph.capture(M, a, u, w, np, steps));
-    INQB_CUDA_TRY(cudaGraphLaunch(graph.exec, st));
-    double change = 0.0;
-    INQB_CUDA_TRY(cudaMemcpyAsync(&change, w.change, sizeof(double), cudaMemcpyDeviceToHost, st));
+    b2[np - 1] = top_back;
+    t2[0] = bot_front;
+    if (np > 1)
+      std::swap(t2[0], t2[1]);
+    else
+      std::swap(t2[0], b2[0]);
+    top.swap(t2);
+    bot.swap(b2);
+  }
+  return sched;
+}
+
+// jade_complex on device arrays a [6][M][M] (rotated in place), u, adiag.  Where a cluster's
+// shared memory holds the matrices, all sweeps run in one launch; else one graph of
+// per-step launches a sweep, the sweep's trace change read back after each.
+int jade_dev(int M, double2* a, double2* u, double2* adiag, int maxsweep, double tol, const MlwfWork& w, int* sweeps,
+             void* stream) {
+  const int np = (M + 1) / 2, steps = 2 * np - 1;
+  cudaStream_t st = (cudaStream_t)stream;
+  const std::vector<int2> sched = jade_schedule(np);
+  INQB_CUDA_TRY(cudaMemcpyAsync(w.pairs, sched.data(), sizeof(int2) * sched.size(), cudaMemcpyHostToDevice, st));
+  double change[2] = {0.0, 0.0};
+  bool one_launch = false;
+  INQB_TRY(launch_jade_cluster(a, u, M, w.pairs, np, steps, maxsweep, tol, w.delta, w.change, &one_launch, stream));
+  int nsweep = 0;
+  if (one_launch) {
+    INQB_CUDA_TRY(cudaMemcpyAsync(change, w.change, sizeof(change), cudaMemcpyDeviceToHost, st));
     INQB_CUDA_TRY(cudaStreamSynchronize(st));
-    if (!std::isfinite(change)) return fail(INQB_ERR_NONFINITE, "TD-MLWF matrices are not finite");
-    if (std::fabs(change) < tol || nsweep >= maxsweep) break;
+    if (!std::isfinite(change[0])) return fail(INQB_ERR_NONFINITE, "TD-MLWF matrices are not finite");
+    nsweep = (int)change[1];
+  } else {
+    INQB_TRY(launch_identity(u, M, stream));
+    SweepGraph graph;
+    INQB_TRY(graph.capture(M, a, u, w, np, steps));
+    for (;;) {
+      ++nsweep;
+      INQB_CUDA_TRY(cudaGraphLaunch(graph.exec, st));
+      INQB_CUDA_TRY(cudaMemcpyAsync(change, w.change, sizeof(double), cudaMemcpyDeviceToHost, st));
+      INQB_CUDA_TRY(cudaStreamSynchronize(st));
+      if (!std::isfinite(change[0])) return fail(INQB_ERR_NONFINITE, "TD-MLWF matrices are not finite");
+      if (std::fabs(change[0]) < tol || nsweep >= maxsweep) break;
+    }
   }
   INQB_TRY(launch_jade_adiag(a, u, M, adiag, stream));
   if (sweeps) *sweeps = nsweep;

@@ -14,6 +14,7 @@
 //            disjoint, so rotating two rows per pair is the same product in O(M) per pair.
 //   adiag    adiag[k][i] = sum_j conj(a_k[i][j]) u[i][j]
 //   rotate   psi <- psi u^H (operations::rotate), tiled through shared memory
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -35,6 +36,7 @@ __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -
 // ------------------------------------------------------------------ gram
 // 256 threads as 16 x 16; thread (tm, tn) holds outputs m = m0 + tm + 16 a (a < TMX),
 // n = n0 + tn + 16 b (b < TNX) for the three directions; CTA tile (16 TMX) x (16 TNX).
+// Axis lengths are those of the FFT size table, N below 2^31.
 // FP64 contexts accumulate in FP64 over the CTA's slab (few slabs).  The mixed context
 // accumulates FP32 products in FP32 over a slab of at most kSlabF32 points and keeps one
 // FP32 partial per slab; the finish kernel adds the slabs in FP64 (the FP32 rounding of
@@ -51,33 +53,52 @@ template <typename T>
 struct GramCfg;
 template <>
 struct GramCfg<double> {
-  static constexpr int TMX = 2, TNX = 2, GP = 16, MINB = 2;  // GP: points per staged chunk
+  static constexpr int TMX = 4, TNX = 2, GP = 16, MINB = 1;  // GP: points per staged chunk
   using P = double2;                                         // partial type
 };
 template <>
 struct GramCfg<float> {
-  static constexpr int TMX = 4, TNX = 2, GP = 32, MINB = 3;
+  static constexpr int TMX = 4, TNX = 2, GP = 16, MINB = 3;
   using P = float2;
 };
 
 __device__ __forceinline__ void store_partial(double2* p, double x, double y) { *p = make_double2(x, y); }
 __device__ __forceinline__ void store_partial(float2* p, float x, float y) { *p = make_float2(x, y); }
 
-// grid (tiles_m * tiles_n, nslab)
+// e^{i theta_d} factorises over the axes: axis table entry [d][j][n] = exp(i pi
+// frac_to_theta[d][j] f_j(n)), n a grid index of axis j (at most kAxisMax of them).
+constexpr int kAxisMax = 256;
+__global__ void k_mlwf_axis(GramGeom geo, double2* __restrict__ tab) {
+  const int j = blockIdx.x % 3, d = blockIdx.x / 3;
+  for (int n = threadIdx.x; n < geo.nr[j]; n += blockDim.x) {
+    const int sy = (n >= (geo.nr[j] + 1) / 2) ? n - geo.nr[j] : n;
+    double sn, cs;
+    sincospi(geo.frac_to_theta[d][j] * ((double)sy / geo.nr[j]), &sn, &cs);
+    tab[(d * 3 + j) * kAxisMax + n] = make_double2(cs, sn);
+  }
+}
+
+// grid (tiles_m * tiles_n, nslab).  Bound by the FP64 (FP32) units: 4 x 2 outputs of three
+// directions take 96 fused multiply-adds for 10 shared loads.  The next chunk's orbitals
+// are fetched into registers and its weights formed from the axis tables while the current
+// chunk is summed.
 template <typename T>
 __global__ void __launch_bounds__(256, GramCfg<T>::MINB)
     k_mlwf_gram(const cplx<T>* __restrict__ pa, long lda, int Ma, const cplx<T>* __restrict__ pb, long ldb, int Mb,
-                long N, GramGeom geo, long pts_per_slab, typename GramCfg<T>::P* __restrict__ partial) {
+                long N, GramGeom geo, const double2* __restrict__ tab, long pts_per_slab,
+                typename GramCfg<T>::P* __restrict__ partial) {
   using R = T;
   constexpr int TMX = GramCfg<T>::TMX, TNX = GramCfg<T>::TNX, kGP = GramCfg<T>::GP;
   constexpr int TILE_M = 16 * TMX, TILE_N = 16 * TNX;
+  constexpr int PA = kGP * TILE_M / 256, PB = kGP * TILE_N / 256;
   __shared__ cplx<R> sA[kGP][TILE_M];
   __shared__ cplx<R> sB[3][kGP][TILE_N];
-  __shared__ cplx<R> sW[3][kGP];
+  __shared__ cplx<R> sW[2][3][kGP];
   const int tiles_m = (Ma + TILE_M - 1) / TILE_M;
   const int m0 = (blockIdx.x % tiles_m) * TILE_M, n0 = (blockIdx.x / tiles_m) * TILE_N;
   const long p_beg = (long)blockIdx.y * pts_per_slab, p_end = min(N, p_beg + pts_per_slab);
-  const int tm = threadIdx.x % 16, tn = threadIdx.x / 16;
+  // a warp is 8 x 4 of the 16 x 16 thread grid (its shared loads take one wavefront each)
+  const int tm = threadIdx.x / 128 * 8 + threadIdx.x % 8, tn = (threadIdx.x / 32) % 4 * 4 + threadIdx.x % 32 / 8;
   R acc[3][TMX][TNX][2];
 #pragma unroll
   for (int d = 0; d < 3; ++d)
@@ -85,44 +106,50 @@ __global__ void __launch_bounds__(256, GramCfg<T>::MINB)
     for (int a = 0; a < TMX; ++a)
 #pragma unroll
       for (int b = 0; b < TNX; ++b) acc[d][a][b][0] = acc[d][a][b][1] = (R)0;
-  for (long pc = p_beg; pc < p_end; pc += kGP) {
-    // weights of the chunk's points, e^{i theta_d}
-    if (threadIdx.x < kGP) {
-      const long p = pc + threadIdx.x;
-      cplx<R> w[3] = {mk<R>(0, 0), mk<R>(0, 0), mk<R>(0, 0)};
-      if (p < p_end) {
-        const int iz = (int)(p % geo.nr[2]), iy = (int)((p / geo.nr[2]) % geo.nr[1]),
-                  ix = (int)(p / ((long)geo.nr[1] * geo.nr[2]));
-        const int id[3] = {ix, iy, iz};
-        double f[3];
-        for (int j = 0; j < 3; ++j) {
-          const int sy = (id[j] >= (geo.nr[j] + 1) / 2) ? id[j] - geo.nr[j] : id[j];
-          f[j] = (double)sy / geo.nr[j];
-        }
-        for (int d = 0; d < 3; ++d) {
-          const double th = geo.frac_to_theta[d][0] * f[0] + geo.frac_to_theta[d][1] * f[1] +
-                            geo.frac_to_theta[d][2] * f[2];
-          double sn, cs;
-          sincospi(th, &sn, &cs);
-          w[d] = mk<R>((R)cs, (R)sn);
-        }
-      }
-      for (int d = 0; d < 3; ++d) sW[d][threadIdx.x] = w[d];
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < kGP * TILE_M; i += blockDim.x) {
-      const int q = i / TILE_M, j = i % TILE_M;
-      const long p = pc + q;
-      sA[q][j] = (p < p_end && m0 + j < Ma) ? pa[p * lda + m0 + j] : mk<R>(0, 0);
-    }
-    for (int i = threadIdx.x; i < kGP * TILE_N; i += blockDim.x) {
-      const int q = i / TILE_N, j = i % TILE_N;
-      const long p = pc + q;
-      const cplx<R> vb = (p < p_end && n0 + j < Mb) ? pb[p * ldb + n0 + j] : mk<R>(0, 0);
+  cplx<R> va[PA], vb[PB];
+  auto fetch = [&](long pc) {
 #pragma unroll
-      for (int d = 0; d < 3; ++d) sB[d][q][j] = sW[d][q] * vb;
+    for (int u = 0; u < PA; ++u) {
+      const int i = threadIdx.x + 256 * u, q = i / TILE_M, j = i % TILE_M;
+      va[u] = (pc + q < p_end && m0 + j < Ma) ? pa[(pc + q) * lda + m0 + j] : mk<R>(0, 0);
+    }
+#pragma unroll
+    for (int u = 0; u < PB; ++u) {
+      const int i = threadIdx.x + 256 * u, q = i / TILE_N, j = i % TILE_N;
+      vb[u] = (pc + q < p_end && n0 + j < Mb) ? pb[(pc + q) * ldb + n0 + j] : mk<R>(0, 0);
+    }
+  };
+  // weights of a chunk's points, e^{i theta_d}
+  auto weights = [&](long pc, int buf) {
+    if (threadIdx.x >= 3 * kGP) return;
+    const int d = threadIdx.x / kGP, q = threadIdx.x % kGP;
+    const unsigned p = (unsigned)min(pc + q, N - 1);
+    const unsigned iz = p % geo.nr[2], r = p / geo.nr[2], iy = r % geo.nr[1], ix = r / geo.nr[1];
+    const double2* t = tab + d * 3 * kAxisMax;
+    const double2 w = cmul(cmul(t[ix], t[kAxisMax + iy]), t[2 * kAxisMax + iz]);
+    sW[buf][d][q] = mk<R>((R)w.x, (R)w.y);
+  };
+  fetch(p_beg);
+  weights(p_beg, 0);
+  __syncthreads();
+  int buf = 0;
+  for (long pc = p_beg; pc < p_end; pc += kGP, buf ^= 1) {
+#pragma unroll
+    for (int u = 0; u < PA; ++u) {
+      const int i = threadIdx.x + 256 * u;
+      sA[i / TILE_M][i % TILE_M] = va[u];
+    }
+#pragma unroll
+    for (int u = 0; u < PB; ++u) {
+      const int i = threadIdx.x + 256 * u, q = i / TILE_N;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) sB[d][q][i % TILE_N] = sW[buf][d][q] * vb[u];
     }
     __syncthreads();
+    if (pc + kGP < p_end) {
+      fetch(pc + kGP);
+      weights(pc + kGP, buf ^ 1);
+    }
 #pragma unroll 2
     for (int q = 0; q < kGP; ++q) {
       cplx<R> av[TMX];
@@ -160,21 +187,33 @@ __global__ void __launch_bounds__(256, GramCfg<T>::MINB)
       }
 }
 
-// Z[e] = sum over the slabs of partial[slab][e] in FP64, e = (d, m, n): the slabs' sums
-// in slab order, reads coalesced along e, eight slabs in flight per thread.
+// Z[e] = sum over the slabs of partial[slab][e] in FP64, e = (d, m, n).  A block holds 32
+// elements x 8 parts: part k adds the slabs k, k + 8, ... in order, four loads in flight, and
+// the parts are added in order (a fixed order; one thread per element left most SMs idle).
 template <typename P>
-__global__ void k_mlwf_slab_sum(const P* __restrict__ partial, int nslab, long n, double2* __restrict__ Z) {
-  for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
-    double zx = 0.0, zy = 0.0;
-    for (int s0 = 0; s0 < nslab; s0 += 8) {
-      P v[8];
+__global__ void __launch_bounds__(256) k_mlwf_slab_sum(const P* __restrict__ partial, int nslab, long n, double2* __restrict__ Z) {
+  __shared__ double2 red[8][32];
+  const int part = threadIdx.x / 32, el = threadIdx.x % 32;
+  const long e = (long)blockIdx.x * 32 + el;
+  double zx = 0.0, zy = 0.0;
+  if (e < n) {
+    for (int s0 = part; s0 < nslab; s0 += 32) {
+      P v[4];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = (s0 + u < nslab) ? partial[(size_t)(s0 + u) * n + e] : P{0, 0};
+      for (int u = 0; u < 4; ++u) v[u] = (s0 + 8 * u < nslab) ? partial[(size_t)(s0 + 8 * u) * n + e] : P{0, 0};
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
+      for (int u = 0; u < 4; ++u) {
         zx += (double)v[u].x;
         zy += (double)v[u].y;
       }
+    }
+  }
+  red[part][el] = make_double2(zx, zy);
+  __syncthreads();
+  if (part == 0 && e < n) {
+    for (int k = 1; k < 8; ++k) {
+      zx += red[k][el].x;
+      zy += red[k][el].y;
     }
     Z[e] = make_double2(zx, zy);
   }
@@ -215,8 +254,15 @@ __device__ void jacobi3_top(double S[3][3], double out[3]) {
     for (int q = 0; q < 3; q++)
 #pragma unroll
       for (int p = 0; p < q; p++) off += S[p][q] * S[p][q];
+    // converged once every rotation left is below 2^-60: it would change no digit of V (the
+    // iteration's last passes only drive the off-diagonal to an exact zero), nor does a
+    // non-finite matrix go on (reported by the sweep's change)
+    constexpr double tiny = 8.7e-19;
+    if (fabs(S[0][1]) <= tiny * fabs(d[1] - d[0]) && fabs(S[0][2]) <= tiny * fabs(d[2] - d[0]) &&
+        fabs(S[1][2]) <= tiny * fabs(d[2] - d[1]))
+      break;
     const double thresh = sqrt(off) / 12.0;
-    if (!(thresh > 0.0)) break;  // converged, or a non-finite matrix (reported by the sweep's change)
+    if (!(thresh > 0.0)) break;
 #pragma unroll
     for (int p = 0; p < 3; p++)
 #pragma unroll
@@ -227,16 +273,13 @@ __device__ void jacobi3_top(double S[3][3], double out[3]) {
           continue;
         }
         if (fabs(S[p][q]) < thresh) continue;
+        // t = tan of the rotation angle, the smaller root: 2 S / (h +- sqrt(h^2 + 4 S^2))
+        // with the sign of h S (+ for h = 0); c, s = 1, t over sqrt(1 + t^2); tau = s / (1 + c)
         double h = d[q] - d[p];
-        double t;
-        if (fabs(h) + big == fabs(h)) {
-          t = S[p][q] / h;
-        } else {
-          const double theta = 0.5 * h / S[p][q];
-          t = 1.0 / (fabs(theta) + sqrt(1.0 + theta * theta));
-          if (theta < 0.0) t = -t;
-        }
-        const double c = 1.0 / sqrt(1.0 + t * t), s = t * c, tau = s / (1.0 + c);
+        const double e2 = 2.0 * fabs(S[p][q]), dd = fabs(h) + sqrt(fma(h, h, e2 * e2));
+        const double sg = (h != 0.0 && (h < 0.0) != (S[p][q] < 0.0)) ? -1.0 : 1.0;
+        const double rn = rsqrt(fma(dd, dd, e2 * e2));
+        const double t = sg * (e2 / dd), c = dd * rn, s = sg * (e2 * rn), tau = s / (1.0 + c);
         h = t * S[p][q];
         inc[p] -= h;
         inc[q] += h;
@@ -259,28 +302,23 @@ __device__ void jacobi3_top(double S[3][3], double out[3]) {
         for (int j = 0; j < 3; j++) INQB_JROT(V[j][p], V[j][q])
 #undef INQB_JROT
       }
+#pragma unroll
     for (int i = 0; i < 3; i++) {
       base[i] += inc[i];
       d[i] = base[i];
       inc[i] = 0.0;
     }
   }
-  for (int k = 0; k < 2; k++) {
-    int m = k;
-    for (int l = k + 1; l < 3; l++)
-      if (d[l] < d[m]) m = l;
-    if (m != k) {
-      const double t = d[m];
-      d[m] = d[k];
-      d[k] = t;
-      for (int i = 0; i < 3; i++) {
-        const double v = V[i][m];
-        V[i][m] = V[i][k];
-        V[i][k] = v;
-      }
-    }
+  // the column that an ascending selection sort of d leaves last (constant indices, so that
+  // everything stays in registers)
+  const int m = (d[1] < d[0]) ? (d[2] < d[1] ? 2 : 1) : (d[2] < d[0] ? 2 : 0);
+  const bool two = m == 2;                        // the two left are (1, 0), else (m == 1 ? 0 : 1, 2)
+  const double da = (m == 1) ? d[0] : d[1], db = two ? d[0] : d[2];
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    const double va = (m == 1) ? V[i][0] : V[i][1], vb = two ? V[i][0] : V[i][2];
+    out[i] = db < da ? va : vb;
   }
-  for (int i = 0; i < 3; i++) out[i] = V[i][2];
 }
 
 constexpr int kJT = 128;  // threads of a pair's CTA
@@ -398,6 +436,175 @@ __global__ void k_jade_change(const double* __restrict__ delta, int nsteps, int 
   }
 }
 
+// ------------------------------------------------------------------ jade in one cluster
+// All sweeps in one launch of one thread-block cluster that holds the six matrices and u in
+// its shared memory (row r in CTA r % CL).  A rotation step is bound by latency, not by
+// bytes: the 3 x 3 eigenproblem is a serial chain, and the launch, the row gathers from L2
+// and the block reductions around it cost several times as much when every step is a launch
+// of its own.  Here a step is one cluster barrier, rows over distributed shared memory, and
+// a group of seven warps per pair: warp k sums and rotates matrix k (warp 6: u).
+//   kJG = 7 warps of a group; E: elements of a row per lane (M <= 32 E); GMAX: groups
+constexpr int kJG = 7 * 32;
+
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+struct JadeShared {
+  double red[6][6];  // warp k: Re, Im of the pair elements (pq, pp, qq) of matrix k
+  double diag[6][2];  // warp k: change of the two diagonal elements
+  double rot[3];     // c, Re s, Im s
+};
+
+template <int E, int GMAX>
+__global__ void __launch_bounds__(GMAX * kJG)
+    k_jade_cluster(double2* __restrict__ a, double2* __restrict__ u, int M, const int2* __restrict__ pairs, int np,
+                   int steps, int maxsweep, double tol, double* delta, double* __restrict__ out) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int CL = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  extern __shared__ __align__(16) double2 rows[];  // [rows of this CTA][7][M]
+  __shared__ JadeShared sh[GMAX];
+  __shared__ double part[GMAX * kJG];
+  const size_t MM = (size_t)M * M;
+  const int mine = (M - rank + CL - 1) / CL;  // rows r = rank, rank + CL, ...
+  for (int e = threadIdx.x; e < mine * 7 * M; e += blockDim.x) {
+    const int i = e % M, k = (e / M) % 7, r = rank + CL * (e / (7 * M));
+    rows[e] = k < 6 ? a[k * MM + (size_t)r * M + i] : make_double2(r == i ? 1.0 : 0.0, 0.0);
+  }
+  const int g = threadIdx.x / kJG, k = (threadIdx.x % kJG) / 32, lane = threadIdx.x & 31;
+  const int PG = blockDim.x / kJG;
+  JadeShared& q = sh[g];
+  int nsweep = 0;
+  double change = 0.0;
+  for (;;) {
+    ++nsweep;
+    for (int st = 0; st < steps; ++st) {
+      cluster.sync();  // the rows of the step before are in place
+      for (int pi = rank + CL * g; pi < np; pi += CL * PG) {
+        const int2 pq = pairs[(size_t)st * np + pi];
+        if (pq.x >= M || pq.y >= M) {
+          if (threadIdx.x % kJG == 0) delta[(size_t)st * np + pi] = 0.0;
+          continue;
+        }
+        double2* rp = cluster.map_shared_rank(rows, pq.x % CL) + (size_t)(pq.x / CL) * 7 * M;
+        double2* rq = cluster.map_shared_rank(rows, pq.y % CL) + (size_t)(pq.y / CL) * 7 * M;
+        double2 xp[E], xq[E];
+#pragma unroll
+        for (int t = 0; t < E; ++t) {
+          const int i = lane + 32 * t;
+          xp[t] = xq[t] = make_double2(0.0, 0.0);
+          if (i < M) {
+            xp[t] = rp[k * M + i];
+            xq[t] = rq[k * M + i];
+          }
+        }
+        if (k < 6) {
+          // sums of conj(a_p) u_q, conj(a_p) u_p, conj(a_q) u_q
+          double s[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+          for (int t = 0; t < E; ++t) {
+            const int i = lane + 32 * t;
+            if (i < M) {
+              const double2 up = rp[6 * M + i], uq = rq[6 * M + i];
+              const double2 x0 = cmul(cconj(xp[t]), uq), x1 = cmul(cconj(xp[t]), up), x2 = cmul(cconj(xq[t]), uq);
+              s[0] += x0.x;
+              s[1] += x0.y;
+              s[2] += x1.x;
+              s[3] += x1.y;
+              s[4] += x2.x;
+              s[5] += x2.y;
+            }
+          }
+#pragma unroll
+          for (int v = 0; v < 6; ++v) s[v] = warp_sum(s[v]);
+          if (lane == 0) {
+#pragma unroll
+            for (int v = 0; v < 6; ++v) q.red[k][v] = s[v];
+          }
+        }
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(kJG) : "memory");
+        if (k == 0) {
+          double G[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+#pragma unroll
+          for (int kk = 0; kk < 6; ++kk) {
+            const double* e = q.red[kk];
+            // h = (aii - ajj, aij + conj(aij), i (aij - conj(aij))), as in k_jade_step
+            const double h0 = e[2] - e[4], h0i = e[3] - e[5], h1 = 2.0 * e[0], h2 = -2.0 * e[1];
+            G[0][0] += h0 * h0 + h0i * h0i;
+            G[0][1] += h0 * h1;
+            G[0][2] += h0 * h2;
+            G[1][1] += h1 * h1;
+            G[1][2] += h1 * h2;
+            G[2][2] += h2 * h2;
+          }
+          G[1][0] = G[0][1];
+          G[2][0] = G[0][2];
+          G[2][1] = G[1][2];
+          double v[3];
+          jacobi3_top(G, v);
+          const double x = fabs(v[0]), y = v[0] < 0.0 ? -v[1] : v[1];
+          const double r = sqrt((x + 1.0) / 2.0);
+          if (lane == 0) {
+            q.rot[0] = r;
+            q.rot[1] = y / (2.0 * r);
+            q.rot[2] = -v[2] / (2.0 * r);
+          }
+        }
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(kJG) : "memory");
+        const double c = q.rot[0];
+        const double2 sv = make_double2(q.rot[1], q.rot[2]), sc = cconj(sv);
+#pragma unroll
+        for (int t = 0; t < E; ++t) {
+          const int i = lane + 32 * t;
+          if (i >= M) continue;
+          const double2 t1 = cmul(sc, xq[t]), t2 = cmul(sv, xp[t]);
+          const double2 np_ = make_double2(c * xp[t].x + t1.x, c * xp[t].y + t1.y);
+          const double2 nq = make_double2(c * xq[t].x - t2.x, c * xq[t].y - t2.y);
+          rp[k * M + i] = np_;
+          rq[k * M + i] = nq;
+          if (k < 6 && i == pq.x) q.diag[k][0] = np_.x - xp[t].x;
+          if (k < 6 && i == pq.y) q.diag[k][1] = nq.x - xq[t].x;
+        }
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(kJG) : "memory");
+        if (threadIdx.x % kJG == 0) {
+          double d = 0.0;
+          for (int kk = 0; kk < 6; ++kk) d += q.diag[kk][0] + q.diag[kk][1];
+          delta[(size_t)st * np + pi] = d;
+        }
+      }
+    }
+    // sum over the steps of 2 |sum over the pairs of the trace change|, in the same order
+    // by every CTA, so all take the same decision
+    __threadfence();
+    cluster.sync();
+    double acc = 0.0;
+    for (int st = threadIdx.x; st < steps; st += blockDim.x) {
+      double t = 0.0;
+      for (int i = 0; i < np; ++i) t += __ldcg(delta + (size_t)st * np + i);
+      acc += 2.0 * fabs(t);
+    }
+    part[threadIdx.x] = acc;
+    __syncthreads();
+    change = 0.0;
+    for (int i = 0; i < min((int)blockDim.x, steps); ++i) change += part[i];
+    __syncthreads();
+    if (!isfinite(change) || fabs(change) < tol || nsweep >= maxsweep) break;
+  }
+  for (int e = threadIdx.x; e < mine * 7 * M; e += blockDim.x) {
+    const int i = e % M, kk = (e / M) % 7, r = rank + CL * (e / (7 * M));
+    double2* dst = kk < 6 ? a + kk * MM : u;
+    dst[(size_t)r * M + i] = rows[e];
+  }
+  if (rank == 0 && threadIdx.x == 0) {
+    out[0] = change;
+    out[1] = (double)nsweep;
+  }
+  cluster.sync();  // no CTA leaves while another may still read its rows
+}
+
 __global__ void k_identity(double2* __restrict__ u, int M) {
   for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < (long)M * M; e += (long)gridDim.x * blockDim.x)
     u[e] = make_double2((e / M == e % M) ? 1.0 : 0.0, 0.0);
@@ -450,7 +657,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 1)
   __shared__ cplx<R> sU[kRK][kRT];      // [j][i] = conj(u[i][j])
   const long p0 = (long)blockIdx.x * kRT;
   const int i0 = blockIdx.y * kRT;
-  const int tp = threadIdx.x % 16, ti = threadIdx.x / 16;
+  const int ti = threadIdx.x / 128 * 8 + threadIdx.x % 8, tp = (threadIdx.x / 32) % 4 * 4 + threadIdx.x % 32 / 8;
   cplx<R> acc[4][4];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
@@ -508,7 +715,7 @@ long gram_slabs(long N, int Ma, int Mb) {
   const long tiles = (long)((Ma + TM - 1) / TM) * ((Mb + TN - 1) / TN);
   const long chunks = (N + kGP - 1) / kGP;
   if (sizeof(T) == 4) return std::max<long>(1, (N + kSlabF32 - 1) / kSlabF32);
-  return std::max<long>(1, std::min<long>(chunks, (148L * 4 + tiles - 1) / tiles));
+  return std::max<long>(1, std::min<long>(chunks, (148L * 2 + tiles - 1) / tiles));
 }
 size_t slab_bytes(long N, int Ma, int Mb) {
   const size_t MM = (size_t)Ma * Mb;
@@ -517,9 +724,10 @@ size_t slab_bytes(long N, int Ma, int Mb) {
 }
 }  // namespace
 
-// the slabs of the larger layout, then Z [3][Ma][Mb] (FP64) at a 256-byte boundary
+// the slabs of the larger layout, then Z [3][Ma][Mb] (FP64) at a 256-byte boundary and the
+// axis tables
 size_t mlwf_partial_bytes(long N, int Ma, int Mb) {
-  return (slab_bytes(N, Ma, Mb) + 255) / 256 * 256 + 3 * (size_t)Ma * Mb * sizeof(double2);
+  return (slab_bytes(N, Ma, Mb) + 255) / 256 * 256 + (3 * (size_t)Ma * Mb + 9 * kAxisMax) * sizeof(double2);
 }
 size_t mlwf_partial_bytes(long N, int M) { return mlwf_partial_bytes(N, M, M); }
 
@@ -534,13 +742,14 @@ static int gram_impl(const void* pa, long lda, int Ma, const void* pb, long ldb,
   const long per = ((N + slabs - 1) / slabs + kGP - 1) / kGP * kGP;
   const long nslab = (N + per - 1) / per;
   const dim3 grid((unsigned)(((Ma + TM - 1) / TM) * ((Mb + TN - 1) / TN)), (unsigned)nslab);
-  k_mlwf_gram<T><<<grid, 256, 0, st>>>((const cplx<T>*)pa, lda, Ma, (const cplx<T>*)pb, ldb, Mb, N, g, per,
+  double2* Z = reinterpret_cast<double2*>(static_cast<char*>(partial) + (slab_bytes(N, Ma, Mb) + 255) / 256 * 256);
+  double2* tab = Z + 3 * (size_t)Ma * Mb;
+  k_mlwf_axis<<<9, 128, 0, st>>>(g, tab);
+  k_mlwf_gram<T><<<grid, 256, 0, st>>>((const cplx<T>*)pa, lda, Ma, (const cplx<T>*)pb, ldb, Mb, N, g, tab, per,
                                        (P*)partial);
   INQB_CUDA_TRY(cudaGetLastError());
   const long work = 3L * Ma * Mb;
-  double2* Z = reinterpret_cast<double2*>(static_cast<char*>(partial) + (slab_bytes(N, Ma, Mb) + 255) / 256 * 256);
-  k_mlwf_slab_sum<P><<<(unsigned)std::min<long>((work + 255) / 256, 148L * 32), 256, 0, st>>>((const P*)partial,
-                                                                                             (int)nslab, work, Z);
+  k_mlwf_slab_sum<P><<<(unsigned)((work + 31) / 32), 256, 0, st>>>((const P*)partial, (int)nslab, work, Z);
   INQB_CUDA_TRY(cudaGetLastError());
   *Zout = Z;
   return INQB_OK;
@@ -597,6 +806,52 @@ int launch_identity(double2* u, int M, void* stream) {
 int launch_jade_step(double2* a, double2* u, int M, const int2* pairs, int np, double* delta, void* stream) {
   k_jade_step<<<np, kJT, 0, (cudaStream_t)stream>>>(a, u, M, pairs, delta);
   INQB_CUDA_TRY(cudaGetLastError());
+  return INQB_OK;
+}
+
+template <int E, int GMAX>
+static int jade_cluster_launch(double2* a, double2* u, int M, const int2* pairs, int np, int steps, int maxsweep,
+                               double tol, double* delta, double* out, bool* done, cudaStream_t st) {
+  // sixteen CTAs (fewer pairs each) where the GPU places such a cluster, else eight
+  for (const int cl : {16, 8}) {
+    const size_t smem = (size_t)((M + cl - 1) / cl) * 7 * M * sizeof(double2);
+    if (smem > 200 * 1024) continue;
+    const int groups = std::min(GMAX, (np + cl - 1) / cl);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cl);
+    cfg.blockDim = dim3(groups * kJG);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cl;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    INQB_CUDA_TRY(cudaFuncSetAttribute(k_jade_cluster<E, GMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (cl > 8)
+      INQB_CUDA_TRY(cudaFuncSetAttribute(k_jade_cluster<E, GMAX>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, k_jade_cluster<E, GMAX>, &cfg) != cudaSuccess || fit < 1) {
+      cudaGetLastError();
+      continue;
+    }
+    INQB_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_jade_cluster<E, GMAX>, a, u, M, pairs, np, steps, maxsweep, tol, delta, out));
+    *done = true;
+    return INQB_OK;
+  }
+  return INQB_OK;
+}
+
+// All sweeps in one launch (a and u on the device; u is set, not read); done: whether the
+// matrices fit a cluster.  out[0], out[1]: the last sweep's trace change, the sweeps.
+int launch_jade_cluster(double2* a, double2* u, int M, const int2* pairs, int np, int steps, int maxsweep, double tol,
+                        double* delta, double* out, bool* done, void* stream) {
+  cudaStream_t st = (cudaStream_t)stream;
+  *done = false;
+  if (M <= 64) return jade_cluster_launch<2, 2>(a, u, M, pairs, np, steps, maxsweep, tol, delta, out, done, st);
+  if (M <= 128) return jade_cluster_launch<4, 4>(a, u, M, pairs, np, steps, maxsweep, tol, delta, out, done, st);
+  if (M <= 192) return jade_cluster_launch<6, 4>(a, u, M, pairs, np, steps, maxsweep, tol, delta, out, done, st);
   return INQB_OK;
 }
 

@@ -25,6 +25,8 @@ int launch_identity(double2* u, int M, void* stream);
 // one JADE rotation step over np pairs (int2 top, bottom; indices >= M are skipped);
 // delta[np] receives each pair's change of sum_k trace(a_k)
 int launch_jade_step(double2* a, double2* u, int M, const int2* pairs, int np, double* delta, void* stream);
+int launch_jade_cluster(double2* a, double2* u, int M, const int2* pairs, int np, int steps, int maxsweep, double tol,
+                        double* delta, double* out, bool* done, void* stream);
 int launch_jade_change(const double* delta, int nsteps, int np, double* out, void* stream);
 int launch_jade_adiag(const double2* a, const double2* u, int M, double2* adiag, void* stream);
 // out = psi u^H (out must not alias psi)

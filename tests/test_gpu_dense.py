@@ -1,6 +1,6 @@
 """The dense orbital kernels at the edges of their tiles: the overlap and rotation tiles
-(16, 32 and 64 wide) and the blocks of 32 of the Cholesky factor and its inverse, against
-numpy.
+(16, 32 and 64 wide), the blocks of 32 of the Cholesky factor and its inverse, and JADE in
+one cluster (rows spread over 16 CTAs, 2 to 6 elements a lane) against numpy and the oracle.
 
 Tolerances: a sum of n rounded FP64 products is within about sqrt(n) 1.1e-16 of its
 2-norm; the factor's condition number (below 10 for these sets) multiplies it once."""
@@ -72,3 +72,21 @@ def test_cholesky_reports_the_first_failing_pivot(pb, M, zero):
         h.orthonormalize_(x)
     assert f"pivot {zero}" in str(e.value)
     assert torch.equal(x, keep)
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 16, 17, 32, 33, 64, 65, 97, 129, 150, 190])
+def test_jade_sizes(pb, oracle_mod, M):
+    """Hermitian matrices diagonal up to a small unitary mixing: the sweeps of the oracle,
+    and its rotation to the accuracy the convergence threshold leaves."""
+    rng = np.random.default_rng(M)
+    g = 0.3 / np.sqrt(M) * (rng.standard_normal((M, M)) + 1j * rng.standard_normal((M, M)))
+    w, v = np.linalg.eigh(1j * (g - g.conj().T))
+    q = v @ np.diag(np.exp(-1j * w)) @ v.conj().T
+    a = np.stack([q @ np.diag(rng.uniform(-1, 1, M)) @ q.conj().T for _ in range(6)])
+    h = _ham(pb)
+    maxsweep = 100 if M < 100 else 2  # the CPU oracle multiplies dense rotations
+    u, adiag, sweeps = h.jade(torch.as_tensor(a).cuda(), maxsweep, 1e-8)
+    _, u_ref, d_ref, sw_ref = oracle_mod.jade(a, maxsweep, 1e-8)
+    assert sweeps == sw_ref
+    assert np.abs(u.cpu().numpy() - u_ref).max() < 1e-10
+    assert np.abs(adiag.cpu().numpy() - d_ref).max() < 1e-10
