@@ -65,9 +65,10 @@ __device__ __forceinline__ void run_stage(const BatchCell<T>& c, int bx, int by,
     constexpr int G = TileGeom<T, N, N, N>::G;
     const int m0 = bx * G;
     const int n = c.pj.nproj * c.pj.L * G;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      const int m = m0 + i % G;
-      if (m < c.M) proj_finish_item(c.pj, c.M, c.ysplit, (long)(i / G) * c.M + m);
+    for (int t = 0; finish_item(t) < n; t += blockDim.x) {
+      const int i = (int)finish_item(t + threadIdx.x), m = m0 + i % G;
+      const bool on = i < n && m < c.M;
+      proj_finish_item(c.pj, c.M, c.ysplit, on ? (unsigned)(i / G) * c.M + m : 0u, on);
     }
   } else if (STAGE == kStageB) {
     for (int t = 0; t < count; t++) {
@@ -78,7 +79,7 @@ __device__ __forceinline__ void run_stage(const BatchCell<T>& c, int bx, int by,
     for (int t = 0; t < count; t++) {
       if (t) __syncthreads();
       tile_inv_body<T, N, N, N, 1>(bx, by + t, c.tmp, c.in, c.ld_in, c.out, c.ld_out, c.M, twy, twz, c.pj, c.ep,
-                                   c.rec_cap_inv, c.seg_cap, c.vio);
+                                   c.seg_cap, c.vio);
     }
   }
 }

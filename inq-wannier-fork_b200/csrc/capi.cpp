@@ -65,20 +65,17 @@ ProjView<T> proj_view(inqb_ctx* ctx) {
   v.max_plane_atoms = t.max_plane_atoms;
   v.max_tile_ent = t.max_tile_ent;
   v.max_tile_seg = t.max_tile_seg;
-  v.pt_stride = t.pt_stride;
+  v.tile_pts = t.tile_pts;
   v.ent_rec = t.d_ent_rec.as<EntRec<T>>();
-  v.ent_rec_pt = t.d_ent_rec_pt.as<EntRec<T>>();
-  v.pt_ptr = t.d_pt_ptr.as<int>();
+  v.ent_rec_rk = t.d_ent_rec_rk.as<EntRec<T>>();
+  v.rk_ptr = t.d_rk_ptr.as<int>();
+  v.rk_start = t.d_rk_start.as<int>();
   v.seg_ptr = t.d_seg_ptr.as<int>();
   v.seg_atom = t.d_seg_atom.as<int>();
   v.seg_ent = t.d_seg_ent.as<int>();
-  v.ent_off = t.d_ent_off.as<int>();
-  v.ent_atom = t.d_ent_atom.as<int>();
   v.seg_local = t.d_seg_local.as<int>();
   v.plane_ptr = t.d_plane_ptr.as<int>();
   v.plane_atom = t.d_plane_atom.as<int>();
-  v.ent_beta = t.d_ent_beta.as<T>();
-  v.ent_phase = t.d_ent_phase.ptr;
   v.scale = t.d_scale.as<double>();
   v.proj = ctx->d_projacc.as<double2>();
   v.pc_ptr = t.d_pc_ptr.as<int>();
@@ -112,9 +109,8 @@ int reserve(inqb_ctx* ctx, int M) {
 int update_phases(inqb_ctx* ctx, void* stream) {
   if (ctx->proj.nproj == 0 || ctx->proj.nent == 0) return INQB_OK;
   INQB_TRY(launch_phases(ctx->precision, ctx->proj.nent, ctx->proj.d_ent_relpos.as<float>(), ctx->kA_cov,
-                         ctx->proj.d_ent_phase.ptr, ctx->proj.d_ent_rec.ptr, ctx->proj.d_ent_rec_pt.ptr,
-                         ctx->proj.d_pt_pos.as<int>(), ctx->proj.d_adj_rec.ptr, ctx->proj.d_atom_pos.as<int>(),
-                         stream));
+                         ctx->proj.d_ent_rec.ptr, ctx->proj.d_ent_rec_rk.ptr, ctx->proj.d_rk_pos.as<int>(),
+                         ctx->proj.d_adj_rec.ptr, ctx->proj.d_atom_pos.as<int>(), stream));
   return launch_project_table(ctx->precision, ctx->proj.pc_chunks, ctx->proj.d_pc_relpos.as<float>(),
                               ctx->proj.d_pc_beta.as<double>(), ctx->kA_cov, ctx->proj.d_pc_table.ptr, stream);
 }
@@ -166,11 +162,10 @@ int apply(inqb_ctx* ctx, int mode, const void* in, long ld_in, void* out, long l
     a.ysplit = sched->second[0];
     for (int k = 0; k < 3; k++) a.threads[k] = sched->second[1 + k];
   }
-  // the fused projection's partial sums: one [4][M] slot per (plane, atom, half)
-  if (mode == LaunchArgs::H && ctx->proj.nproj > 0 && ctx->proj_mode == INQB_PROJECTION_FUSED) {
-    const int ys = a.ysplit > 0 ? a.ysplit : ctx->plan->ysplit;
-    INQB_TRY(ctx->d_slots.ensure(sizeof(double2) * (size_t)ctx->proj.aslot.size() * ys * 4 * M));
-  }
+  if (a.ysplit <= 0) a.ysplit = ctx->plan->ysplit;
+  // the fused projection's partial sums: one [4][M] slot per (plane, atom, CTA of the plane)
+  if (mode == LaunchArgs::H && ctx->proj.nproj > 0 && ctx->proj_mode == INQB_PROJECTION_FUSED)
+    INQB_TRY(ctx->d_slots.ensure(sizeof(double2) * (size_t)ctx->proj.aslot.size() * a.ysplit * 4 * M));
   if (ctx->timing_on && mode == LaunchArgs::H && !batch_cell && ctx->timing_count < ctx->timing_capacity) {
     for (int i = 0; i < 6; i++) a.events[i] = ctx->timing_events[6 * ctx->timing_count + i];
     ctx->timing_count++;

@@ -36,23 +36,30 @@ struct Axis {
   __host__ __device__ static constexpr int slot_of_freq(int k) { return at(k % N1, k / N1); }
 };
 
-// Twiddle table layout in shared memory: tw[k1 * N2 + j2] = exp(-2 pi i j2 k1 / N).
-template <typename A, bool INV, typename T>
-__device__ __forceinline__ cplx<T> twiddle(cplx<T> v, const cplx<T>* tw, int k1, int j2) {
-  cplx<T> w = tw[k1 * A::N2 + j2];
-  return INV ? mul_conj(v, w) : v * w;
+// Twiddle table layout in shared memory: tw[k1 * N2 + j2] = exp(-2 pi i j2 k1 / N), as
+// lanes (the value for both orbitals of a lane).
+template <typename A, bool INV, typename P>
+__device__ __forceinline__ cplx<P> twiddle(cplx<P> v, const cplx<P>* tw, int k1, int j2) {
+  const cplx<P> w = tw[k1 * A::N2 + j2];
+  return INV ? lmul_conj(v, w) : lmul(v, w);
 }
 
 // Step 1 (forward or inverse-from-natural when INV): items map to (base, es, j2).
-template <typename A, bool INV, typename T, typename Map>
-__device__ __forceinline__ void step1(cplx<T>* S, int nitems, const cplx<T>* tw, Map map) {
+// ORB: the tile holds orbital-layout values (as copied from an orbital block); they are
+// put into the lane layout here.
+template <typename A, bool INV, bool ORB = false, typename P, typename Map>
+__device__ __forceinline__ void step1(cplx<P>* S, int nitems, const cplx<P>* tw, Map map) {
   for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
     int base, es, j2;
     map(it, base, es, j2);
-    cplx<T> v[A::N1];
+    cplx<P> v[A::N1];
 #pragma unroll
     for (int j1 = 0; j1 < A::N1; ++j1) v[j1] = S[base + A::at(j1, j2) * es];
-    DFT<A::N1, INV, T>::run(v);
+    if (ORB) {
+#pragma unroll
+      for (int j1 = 0; j1 < A::N1; ++j1) v[j1] = flip(v[j1]);
+    }
+    DFT<A::N1, INV, P>::run(v);
     if (A::N2 > 1) {
 #pragma unroll
       for (int k1 = 1; k1 < A::N1; ++k1) v[k1] = twiddle<A, INV>(v[k1], tw, k1, j2);
@@ -63,16 +70,16 @@ __device__ __forceinline__ void step1(cplx<T>* S, int nitems, const cplx<T>* tw,
 }
 
 // Step 2 (forward / inverse-from-natural): items map to (base, es, k1).
-template <typename A, bool INV, typename T, typename Map>
-__device__ __forceinline__ void step2(cplx<T>* S, int nitems, Map map) {
+template <typename A, bool INV, typename P, typename Map>
+__device__ __forceinline__ void step2(cplx<P>* S, int nitems, Map map) {
   if (A::N2 == 1) return;
   for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
     int base, es, k1;
     map(it, base, es, k1);
-    cplx<T> v[A::N2];
+    cplx<P> v[A::N2];
 #pragma unroll
     for (int j2 = 0; j2 < A::N2; ++j2) v[j2] = S[base + A::at(k1, j2) * es];
-    DFT<A::N2, INV, T>::run(v);
+    DFT<A::N2, INV, P>::run(v);
 #pragma unroll
     for (int k2 = 0; k2 < A::N2; ++k2) S[base + A::at(k1, k2) * es] = v[k2];
   }
@@ -81,16 +88,16 @@ __device__ __forceinline__ void step2(cplx<T>* S, int nitems, Map map) {
 // Step 2' of the inverse from transposed order: inverse DFT_N2 over k2 then the
 // conjugate twiddle; `pre` is applied to the frequency-domain values first
 // (pre(k, value) with k = k1 + N1 k2), which fuses a pointwise operator.
-template <typename A, typename T, typename Map, typename Pre>
-__device__ __forceinline__ void step2_inv_transposed(cplx<T>* S, int nitems, const cplx<T>* tw, Map map,
+template <typename A, typename P, typename Map, typename Pre>
+__device__ __forceinline__ void step2_inv_transposed(cplx<P>* S, int nitems, const cplx<P>* tw, Map map,
                                                      Pre pre) {
   for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
     int base, es, k1;
     map(it, base, es, k1);
-    cplx<T> v[A::N2];
+    cplx<P> v[A::N2];
 #pragma unroll
     for (int k2 = 0; k2 < A::N2; ++k2) v[k2] = pre(it, k1 + A::N1 * k2, S[base + A::at(k1, k2) * es]);
-    DFT<A::N2, true, T>::run(v);
+    DFT<A::N2, true, P>::run(v);
     if (A::N2 > 1) {
 #pragma unroll
       for (int j2 = 0; j2 < A::N2; ++j2)
@@ -103,18 +110,18 @@ __device__ __forceinline__ void step2_inv_transposed(cplx<T>* S, int nitems, con
 
 // Forward step 2 fused with a pointwise operator and the inverse step 2'
 // (the kinetic multiply of H between a forward and an inverse transform).
-template <typename A, typename T, typename Map, typename Op>
-__device__ __forceinline__ void step2_fwd_op_inv(cplx<T>* S, int nitems, const cplx<T>* tw, Map map, Op op) {
+template <typename A, typename P, typename Map, typename Op>
+__device__ __forceinline__ void step2_fwd_op_inv(cplx<P>* S, int nitems, const cplx<P>* tw, Map map, Op op) {
   for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
     int base, es, k1;
     map(it, base, es, k1);
-    cplx<T> v[A::N2];
+    cplx<P> v[A::N2];
 #pragma unroll
     for (int j2 = 0; j2 < A::N2; ++j2) v[j2] = S[base + A::at(k1, j2) * es];
-    DFT<A::N2, false, T>::run(v);
+    DFT<A::N2, false, P>::run(v);
 #pragma unroll
     for (int k2 = 0; k2 < A::N2; ++k2) v[k2] = op(it, k1 + A::N1 * k2, v[k2]);
-    DFT<A::N2, true, T>::run(v);
+    DFT<A::N2, true, P>::run(v);
     if (A::N2 > 1) {
 #pragma unroll
       for (int j2 = 0; j2 < A::N2; ++j2)
@@ -126,15 +133,15 @@ __device__ __forceinline__ void step2_fwd_op_inv(cplx<T>* S, int nitems, const c
 }
 
 // Step 1' of the inverse from transposed order: inverse DFT_N1 over k1, natural out.
-template <typename A, typename T, typename Map>
-__device__ __forceinline__ void step1_inv_transposed(cplx<T>* S, int nitems, Map map) {
+template <typename A, typename P, typename Map>
+__device__ __forceinline__ void step1_inv_transposed(cplx<P>* S, int nitems, Map map) {
   for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
     int base, es, j2;
     map(it, base, es, j2);
-    cplx<T> v[A::N1];
+    cplx<P> v[A::N1];
 #pragma unroll
     for (int k1 = 0; k1 < A::N1; ++k1) v[k1] = S[base + A::at(k1, j2) * es];
-    DFT<A::N1, true, T>::run(v);
+    DFT<A::N1, true, P>::run(v);
 #pragma unroll
     for (int j1 = 0; j1 < A::N1; ++j1) S[base + A::at(j1, j2) * es] = v[j1];
   }

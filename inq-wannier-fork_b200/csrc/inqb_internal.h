@@ -72,7 +72,7 @@ struct DevBuf {
 };
 
 // One sphere entry as the H tiles read it: exp(+i (k+A).r), the KB radial values
-// (zero past L) and the tile-local offset (row * NZ + z), padded to whole
+// (zero past L) and the point's slot in the tile's shared-memory rows, padded to whole
 // 16-byte vectors so a tile's run of entries is copied with cp.async.
 template <typename T>
 struct alignas(16) EntRec {
@@ -132,16 +132,19 @@ struct ProjTables {
   DevBuf d_aslot_ptr, d_aslot;
   DevBuf d_adj_rec, d_atom_pos;     // [nent] AdjRec<T> in atom-major order
   // device copies
-  DevBuf d_seg_ptr, d_seg_atom, d_seg_ent, d_seg_local, d_plane_ptr, d_plane_atom, d_ent_off, d_ent_atom;
-  DevBuf d_ent_beta;                // [nent][L] in the context precision
+  DevBuf d_seg_ptr, d_seg_atom, d_seg_ent, d_seg_local, d_plane_ptr, d_plane_atom;
   DevBuf d_ent_relpos;              // [nent][3] float
-  DevBuf d_ent_phase;               // [nent] complex, exp(+i (k+A).r), context precision
-  DevBuf d_ent_rec;                 // [nent] EntRec<T>, phases filled with d_ent_phase
-  // the same records in point order inside each tile (for the owner-computes
-  // nonlocal scatter): rec_pt[pt_pos[e]] is entry e; pt_ptr[tile * pt_stride + q]
-  // is the first record of tile-local point q relative to the tile's first entry
+  DevBuf d_ent_rec;                 // [nent] EntRec<T>, phases filled for each k + A
+  // point order inside each tile: pt_pos[e] is the place of entry e, and
+  // pt_ptr[tile * pt_stride + q] the first place of tile-local point q relative to the
+  // tile's first entry
   std::vector<int> pt_pos, pt_ptr;
-  DevBuf d_ent_rec_pt, d_pt_pos, d_pt_ptr;
+  // rank order inside each tile, the records' order of the nonlocal scatter: first the
+  // first entry of every point, then the second entries, and so on, so
+  // that the entries of one rank touch different points.  rk_pos[e] is the place of entry
+  // e; tile t's ranks are rk_start[k] .. rk_start[k + 1] for rk_ptr[t] <= k < rk_ptr[t + 1].
+  std::vector<int> rk_pos, rk_ptr, rk_start;
+  DevBuf d_ent_rec_rk, d_rk_pos, d_rk_ptr, d_rk_start;
   DevBuf d_scale;                   // [nproj][L] double
   DevBuf d_atom_ptr, d_atom_ent, d_ent_pt, d_ent_xyz;
   DevBuf d_chunk_atom, d_chunk_beg, d_atom_chunk_ptr;
@@ -150,20 +153,17 @@ struct ProjTables {
 // Kernel view of the projector tables (T = float or double).
 template <typename T>
 struct ProjView {
-  int nproj, L, max_plane_atoms, max_tile_ent, max_tile_seg, pt_stride;
+  int nproj, L, max_plane_atoms, max_tile_ent, max_tile_seg, tile_pts;
   const int* seg_ptr;     // [NX * Y1 + 1] segments of tile (ix, y1)
   const int* seg_atom;
   const int* seg_ent;     // [nseg + 1] entry ranges
   const int* seg_local;   // plane-local atom index of a segment
   const int* plane_ptr;   // [NX + 1] atoms of plane ix
   const int* plane_atom;
-  const int* ent_off;     // tile-local (row * NZ + z)
-  const int* ent_atom;
-  const T* ent_beta;
-  const void* ent_phase;  // cplx<T>*
   const EntRec<T>* ent_rec;     // segment (atom) order
-  const EntRec<T>* ent_rec_pt;  // point order inside each tile
-  const int* pt_ptr;            // [tiles][pt_stride]
+  const EntRec<T>* ent_rec_rk;  // rank order inside each tile
+  const int* rk_ptr;            // [NX * Y1 + 1] ranks of a tile
+  const int* rk_start;          // first record of each rank
   const double* scale;
   double2* proj;          // [nproj][L][M] accumulators (FP64 in both precisions)
   // the projection kernels' chunk tables (project.h)

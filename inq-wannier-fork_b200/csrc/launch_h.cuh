@@ -85,8 +85,8 @@ struct BatchCell {
   long ld_in;
   cplx<T>* out;
   long ld_out;
-  int M, ysplit, acc_cap, rec_cap_a, rec_cap_inv, seg_cap, vin, vio;
-  cplx<T>* tmp;
+  int M, ysplit, acc_cap, rec_cap_a, seg_cap, vin, vio;
+  Lane<T>* tmp;
   const cplx<T>* tw;  // x | y | z twiddles
   ProjView<T> pj;
   KinParams<T> kp;
@@ -102,6 +102,24 @@ namespace inqb {
 // ---------------------------------------------------------------- launch
 inline bool aligned16(const void* p, long ld, size_t esz) {
   return ((uintptr_t)p % 16 == 0) && ((ld * (long)esz) % 16 == 0);
+}
+
+// A launch that may be scheduled while the launch before it on the stream drains; the
+// kernel waits (chain_wait, tiles.cuh) before it reads what that one wrote.
+template <typename... K, typename... A>
+int launch_chained(void (*kernel)(K...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  INQB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...));
+  return INQB_OK;
 }
 
 template <typename T, int NX, int NY, int NZ>
@@ -126,9 +144,9 @@ int launch_h_impl(const LaunchArgs& a) {
       INQB_CUDA_TRY(cudaFuncSetAttribute(k_tile_x_fft<T, NX, NY, NZ, 1>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TG::SMEM_X));
       INQB_CUDA_TRY(cudaFuncSetAttribute(k_tile_inv<T, NX, NY, NZ, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)std::min(TG::smem_inv(kRecCapMax, kAccAtomsMax), TG::SMEM_MAX)));
+                                         (int)std::min(TG::smem_inv(kSegMax), TG::SMEM_MAX)));
       INQB_CUDA_TRY(cudaFuncSetAttribute(k_tile_inv<T, NX, NY, NZ, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)TG::smem_inv(0, 0)));
+                                         (int)TG::smem_inv(0)));
       return (int)INQB_OK;
     }();
   });
@@ -137,18 +155,17 @@ int launch_h_impl(const LaunchArgs& a) {
   const cplx<T>* twx = tw;
   const cplx<T>* twy = tw + NX;
   const cplx<T>* twz = tw + NX + NY;
-  cplx<T>* tmp = reinterpret_cast<cplx<T>*>(a.tmp);
+  Lane<T>* tmp = reinterpret_cast<Lane<T>*>(a.tmp);
   cudaStream_t st = (cudaStream_t)a.stream;
   const size_t esz = sizeof(cplx<T>);
   const int tgroups = (a.M + GT - 1) / GT;
   // 16-byte vectors of G orbitals: full groups, aligned pointers and leading dimensions
   const int vin = aligned16(a.in, a.ld_in, esz);
   const int vout = aligned16(a.out, a.ld_out, esz);
+  const int vbase = a.base && aligned16(a.base, a.ld_base, esz);
   int ysplit = a.ysplit > 0 ? a.ysplit : TG::YSPLIT;
   if (TG::Y1 % ysplit != 0) return fail(INQB_ERR_INVALID, "schedule: ysplit must divide the tiles per plane");
-  // compiled defaults: 256 threads per CTA, except the x-line pass in FP64, which the
-  // autotuner measured faster with 128 (64^3: 295 -> 258 us)
-  const int thr_default[3] = {TG::THREADS, sizeof(T) == 8 ? 128 : TG::THREADS, TG::THREADS};
+  const int thr_default[3] = {TG::THREADS, TG::X_THREADS, TG::Z_THREADS};
   int thr[3];
   for (int k = 0; k < 3; k++) {
     thr[k] = a.threads[k] > 0 ? a.threads[k] : thr_default[k];
@@ -179,15 +196,16 @@ int launch_h_impl(const LaunchArgs& a) {
                      project_supported(sizeof(T) == 8 ? INQB_FP64 : INQB_MIXED, a.in, a.ld_in);
     ProjView<T> pjA = pj;
     if (sep) pjA.nproj = 0;
-    const int acc_cap = pjA.nproj > 0 ? std::min(pj.max_plane_atoms, kAccAtomsMax) : 0;
-    const int seg_cap = pj.nproj > 0 ? std::min(pj.max_tile_seg, kAccAtomsMax) : 0;
+    // accumulators for as many of a plane's atoms as fit beside the tile
+    int acc_cap = pjA.nproj > 0 ? std::min(pj.max_plane_atoms, kAccAtomsMax) : 0;
+    while (acc_cap > 0 && TG::smem_fwd(acc_cap, 0) > TG::SMEM_MAX) acc_cap--;
     // stage a tile's records only when all of them fit beside the tile (the kernel
     // reads them from global memory otherwise)
-    int rec_cap = (pj.nproj > 0 && pj.max_tile_ent <= kRecCapMax) ? pj.max_tile_ent : 0;
-    const int rec_cap_fwd = pjA.nproj > 0 ? rec_cap : 0;
-    if (TG::smem_fwd(acc_cap, rec_cap) > TG::SMEM_MAX) rec_cap = 0;
-    const int rec_cap_a = (TG::smem_fwd(acc_cap, rec_cap_fwd) > TG::SMEM_MAX) ? 0 : rec_cap_fwd;
-    if (pj.nproj > 0 && pj.pt_stride != TG::PSTRIDE)
+    int rec_cap_a = (pjA.nproj > 0 && pj.max_tile_ent <= kRecCapMax) ? pj.max_tile_ent : 0;
+    if (TG::smem_fwd(acc_cap, rec_cap_a) > TG::SMEM_MAX) rec_cap_a = 0;
+    int seg_cap = pj.nproj > 0 ? std::min(pj.max_tile_seg, kSegMax) : 0;
+    while (seg_cap > 0 && TG::smem_inv(seg_cap) > TG::SMEM_MAX) seg_cap--;
+    if (pj.nproj > 0 && pj.tile_pts != TG::PTS)
       return fail(INQB_ERR_INVALID, "projector tables were built for another tiling of this grid");
     EpiParams<T> ep;
     ep.V = (const T*)a.V;
@@ -196,12 +214,7 @@ int launch_h_impl(const LaunchArgs& a) {
     ep.ld_base = a.ld_base;
     ep.alpha = mk<T>((T)a.alpha[0], (T)a.alpha[1]);
     ep.beta = mk<T>((T)a.beta[0], (T)a.beta[1]);
-    // pass C stages the records in shared memory only in FP64 (where the orbital
-    // prefetch already limits it to two CTAs per SM); in FP32 the smem is worth more
-    // as a fourth CTA per SM, and the epilogue prefetches records into registers
-    int rec_cap_inv = TG::PREFETCH ? rec_cap : 0;
-    if (TG::smem_inv(rec_cap_inv, seg_cap) > TG::SMEM_MAX) rec_cap_inv = 0;
-    if (TG::smem_inv(rec_cap_inv, seg_cap) > TG::SMEM_MAX)
+    if (TG::smem_inv(seg_cap) > TG::SMEM_MAX)
       return fail(INQB_ERR_UNSUPPORTED, "tile of this grid does not fit in shared memory");
     if (a.batch_cell) {
       // describe the apply for the persistent batch launch instead of launching it
@@ -219,7 +232,6 @@ int launch_h_impl(const LaunchArgs& a) {
       c.ysplit = ysplit;
       c.acc_cap = acc_cap;
       c.rec_cap_a = rec_cap_a;
-      c.rec_cap_inv = rec_cap_inv;
       c.seg_cap = seg_cap;
       c.vin = vin;
       c.vio = vin && vout;
@@ -233,7 +245,7 @@ int launch_h_impl(const LaunchArgs& a) {
       d->b_per = TG::Y2 * NZ;
       d->c_per = NX * TG::Y1;
       d->finish = pj.nproj > 0 ? 1 : 0;
-      d->smem = std::max({TG::smem_fwd(acc_cap, rec_cap_a), TG::SMEM_X, TG::smem_inv(rec_cap_inv, seg_cap)});
+      d->smem = std::max({TG::smem_fwd(acc_cap, rec_cap_a), TG::SMEM_X, TG::smem_inv(seg_cap)});
       d->bytes.resize(sizeof(c));
       memcpy(d->bytes.data(), &c, sizeof(c));
       return INQB_OK;
@@ -247,19 +259,19 @@ int launch_h_impl(const LaunchArgs& a) {
     }
     if (a.events[1]) INQB_CUDA_TRY(cudaEventRecord((cudaEvent_t)a.events[1], st));
     if (a.events[2]) INQB_CUDA_TRY(cudaEventRecord((cudaEvent_t)a.events[2], st));
-    k_tile_fwd<T, NX, NY, NZ><<<gfwd, thr[0], TG::smem_fwd(acc_cap, rec_cap_a), st>>>(
-        (const cplx<T>*)a.in, a.ld_in, a.M, tmp, twy, twz, pjA, acc_cap, rec_cap_a, ysplit, vin);
+    INQB_TRY(launch_chained(k_tile_fwd<T, NX, NY, NZ>, gfwd, thr[0], TG::smem_fwd(acc_cap, rec_cap_a), st,
+            (const cplx<T>*)a.in, a.ld_in, a.M, tmp, twy, twz, pjA, acc_cap, rec_cap_a, ysplit, vin));
     if (a.events[3]) INQB_CUDA_TRY(cudaEventRecord((cudaEvent_t)a.events[3], st));
     // the second pass also adds the fused projection's partial sums per atom, in a
     // fixed order (its first CTAs; the third pass reads the result)
     ProjView<T> fin = pj;
     if (sep || pj.nproj == 0) fin.slots = nullptr;
-    k_tile_x<T, NX, NY, NZ><<<gx, thr[1], TG::SMEM_X, st>>>(tmp, twx, kp, (cplx<T>*)a.fourier_out, fin, a.M,
-                                                             ysplit);
+    INQB_TRY(launch_chained(k_tile_x<T, NX, NY, NZ>, gx, thr[1], TG::SMEM_X, st, tmp, twx, kp,
+            (cplx<T>*)a.fourier_out, fin, a.M, ysplit));
     if (a.events[4]) INQB_CUDA_TRY(cudaEventRecord((cudaEvent_t)a.events[4], st));
-    k_tile_inv<T, NX, NY, NZ, 1><<<ginv, thr[2], TG::smem_inv(rec_cap_inv, seg_cap), st>>>(
-        tmp, (const cplx<T>*)a.in, a.ld_in, (cplx<T>*)a.out, a.ld_out, a.M, twy, twz, pj, ep, rec_cap_inv, seg_cap,
-        vin && vout);
+    INQB_TRY(launch_chained(k_tile_inv<T, NX, NY, NZ, 1>, ginv, thr[2], TG::smem_inv(seg_cap), st, tmp,
+            (const cplx<T>*)a.in, a.ld_in, (cplx<T>*)a.out, a.ld_out, a.M, twy, twz, pj, ep, seg_cap,
+            (vin && vout) | (vbase << 1)));
     if (a.events[5]) INQB_CUDA_TRY(cudaEventRecord((cudaEvent_t)a.events[5], st));
   } else if (a.mode == LaunchArgs::POISSON) {
     // solvers::poisson on M complex fields: forward z and inner y, then the outer y
@@ -267,8 +279,8 @@ int launch_h_impl(const LaunchArgs& a) {
     // the factor holds it)
     ProjView<T> none = pj;
     none.nproj = 0;
-    k_tile_fwd<T, NX, NY, NZ><<<gfwd, thr[0], TG::smem_fwd(0, 0), st>>>(
-        (const cplx<T>*)a.in, a.ld_in, a.M, tmp, twy, twz, none, 0, 0, ysplit, vin);
+    INQB_TRY(launch_chained(k_tile_fwd<T, NX, NY, NZ>, gfwd, thr[0], TG::smem_fwd(0, 0), st, (const cplx<T>*)a.in,
+            a.ld_in, a.M, tmp, twy, twz, none, 0, 0, ysplit, vin));
     KinParams<T> kq = kp;
     for (int d = 0; d < 3; d++) kq.kA[d] = (T)0;
     kq.scale = (T)1;
@@ -277,27 +289,27 @@ int launch_h_impl(const LaunchArgs& a) {
     kq.pois = (T)(2.0 * M_PI / ((double)NX * NY * NZ));
     ProjView<T> nofin = pj;
     nofin.slots = nullptr;
-    k_tile_x<T, NX, NY, NZ><<<gx, thr[1], TG::SMEM_X, st>>>(tmp, twx, kq, nullptr, nofin, 0, 1);
+    INQB_TRY(launch_chained(k_tile_x<T, NX, NY, NZ>, gx, thr[1], TG::SMEM_X, st, tmp, twx, kq, nullptr, nofin, 0, 1));
     EpiParams<T> ep{};
     ep.alpha = mk<T>((T)1, (T)0);
-    k_tile_inv<T, NX, NY, NZ, 0><<<ginv, thr[2], TG::smem_inv(0, 0), st>>>(
-        tmp, nullptr, 0, (cplx<T>*)a.out, a.ld_out, a.M, twy, twz, none, ep, 0, 0, vout);
+    INQB_TRY(launch_chained(k_tile_inv<T, NX, NY, NZ, 0>, ginv, thr[2], TG::smem_inv(0), st, tmp, nullptr, 0,
+            (cplx<T>*)a.out, a.ld_out, a.M, twy, twz, none, ep, 0, vout));
   } else if (a.mode == LaunchArgs::FFT_FWD) {
     ProjView<T> none = pj;
     none.nproj = 0;
-    k_tile_fwd<T, NX, NY, NZ><<<gfwd, thr[0], TG::smem_fwd(0, 0), st>>>(
-        (const cplx<T>*)a.in, a.ld_in, a.M, tmp, twy, twz, none, 0, 0, ysplit, vin);
-    k_tile_x_fft<T, NX, NY, NZ, 0><<<gx, thr[1], TG::SMEM_X, st>>>(tmp, nullptr, (cplx<T>*)a.out, a.ld_out,
-                                                                       a.M, twx, vout);
+    INQB_TRY(launch_chained(k_tile_fwd<T, NX, NY, NZ>, gfwd, thr[0], TG::smem_fwd(0, 0), st, (const cplx<T>*)a.in,
+            a.ld_in, a.M, tmp, twy, twz, none, 0, 0, ysplit, vin));
+    INQB_TRY(launch_chained(k_tile_x_fft<T, NX, NY, NZ, 0>, gx, thr[1], TG::SMEM_X, st, tmp, nullptr,
+            (cplx<T>*)a.out, a.ld_out, a.M, twx, vout));
   } else {
-    k_tile_x_fft<T, NX, NY, NZ, 1><<<gx, thr[1], TG::SMEM_X, st>>>(tmp, (const cplx<T>*)a.in, nullptr, a.ld_in,
-                                                                       a.M, twx, vin);
+    INQB_TRY(launch_chained(k_tile_x_fft<T, NX, NY, NZ, 1>, gx, thr[1], TG::SMEM_X, st, tmp, (const cplx<T>*)a.in,
+            nullptr, a.ld_in, a.M, twx, vin));
     EpiParams<T> ep{};
     ep.alpha = mk<T>(kp.scale, (T)0);
     ProjView<T> none = pj;
     none.nproj = 0;
-    k_tile_inv<T, NX, NY, NZ, 0><<<ginv, thr[2], TG::smem_inv(0, 0), st>>>(
-        tmp, nullptr, 0, (cplx<T>*)a.out, a.ld_out, a.M, twy, twz, none, ep, 0, 0, vout);
+    INQB_TRY(launch_chained(k_tile_inv<T, NX, NY, NZ, 0>, ginv, thr[2], TG::smem_inv(0), st, tmp, nullptr, 0,
+            (cplx<T>*)a.out, a.ld_out, a.M, twy, twz, none, ep, 0, vout));
   }
   INQB_CUDA_TRY(cudaGetLastError());
   return INQB_OK;

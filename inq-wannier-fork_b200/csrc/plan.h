@@ -51,7 +51,7 @@ struct Plan {
 };
 
 const Plan* find_plan(int nx, int ny, int nz, int precision);
-int launch_phases(int precision, int nent, const float* relpos, const double kA[3], void* phase, void* rec,
-                  void* rec_pt, const int* pt_pos, void* adj, const int* atom_pos, void* stream);
+int launch_phases(int precision, int nent, const float* relpos, const double kA[3], void* rec, void* rec_rk,
+                  const int* rk_pos, void* adj, const int* atom_pos, void* stream);
 
 }  // namespace inqb

@@ -304,6 +304,36 @@ int build_proj_tables(const inqb_ctx& ctx, int nproj, int L, int smax, const int
     std::vector<int> fill(tp, tp + t.tile_pts);
     for (int e = e0; e < e1; e++) t.pt_pos[e] = e0 + fill[t.ent_off[e]]++;
   }
+  // rank order inside each tile: an entry's rank is its place among its point's entries;
+  // within a rank the entries keep their (atom, point) order
+  t.rk_pos.assign(total, 0);
+  t.rk_ptr.assign(ntile + 1, 0);
+  t.rk_start.clear();
+  {
+    std::vector<int> count;
+    for (int tile = 0; tile < ntile; tile++) {
+      const int e0 = t.seg_ent[t.seg_ptr[tile]], e1 = t.seg_ent[t.seg_ptr[tile + 1]];
+      const int* tp = &t.pt_ptr[(size_t)tile * t.pt_stride];
+      t.rk_ptr[tile] = (int)t.rk_start.size();
+      count.clear();
+      for (int e = e0; e < e1; e++) {
+        const int r = t.pt_pos[e] - e0 - tp[t.ent_off[e]];
+        if (r >= (int)count.size()) count.resize(r + 1, 0);
+        t.rk_pos[e] = r;
+        count[r]++;
+      }
+      int at = e0;
+      for (int& c : count) {
+        t.rk_start.push_back(at);
+        const int n = c;
+        c = at;
+        at += n;
+      }
+      for (int e = e0; e < e1; e++) t.rk_pos[e] = count[t.rk_pos[e]]++;
+    }
+    t.rk_ptr[ntile] = (int)t.rk_start.size();
+    t.rk_start.push_back((int)total);
+  }
   // grid point of every entry, in entry order
   std::vector<long> pt_of(total);
   {
@@ -387,17 +417,25 @@ static int upload(DevBuf& b, const std::vector<T>& v) {
 }
 
 // Entry records with zero phases (the phase kernel fills them for each k + A).
-// point_order: record e goes to pt_pos[e] instead of e.
+// rank_order: record e goes to rk_pos[e] instead of e.  The records' offset is the
+// point's slot in the tile's shared-memory rows (Axis in fft_tile.cuh: an n1 x n2 four-step
+// view of the z axis, rows of n2 padded by one slot for even n2): natural order for the
+// projection in the first pass, the transposed order that the inverse transform leaves for
+// the scatter in the third (rank order).
 template <typename T>
-static std::vector<EntRec<T>> ent_records(const ProjTables& t, bool point_order = false) {
+static std::vector<EntRec<T>> ent_records(const ProjTables& t, int nz, bool rank_order = false) {
   std::vector<EntRec<T>> rec((size_t)t.nent);
+  int n1 = 1, n2 = nz;
+  split_of(nz, &n1, &n2);
+  const int row = n2 + ((n2 % 2 == 0 && n2 > 1) ? 1 : 0), zs = n1 * row;
   for (int tile = 0; tile + 1 < (int)t.seg_ptr.size(); tile++)
     for (int s = t.seg_ptr[tile]; s < t.seg_ptr[tile + 1]; s++)
       for (int e = t.seg_ent[s]; e < t.seg_ent[s + 1]; e++) {
-        EntRec<T>& r = rec[point_order ? t.pt_pos[e] : e];
+        EntRec<T>& r = rec[rank_order ? t.rk_pos[e] : e];
         r.ph[0] = r.ph[1] = (T)0;
         for (int l = 0; l < 4; l++) r.beta[l] = (l < t.L) ? (T)t.ent_beta[(size_t)e * t.L + l] : (T)0;
-        r.off = t.ent_off[e];
+        const int y = t.ent_off[e] / nz, z = t.ent_off[e] % nz;
+        r.off = y * zs + (rank_order ? (z % n1) * row + z / n1 : (z / n2) * row + z % n2);
         r.tseg = s - t.seg_ptr[tile];
       }
   return rec;
@@ -422,8 +460,6 @@ int upload_proj_tables(const inqb_ctx& ctx, ProjTables& t) {
   INQB_TRY(upload(t.d_seg_ptr, t.seg_ptr));
   INQB_TRY(upload(t.d_seg_atom, t.seg_atom));
   INQB_TRY(upload(t.d_seg_ent, t.seg_ent));
-  INQB_TRY(upload(t.d_ent_off, t.ent_off));
-  INQB_TRY(upload(t.d_ent_atom, t.ent_atom));
   INQB_TRY(upload(t.d_seg_local, t.seg_local));
   INQB_TRY(upload(t.d_plane_ptr, t.plane_ptr));
   INQB_TRY(upload(t.d_plane_atom, t.plane_atom));
@@ -437,27 +473,21 @@ int upload_proj_tables(const inqb_ctx& ctx, ProjTables& t) {
   INQB_TRY(upload(t.d_chunk_beg, t.chunk_beg));
   INQB_TRY(upload(t.d_atom_chunk_ptr, t.atom_chunk_ptr));
   if (ctx.precision == INQB_FP64) {
-    INQB_TRY(upload(t.d_ent_beta, t.ent_beta));
+    INQB_TRY(upload(t.d_ent_rec, ent_records<double>(t, ctx.nr[2])));
+    INQB_TRY(upload(t.d_ent_rec_rk, ent_records<double>(t, ctx.nr[2], true)));
   } else {
-    std::vector<float> bf(t.ent_beta.begin(), t.ent_beta.end());
-    INQB_TRY(upload(t.d_ent_beta, bf));
+    INQB_TRY(upload(t.d_ent_rec, ent_records<float>(t, ctx.nr[2])));
+    INQB_TRY(upload(t.d_ent_rec_rk, ent_records<float>(t, ctx.nr[2], true)));
   }
-  INQB_TRY(t.d_ent_phase.ensure(std::max<size_t>((size_t)t.nent * ctx.elem_bytes(), 16)));
-  if (ctx.precision == INQB_FP64) {
-    INQB_TRY(upload(t.d_ent_rec, ent_records<double>(t)));
-    INQB_TRY(upload(t.d_ent_rec_pt, ent_records<double>(t, true)));
-  } else {
-    INQB_TRY(upload(t.d_ent_rec, ent_records<float>(t)));
-    INQB_TRY(upload(t.d_ent_rec_pt, ent_records<float>(t, true)));
-  }
-  INQB_TRY(upload(t.d_pt_pos, t.pt_pos));
+  INQB_TRY(upload(t.d_rk_pos, t.rk_pos));
   INQB_TRY(upload(t.d_atom_pos, t.atom_pos));
   if (ctx.precision == INQB_FP64) {
     INQB_TRY(upload(t.d_adj_rec, adj_records<double>(t)));
   } else {
     INQB_TRY(upload(t.d_adj_rec, adj_records<float>(t)));
   }
-  INQB_TRY(upload(t.d_pt_ptr, t.pt_ptr));
+  INQB_TRY(upload(t.d_rk_ptr, t.rk_ptr));
+  INQB_TRY(upload(t.d_rk_start, t.rk_start));
   INQB_TRY(upload(t.d_aslot_ptr, t.aslot_ptr));
   INQB_TRY(upload(t.d_aslot, t.aslot));
   INQB_TRY(upload(t.d_pc_ptr, t.pc_ptr));

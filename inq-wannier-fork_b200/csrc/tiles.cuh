@@ -36,12 +36,19 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(PENDING) : "memory");
 }
 
+// The three passes of an apply are launched with programmatic dependence: a pass may be
+// scheduled while the one before it drains, fills its tables (which no pass writes) and
+// waits here before it touches anything the passes exchange.  The next pass is let in as
+// the CTAs of this one exit; letting it in earlier (launch_dependents) parks its CTAs in
+// the slots of running ones and measured slower (64^3 x 128 mixed: 548 -> 595 us).
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Loads of data another CTA of the same launch wrote (the Fourier intermediate, the
 // projection partial sums and results): through L2 (ld.global.cg), never a line an
 // earlier load left in this SM's L1, so one persistent launch can run the passes.
-__device__ __forceinline__ cplx<float> ld_l2(const cplx<float>* p) {
-  const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
-  return mk<float>(v.x, v.y);
+__device__ __forceinline__ cplx<F2> ld_l2(const cplx<F2>* p) {
+  const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2*>(p));
+  return {F2{v.x}, F2{v.y}};
 }
 __device__ __forceinline__ cplx<double> ld_l2(const cplx<double>* p) {
   const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
@@ -63,40 +70,59 @@ struct TileGeom {
   // per SM (measured: FP32 144^3 apply 75 -> 65 ms; FP64 is faster with 64 bytes)
   static constexpr int RUN = (sizeof(T) == 4 && Y2 * ZS * 64 > 80 * 1024) ? 32 : 64;
   static constexpr int G = RUN / (int)sizeof(cplx<T>);
-  static constexpr int PV = 16 / (int)sizeof(cplx<T>);  // complex values per 16-byte vector
-  static constexpr int VP = G / PV;                      // 16-byte vectors per point
-  static constexpr int TILE = Y2 * ZS * G;  // complex values of a tile in shared memory
-  static constexpr int PTS = Y2 * NZ;       // grid points of a tile
-  static constexpr int XS = (Y1 + 1) * G;   // x-slot stride of the x-line block (one point of padding)
+  static constexpr int PV = 16 / (int)sizeof(cplx<T>);  // orbitals per 16-byte lane
+  static constexpr int VP = G / PV;                      // lanes per point
+  // the sizes below count 16-byte lanes
+  static constexpr int TILE = Y2 * ZS * VP;  // a tile in shared memory
+  static constexpr int PTS = Y2 * NZ;        // grid points of a tile
+  static constexpr int XS = (Y1 + 1) * VP;   // x-slot stride of the x-line block (one point of padding)
   static constexpr int XBLK = AX::SLOTS * XS;
-  static constexpr int BLK = NX * Y1 * G;   // complex values of one tmp block [ix][y1][G]
+  static constexpr int BLK = NX * Y1 * VP;   // one tmp block [ix][y1][G]
   static constexpr int THREADS = 256;
   static constexpr size_t SMEM_MAX = 227 * 1024;  // dynamic shared memory a CTA may have
   static constexpr size_t smem_fwd(int acc_atoms, int rec_cap) {
-    return sizeof(cplx<T>) * ((size_t)TILE + NY + NZ) + sizeof(double2) * (size_t)acc_atoms * LMAX * G +
+    return sizeof(Lane<T>) * ((size_t)TILE + NY + NZ) + sizeof(double2) * (size_t)acc_atoms * LMAX * G +
            sizeof(EntRec<T>) * (size_t)rec_cap;
   }
-  static constexpr size_t SMEM_X = sizeof(cplx<T>) * ((size_t)XBLK + NX) + sizeof(T) * 2 * Y1;
-  static constexpr int PSTRIDE = (PTS + 1 + 3) / 4 * 4;  // ints of a tile's point index
-  // pass C prefetches the input orbitals of its tile into shared memory in FP64
-  // (two CTAs per SM either way, so the copy overlaps the transforms for free);
-  // in FP32 the smaller footprint buys a third CTA per SM instead.
-  static constexpr size_t TILE_BYTES = sizeof(cplx<T>) * (size_t)TILE;
-  static constexpr bool PREFETCH = sizeof(T) == 8 && 2 * TILE_BYTES <= 150 * 1024;
-  // pass C keeps four CTAs per SM in FP32 (64 registers a thread) and two with the
-  // FP64 orbital prefetch (128 registers), where the shared memory allows them
-  static constexpr int INV_MIN_CTAS = PREFETCH ? 2 : (TILE_BYTES <= 40 * 1024) ? 4 : 1;
-  // complex values per atom segment of pass C's staged projections [l][orbital]: 64
-  // bytes of padding, so that consecutive segments start in opposite halves of the
+  static constexpr size_t SMEM_X = sizeof(Lane<T>) * ((size_t)XBLK + NX) + sizeof(T) * 2 * Y1;
+  static constexpr size_t TILE_BYTES = sizeof(Lane<T>) * (size_t)TILE;
+  // CTAs of 256 threads per SM that a pass asks the compiler for: four where the radices
+  // fit 64 registers a thread (up to 8 lanes of a transform), three (80 registers) up to
+  // 12, two (128) beyond, and no more than the tiles in shared memory allow
+  static constexpr int radix_ctas(int r) { return r <= 8 ? 4 : r <= 12 ? 3 : 2; }
+  static constexpr int cmin(int a, int b) { return a < b ? a : b; }
+  static constexpr int cmax(int a, int b) { return a > b ? a : b; }
+  static constexpr int fit(size_t bytes) { return (int)(SMEM_MAX / (bytes + 1024)); }
+  static constexpr int RZ = cmax(AZ::N1, AZ::N2), RX = cmax(AX::N1, AX::N2);
+  static constexpr int FWD_MIN_CTAS = cmax(1, cmin(cmin(3, radix_ctas(cmax(RZ, Y2))), fit(TILE_BYTES)));
+  static constexpr int X_MIN_CTAS = cmax(1, cmin(radix_ctas(cmax(RX, Y1)), fit(SMEM_X)));
+  static constexpr int INV_MIN_CTAS = cmax(1, cmin(radix_ctas(cmax(RZ, Y2)), fit(TILE_BYTES)));
+  // lanes per atom segment of pass C's staged projections [l][orbital]: 64 bytes of
+  // padding, so that consecutive segments start in opposite halves of the
   // shared-memory banks
-  static constexpr int PT_STRIDE = LMAX * G + 64 / (int)sizeof(cplx<T>);
-  static constexpr size_t smem_inv(int rec_cap, int seg_cap) {
-    return sizeof(cplx<T>) * ((size_t)TILE + (PREFETCH ? (size_t)PTS * G : 0) + NY + NZ) +
-           sizeof(EntRec<T>) * (size_t)rec_cap + sizeof(int) * (size_t)PSTRIDE +
-           sizeof(cplx<T>) * (size_t)seg_cap * PT_STRIDE;
+  static constexpr int PT_STRIDE = LMAX * VP + 4;
+  static constexpr size_t smem_inv(int seg_cap) {
+    return sizeof(Lane<T>) * ((size_t)TILE + NY + NZ + (size_t)seg_cap * PT_STRIDE);
   }
-  // pass A default: two CTAs per x-plane where Y1 is even
-  static constexpr int YSPLIT = (Y1 % 2 == 0) ? 2 : 1;
+  // Pass A default: the CTAs that share an x-plane.  Each walks its tiles one after the
+  // other, so fewer tiles per CTA end the launch more evenly; more CTAs add partial sums of
+  // the projection.  Measured (mixed; CTAs per plane: us of the pass): 144^3 1: 2487,
+  // 3: 2223, 9: 2104; 128^3 2: 735, 4: 608, 8: 626; 96^3 2: 315, 4: 275, 8: 280; 60^3 1: 118,
+  // 5: 95; 40^3 1: 25.8, 5: 18.7; 32^3 2: 14.1, 4: 10.7; 24^3 1: 18.7, 3: 12.3; but 64^3 2: 184,
+  // 4: 193, 8: 187 and 72^3 2: 135, 8: 136.
+  static constexpr int YSPLIT = (Y1 % 2 == 1 || Y1 <= 4) ? Y1 : Y1 == 6 ? 3 : (TILE_BYTES > 40 * 1024) ? 4 : 2;
+  // default threads of the passes: the columns of a pass's stages in as few equal rounds as
+  // its register budget suggests (blockDim need not match; idle lanes in the last round of
+  // every stage do cost).  Measured (mixed, us): pass B 144^3 256 threads 1302, 160 1111;
+  // 96^3 256 242, 192 232; 60^3 256 57, 128 52; 48^3 256 36.8, 192 34.8; pass C 40^3 256 22.7,
+  // 160 20.1; 36^3 256 31, 160 28.7.
+  static constexpr int round_threads(int cols, int most) {
+    const int rounds = (cols + most - 1) / most;
+    return cmin(THREADS, cmax(64, ((cols + rounds - 1) / rounds + 31) / 32 * 32));
+  }
+  static constexpr int X_THREADS =
+      round_threads(NX * VP, sizeof(T) == 8 ? 192 : (cmax(RX, Y1) > 8 || NX * VP > 256) ? 192 : 256);
+  static constexpr int Z_THREADS = (NZ * VP > 128 && NZ * VP <= 192) ? round_threads(NZ * VP, 192) : THREADS;
 };
 
 // Entry records staged in shared memory per tile; a tile with more entries
@@ -124,28 +150,28 @@ __device__ __forceinline__ const EntRec<T>* stage_entries(const ProjView<T>& pj,
 
 // Plane accumulators held in shared memory by pass A; atoms beyond this many per
 // plane accumulate straight into global memory.
-constexpr int kAccAtomsMax = 48;
-
-template <typename T>
-__device__ __forceinline__ int roff_base(const ProjView<T>& pj, int s0, bool on) {
-  return on ? pj.seg_ent[s0] : 0;
-}
+constexpr int kAccAtomsMax = 192;
+// Atom segments of a tile whose projections pass C stages in shared memory; a tile with
+// more reads its projections from global memory.
+constexpr int kSegMax = 320;
 
 // ---------------------------------------------------------------- pass A
 // The body of one CTA (bx, by) of the pass; k_tile_fwd runs it at (blockIdx.x,
 // blockIdx.y), the persistent batch kernel at the coordinates of a work item.
 template <typename T, int NX, int NY, int NZ>
 __device__ __forceinline__ void tile_fwd_body(int bx, int by, const cplx<T>* __restrict__ in, long ld, int M,
-                                              cplx<T>* __restrict__ tmp, const cplx<T>* __restrict__ tw_y,
+                                              Lane<T>* __restrict__ tmp, const cplx<T>* __restrict__ tw_y,
                                               const cplx<T>* __restrict__ tw_z, ProjView<T> pj, int acc_cap,
                                               int rec_cap, int ysplit, int vec) {
   using TG = TileGeom<T, NX, NY, NZ>;
   using AZ = typename TG::AZ;
+  using V = Lane<T>;
+  using P = LaneP<T>;
   constexpr int G = TG::G, PV = TG::PV, VP = TG::VP, Y1 = TG::Y1, Y2 = TG::Y2, ZS = TG::ZS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<T>* S = reinterpret_cast<cplx<T>*>(smem_raw);
-  cplx<T>* twy = S + TG::TILE;
-  cplx<T>* twz = twy + NY;
+  V* S = reinterpret_cast<V*>(smem_raw);
+  V* twy = S + TG::TILE;
+  V* twz = twy + NY;
   double2* acc = reinterpret_cast<double2*>(twz + NZ);  // [acc_cap][LMAX][G]
   EntRec<T>* R = reinterpret_cast<EntRec<T>*>(acc + acc_cap * LMAX * G);  // [rec_cap]
 
@@ -157,100 +183,124 @@ __device__ __forceinline__ void tile_fwd_body(int bx, int by, const cplx<T>* __r
   const bool v16 = vec && gcount == G;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const bool proj_on = pj.nproj > 0;
-  for (int i = threadIdx.x; i < NY; i += blockDim.x) twy[i] = tw_y[i];
-  for (int i = threadIdx.x; i < NZ; i += blockDim.x) twz[i] = tw_z[i];
-  if (proj_on) {
+  for (int i = threadIdx.x; i < NY; i += blockDim.x) twy[i] = lane_splat(tw_y[i]);
+  for (int i = threadIdx.x; i < NZ; i += blockDim.x) twz[i] = lane_splat(tw_z[i]);
+  if (proj_on)
     for (int i = threadIdx.x; i < acc_cap * LMAX * G; i += blockDim.x) acc[i] = make_double2(0.0, 0.0);
-    // slots of the plane's atoms beyond the shared-memory accumulators start at zero
-    if (pj.slots) {
-      const int a0 = pj.plane_ptr[ix], na = pj.plane_ptr[ix + 1] - a0;
-      for (int i = threadIdx.x; i < max(0, na - acc_cap) * LMAX * G; i += blockDim.x) {
-        const int j = i % G, l = (i / G) % LMAX, sl = acc_cap + i / (G * LMAX);
-        if (j < gcount) pj.slots[(((long)(a0 + sl) * YS + yh) * LMAX + l) * M + m0 + j] = make_double2(0.0, 0.0);
-      }
+  chain_wait();
+  // slots of the plane's atoms beyond the shared-memory accumulators start at zero
+  if (proj_on && pj.slots) {
+    const int a0 = pj.plane_ptr[ix], na = pj.plane_ptr[ix + 1] - a0;
+    for (int i = threadIdx.x; i < max(0, na - acc_cap) * LMAX * G; i += blockDim.x) {
+      const int j = i % G, l = (i / G) % LMAX, sl = acc_cap + i / (G * LMAX);
+      if (j < gcount) pj.slots[(((long)(a0 + sl) * YS + yh) * LMAX + l) * M + m0 + j] = make_double2(0.0, 0.0);
     }
   }
 
-  for (int y1 = yh * YPER; y1 < (yh + 1) * YPER; ++y1) {
-    // -- rows y1 + Y1 r of plane ix, G orbitals per point
+  // rows y1 + Y1 r of plane ix, G orbitals per point, in the orbital layout, and the tile's
+  // entry records: the copies of tile y1
+  int roff = 0;
+  const EntRec<T>* rec = pj.ent_rec;
+  auto load_tile = [&](int y1) {
     if (v16) {
+#pragma unroll 1
       for (int q = threadIdx.x; q < TG::PTS * VP; q += blockDim.x) {
         const int v = q % VP, pt = q / VP;
         const int z = pt % NZ, r = pt / NZ;
         const long p = ((long)ix * NY + y1 + Y1 * r) * NZ + z;
-        cp_async16(S + (r * ZS + AZ::slot(z)) * G + v * PV, in + p * ld + m0 + v * PV);
+        cp_async16(S + (r * ZS + AZ::slot(z)) * VP + v, in + p * ld + m0 + v * PV);
       }
     } else {
+      cplx<T>* Sj = reinterpret_cast<cplx<T>*>(S);
       for (int q = threadIdx.x; q < TG::PTS * G; q += blockDim.x) {
         const int j = q % G, pt = q / G;
         const int z = pt % NZ, r = pt / NZ;
         const long p = ((long)ix * NY + y1 + Y1 * r) * NZ + z;
-        S[(r * ZS + AZ::slot(z)) * G + j] = (j < gcount) ? in[p * ld + m0 + j] : mk<T>(0, 0);
+        Sj[(r * ZS + AZ::slot(z)) * G + j] = (j < gcount) ? in[p * ld + m0 + j] : mk<T>(0, 0);
       }
     }
-    int roff = 0;
-    const EntRec<T>* rec = proj_on ? stage_entries(pj, pj.ent_rec, ix * Y1 + y1, rec_cap, R, roff) : pj.ent_rec;
+    if (proj_on) rec = stage_entries(pj, pj.ent_rec, ix * Y1 + y1, rec_cap, R, roff);
     cp_async_commit();
+  };
+  load_tile(yh * YPER);
+
+  for (int y1 = yh * YPER; y1 < (yh + 1) * YPER; ++y1) {
     cp_async_wait<0>();
     __syncthreads();
 
-    // -- KB projection of the tile (projector_all.hpp:104-165): lanes = (orbital j,
-    // segment group); each group of G lanes walks one atom segment's entries, so a
-    // warp has 32 / G segments in flight and no cross-lane reduction is needed
+    // -- KB projection of the tile (projector_all.hpp:104-165).  A group of 4 VP lanes
+    // walks one atom segment: lane = (orbital lane v, entry lane e of four).  The four
+    // entry lanes' sums meet in two exchange steps that leave entry lane e with
+    // projector l = e, which adds it to the plane accumulators.
     if (proj_on) {
-      constexpr int SGRP = 32 / G;
-      const int j = lane % G, sg = lane / G;
+      static_assert(LMAX == 4, "an entry lane ends with one projector");
+      constexpr int SGRP = 32 / (4 * VP);
+      const int v = lane % VP, el = (lane / VP) % 4, sg = lane / (4 * VP);
       const int tile = ix * Y1 + y1;
       const int s0 = pj.seg_ptr[tile], s1 = pj.seg_ptr[tile + 1];
       for (int sb = s0 + warp * SGRP; sb < s1; sb += nw * SGRP) {
         const int s = sb + sg;
-        if (s >= s1) continue;
-        const int e0 = pj.seg_ent[s], e1 = pj.seg_ent[s + 1];
-        cplx<T> a[LMAX];
+        const int e1 = s < s1 ? pj.seg_ent[s + 1] : 0;
+        V a[LMAX];
 #pragma unroll
-        for (int l = 0; l < LMAX; ++l) a[l] = mk<T>(0, 0);
-        for (int e = e0; e < e1; ++e) {
-          const EntRec<T>& re = rec[e - roff];
-          const int off = re.off;
-          const int r = off / NZ, z = off - r * NZ;
-          const cplx<T> x = mk<T>(re.ph[0], re.ph[1]) * S[(r * ZS + AZ::slot(z)) * G + j];
+        for (int l = 0; l < LMAX; ++l) a[l] = {splat<P>(0.0), splat<P>(0.0)};
+        auto add = [&](const EntRec<T>& re) {
+          const V u = flip(S[re.off * VP + v]);
+          const P pr = splat_of(re.ph[0]), pi = splat_of(re.ph[1]), npi = splat_of(-re.ph[1]);
+          const V x = {vfma(u.x, pr, u.y * npi), vfma(u.x, pi, u.y * pr)};
 #pragma unroll
           for (int l = 0; l < LMAX; ++l) {
-            const T b = re.beta[l];
-            a[l].x = fma(b, x.x, a[l].x);
-            a[l].y = fma(b, x.y, a[l].y);
+            const P b = splat_of(re.beta[l]);
+            a[l].x = vfma(b, x.x, a[l].x);
+            a[l].y = vfma(b, x.y, a[l].y);
           }
+        };
+        int e = s < s1 ? pj.seg_ent[s] + el : 0;
+        if constexpr (TG::TILE_BYTES > 40 * 1024) {
+          // a tile this large seldom has its records staged: the next one is fetched ahead
+          EntRec<T> nx;
+          if (e < e1) nx = rec[e - roff];
+          for (; e < e1; e += 4) {
+            const EntRec<T> re = nx;
+            if (e + 4 < e1) nx = rec[e + 4 - roff];
+            add(re);
+          }
+        } else {
+#pragma unroll 1
+          for (; e < e1; e += 4) add(rec[e - roff]);
         }
-        if (j < gcount) {
-          const int sl = pj.seg_local[s];
-          if (sl < acc_cap) {
-            // one segment per atom in a tile, tiles separated by barriers: no race
+        __syncwarp();
+        // entry lanes 0, 1 keep l = 0, 1 and 2, 3 keep l = 2, 3; then one each
+        const bool hi = (el & 2) != 0, odd = (el & 1) != 0;
+        const V b0 = (hi ? a[2] : a[0]) + lane_shfl_xor(hi ? a[0] : a[2], 2 * VP);
+        const V b1 = (hi ? a[3] : a[1]) + lane_shfl_xor(hi ? a[1] : a[3], 2 * VP);
+        const V c = (odd ? b1 : b0) + lane_shfl_xor(odd ? b0 : b1, VP);
+        if (s < s1) {
+          const int sl = pj.seg_local[s], l = el;
 #pragma unroll
-            for (int l = 0; l < LMAX; ++l) {
+          for (int k = 0; k < PV; ++k) {
+            const int j = v * PV + k;
+            const cplx<T> w = lane_get(c, k);
+            if (j >= gcount) continue;
+            if (sl < acc_cap) {
+              // one segment per atom in a tile, tiles separated by barriers: no race
               double2& d = acc[(sl * LMAX + l) * G + j];
-              d.x += (double)a[l].x;
-              d.y += (double)a[l].y;
-            }
-          } else if (pj.slots) {
-            // beyond the shared-memory accumulators: this CTA's own slot in global
-            // memory (zeroed at the start), the same ownership
-            double2* d = pj.slots + (((long)(pj.plane_ptr[ix] + sl) * YS + yh) * LMAX) * M + m0 + j;
-#pragma unroll
-            for (int l = 0; l < LMAX; ++l) {
-              double2 v = ld_l2(d + (long)l * M);
-              v.x += (double)a[l].x;
-              v.y += (double)a[l].y;
-              d[(long)l * M] = v;
-            }
-          } else {
-            const int at = pj.seg_atom[s];
-#pragma unroll
-            for (int l = 0; l < LMAX; ++l) {
-              if (l >= pj.L) break;
+              d.x += (double)w.x;
+              d.y += (double)w.y;
+            } else if (pj.slots) {
+              // beyond the shared-memory accumulators: this CTA's own slot in global
+              // memory (zeroed at the start), the same ownership
+              double2* d = pj.slots + (((long)(pj.plane_ptr[ix] + sl) * YS + yh) * LMAX + l) * M + m0 + j;
+              double2 o = ld_l2(d);
+              o.x += (double)w.x;
+              o.y += (double)w.y;
+              *d = o;
+            } else if (l < pj.L) {
+              const int at = pj.seg_atom[s];
               const double sc = pj.scale[at * pj.L + l];
               double2* dst = &pj.proj[((long)at * pj.L + l) * M + m0 + j];
-              atomicAdd(&dst->x, sc * (double)a[l].x);
-              atomicAdd(&dst->y, sc * (double)a[l].y);
+              atomicAdd(&dst->x, sc * (double)w.x);
+              atomicAdd(&dst->y, sc * (double)w.y);
             }
           }
         }
@@ -258,38 +308,43 @@ __device__ __forceinline__ void tile_fwd_body(int bx, int by, const cplx<T>* __r
       __syncthreads();
     }
 
-    // -- z lines: (r, j), element stride G
-    step1<AZ, false>(S, Y2 * G * AZ::N2, twz, [](int it, int& base, int& es, int& j2) {
-      const int j = it % G, rest = it / G;
+    // -- z lines: (r, v), element stride VP; the first step leaves the lane layout
+    step1<AZ, false, true>(S, Y2 * VP * AZ::N2, twz, [](int it, int& base, int& es, int& j2) {
+      const int v = it % VP, rest = it / VP;
       j2 = rest % AZ::N2;
-      base = (rest / AZ::N2) * ZS * G + j;
-      es = G;
+      base = (rest / AZ::N2) * ZS * VP + v;
+      es = VP;
     });
     __syncthreads();
-    step2<AZ, false>(S, Y2 * G * AZ::N1, [](int it, int& base, int& es, int& k1) {
-      const int j = it % G, rest = it / G;
+    step2<AZ, false>(S, Y2 * VP * AZ::N1, [](int it, int& base, int& es, int& k1) {
+      const int v = it % VP, rest = it / VP;
       k1 = rest % AZ::N1;
-      base = (rest / AZ::N1) * ZS * G + j;
-      es = G;
+      base = (rest / AZ::N1) * ZS * VP + v;
+      es = VP;
     });
     __syncthreads();
 
     // -- inner y stage: DFT_Y2 over the rows, twiddle w_NY^{y1 ka}, written straight
-    // to tmp[g][ka][kz][ix][y1][G] (lanes along j write whole 64-byte runs)
-    for (int it = threadIdx.x; it < NZ * G; it += blockDim.x) {
-      const int j = it % G, kz = it / G;
-      const int base = AZ::slot_of_freq(kz) * G + j;
-      cplx<T> u[Y2];
+    // to tmp[g][ka][kz][ix][y1][G] (lanes along v write whole 64-byte runs).  (Starting the
+    // next tile's copies once the columns are in registers, before they are transformed and
+    // stored, spilled and measured slower: 64^3 x 128 mixed 178 -> 193 us.)
+    for (int it0 = 0; it0 < NZ * VP; it0 += blockDim.x) {
+      const int it = it0 + threadIdx.x;
+      if (it >= NZ * VP) continue;
+      const int v = it % VP, kz = it / VP;
+      const int base = AZ::slot_of_freq(kz) * VP + v;
+      V u[Y2];
 #pragma unroll
-      for (int r = 0; r < Y2; ++r) u[r] = S[base + r * ZS * G];
-      DFT<Y2, false, T>::run(u);
+      for (int r = 0; r < Y2; ++r) u[r] = S[base + r * ZS * VP];
+      DFT<Y2, false, P>::run(u);
 #pragma unroll
-      for (int ka = 1; ka < Y2; ++ka) u[ka] = u[ka] * twy[ka * Y1 + y1];
-      cplx<T>* dst = tmp + (((long)grp * Y2 * NZ + kz) * NX + ix) * (Y1 * G) + y1 * G + j;
+      for (int ka = 1; ka < Y2; ++ka) u[ka] = lmul(u[ka], twy[ka * Y1 + y1]);
+      V* dst = tmp + (((long)grp * Y2 * NZ + kz) * NX + ix) * (Y1 * VP) + y1 * VP + v;
 #pragma unroll
       for (int ka = 0; ka < Y2; ++ka) dst[(long)ka * NZ * TG::BLK] = u[ka];
     }
     __syncthreads();
+    if (y1 + 1 < (yh + 1) * YPER) load_tile(y1 + 1);
   }
 
   // -- flush the plane accumulators: into this CTA's (plane, half) slots, which the
@@ -316,8 +371,8 @@ __device__ __forceinline__ void tile_fwd_body(int bx, int by, const cplx<T>* __r
 }
 
 template <typename T, int NX, int NY, int NZ>
-__global__ void __launch_bounds__(256)
-    k_tile_fwd(const cplx<T>* __restrict__ in, long ld, int M, cplx<T>* __restrict__ tmp,
+__global__ void __launch_bounds__(256, TileGeom<T, NX, NY, NZ>::FWD_MIN_CTAS)
+    k_tile_fwd(const cplx<T>* __restrict__ in, long ld, int M, Lane<T>* __restrict__ tmp,
                const cplx<T>* __restrict__ tw_y, const cplx<T>* __restrict__ tw_z, ProjView<T> pj, int acc_cap,
                int rec_cap, int ysplit, int vec) {
   tile_fwd_body<T, NX, NY, NZ>(blockIdx.x, blockIdx.y, in, ld, M, tmp, tw_y, tw_z, pj, acc_cap, rec_cap, ysplit,
@@ -325,19 +380,25 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---------------------------------------------------------------- projection finish
-// proj[a][l][m] = dV ekb[a][l] sum over the atom's (plane, half) slots, in the order of
-// its planes and halves: pass A wrote one partial per slot, no atomics.  Item i =
-// (a * L + l) * M + m; eight loads in flight, added in order.
+// proj[a][l][m] = dV ekb[a][l] sum over the atom's (plane, CTA of the plane) slots: pass A
+// wrote one partial per slot, no atomics.  Eight lanes (kFinParts) share an item
+// i = (a * L + l) * M + m: part k adds the slots k, k + 8, ... in order and the parts meet
+// by shuffles, so the sum has one fixed order and a chain of only slots / 8 loads (one
+// thread per item: 24^3, 57 slots an atom, pass B 12 -> 19 us).  Lanes of a warp: four
+// items next to each other in m, eight parts; every lane of the warp calls it.
+constexpr int kFinParts = 8;
 template <typename T>
-__device__ __forceinline__ void proj_finish_item(const ProjView<T>& pj, int M, int ysplit, long i) {
-  const int m = (int)(i % M), l = (int)((i / M) % pj.L), a = (int)(i / ((long)M * pj.L));
-  const int q0 = pj.aslot_ptr[a] * ysplit, q1 = pj.aslot_ptr[a + 1] * ysplit;
+__device__ __forceinline__ void proj_finish_item(const ProjView<T>& pj, int M, int ysplit, unsigned i, bool on) {
+  const int part = (threadIdx.x & 31) / (32 / kFinParts);
+  const unsigned al = i / M;
+  const int m = (int)(i - al * M), a = on ? (int)(al / pj.L) : 0, l = (int)(al % pj.L);
+  const int q0 = pj.aslot_ptr[a] * ysplit, q1 = on ? pj.aslot_ptr[a + 1] * ysplit : 0;
   double sx = 0.0, sy = 0.0;
-  for (int qb = q0; qb < q1; qb += 8) {
-    double2 v[8];
+  for (int qb = q0 + part; qb < q1; qb += 4 * kFinParts) {
+    double2 v[4];
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int q = qb + u;
+    for (int u = 0; u < 4; u++) {
+      const int q = qb + u * kFinParts;
       v[u] = make_double2(0.0, 0.0);
       if (q < q1) {
         const long slot = (long)pj.aslot[q / ysplit] * ysplit + q % ysplit;
@@ -345,14 +406,25 @@ __device__ __forceinline__ void proj_finish_item(const ProjView<T>& pj, int M, i
       }
     }
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
+    for (int u = 0; u < 4; u++) {
       sx += v[u].x;
       sy += v[u].y;
     }
   }
-  const double sc = pj.scale[a * pj.L + l];
-  pj.proj[i] = make_double2(sc * sx, sc * sy);
+  __syncwarp();
+#pragma unroll
+  for (int o = 32 / kFinParts; o < 32; o *= 2) {
+    sx += __shfl_xor_sync(0xffffffffu, sx, o);
+    sy += __shfl_xor_sync(0xffffffffu, sy, o);
+  }
+  if (on && part == 0) {
+    const double sc = pj.scale[a * pj.L + l];
+    pj.proj[i] = make_double2(sc * sx, sc * sy);
+  }
 }
+// the item of this thread among the warps' groups of four: thread t of a run of threads
+// handles item (t / 32) * 4 + t % 4
+__device__ __forceinline__ long finish_item(long t) { return t / 32 * (32 / kFinParts) + t % (32 / kFinParts); }
 
 // ---------------------------------------------------------------- pass B
 // One contiguous block tmp[g][ka][kz] = [ix][y1][G]; in shared memory the x
@@ -361,21 +433,23 @@ __device__ __forceinline__ void proj_finish_item(const ProjView<T>& pj, int M, i
 // thread t of CTA b handles item b * blockDim + t, so the few CTAs that carry the
 // finish run beside thousands that do not.
 template <typename T, int NX, int NY, int NZ>
-__device__ __forceinline__ void tile_x_body(int bx, int by, cplx<T>* __restrict__ tmp,
+__device__ __forceinline__ void tile_x_body(int bx, int by, Lane<T>* __restrict__ tmp,
                                             const cplx<T>* __restrict__ tw_x, KinParams<T> kp,
                                             cplx<T>* __restrict__ fout) {
   using TG = TileGeom<T, NX, NY, NZ>;
   using AX = typename TG::AX;
-  constexpr int G = TG::G, PV = TG::PV, VP = TG::VP, Y1 = TG::Y1, Y2 = TG::Y2, XS = TG::XS;
+  using V = Lane<T>;
+  using P = LaneP<T>;
+  constexpr int VP = TG::VP, Y1 = TG::Y1, Y2 = TG::Y2, XS = TG::XS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<T>* X = reinterpret_cast<cplx<T>*>(smem_raw);
-  cplx<T>* twx = X + TG::XBLK;
+  V* X = reinterpret_cast<V*>(smem_raw);
+  V* twx = X + TG::XBLK;
   T* kinB = reinterpret_cast<T*>(twx + NX);  // [Y1] linear and [Y1] constant term per kb
   T* kinC = kinB + Y1;
 
   const int kz = bx % NZ, ka = bx / NZ, grp = by;
-  cplx<T>* blk = tmp + ((long)(grp * Y2 + ka) * NZ + kz) * TG::BLK;
-  for (int i = threadIdx.x; i < NX; i += blockDim.x) twx[i] = tw_x[i];
+  V* blk = tmp + ((long)(grp * Y2 + ka) * NZ + kz) * TG::BLK;
+  for (int i = threadIdx.x; i < NX; i += blockDim.x) twx[i] = lane_splat(tw_x[i]);
   // Along an x line 1/2 |G + k + A|^2 / N = kA2 n0^2 + kinB n0 + kinC with
   // q = n1 b1 + n2 b2 + k + A:  kA2 = |b0|^2 / 2N, kinB = b0.q / N, kinC = |q|^2 / 2N
   if (threadIdx.x < Y1) {
@@ -394,86 +468,80 @@ __device__ __forceinline__ void tile_x_body(int bx, int by, cplx<T>* __restrict_
   const T kinA = (T)0.5 * kp.scale *
                  (kp.b[0][0] * kp.b[0][0] + kp.b[0][1] * kp.b[0][1] + kp.b[0][2] * kp.b[0][2]);
 
-  // outer y stage straight from HBM: a thread loads the Y1 values of its (ix, j)
-  // column (lanes along j read whole 64-byte runs), DFT_Y1 over y1 -> kb, and
-  // writes the column to shared memory once; two columns per thread in flight
-  for (int it0 = threadIdx.x; it0 < NX * G; it0 += 2 * blockDim.x) {
-    cplx<T> u[2][Y1];
+  chain_wait();
+  // outer y stage straight from HBM: a thread loads the Y1 lanes of its (ix, v)
+  // column (neighbouring threads read whole 64-byte runs), DFT_Y1 over y1 -> kb, and
+  // writes the column to shared memory once
+  for (int it = threadIdx.x; it < NX * VP; it += blockDim.x) {
+    const int v = it % VP, ix = it / VP;
+    V u[Y1];
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const int it = it0 + c * blockDim.x;
-      if (it >= NX * G) continue;
-      const int j = it % G, ix = it / G;
+    for (int y = 0; y < Y1; ++y) u[y] = ld_l2(blk + (ix * Y1 + y) * VP + v);
+    DFT<Y1, false, P>::run(u);
+    const int base = AX::slot(ix) * XS + v;
 #pragma unroll
-      for (int y = 0; y < Y1; ++y) u[c][y] = ld_l2(blk + (ix * Y1 + y) * G + j);
-    }
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const int it = it0 + c * blockDim.x;
-      if (it >= NX * G) continue;
-      const int j = it % G, ix = it / G;
-      DFT<Y1, false, T>::run(u[c]);
-      const int base = AX::slot(ix) * XS + j;
-#pragma unroll
-      for (int y = 0; y < Y1; ++y) X[base + y * G] = u[c][y];
-    }
+    for (int y = 0; y < Y1; ++y) X[base + y * VP] = u[y];
   }
   __syncthreads();
 
   auto map1 = [](int it, int& base, int& es, int& j2) {
-    const int j = it % G, rest = it / G;
+    const int v = it % VP, rest = it / VP;
     j2 = rest % AX::N2;
-    base = (rest / AX::N2) * G + j;
+    base = (rest / AX::N2) * VP + v;
     es = XS;
   };
   auto map2 = [](int it, int& base, int& es, int& k1) {
-    const int j = it % G, rest = it / G;
+    const int v = it % VP, rest = it / VP;
     k1 = rest % AX::N1;
-    base = (rest / AX::N1) * G + j;
+    base = (rest / AX::N1) * VP + v;
     es = XS;
   };
   const int n2 = sym_freq(kz, NZ);
-  step1<AX, false>(X, Y1 * G * AX::N2, twx, map1);
+  step1<AX, false>(X, Y1 * VP * AX::N2, twx, map1);
   __syncthreads();
   // fout (optional): the forward coefficients of this block, before the kinetic
-  // factor, as [kx][kb][G] (the adjoint's velocity terms read them)
-  cplx<T>* fblk = fout ? fout + ((long)(grp * Y2 + ka) * NZ + kz) * TG::BLK : nullptr;
-  step2_fwd_op_inv<AX>(X, Y1 * G * AX::N1, twx, map2, [&](int it, int kx, cplx<T> v) {
-    const int kb = (it / G) / AX::N1;
-    if (fblk) fblk[(kx * Y1 + kb) * G + it % G] = v;
+  // factor, as [kx][kb][G] in the orbital layout (the adjoint's velocity terms read them)
+  V* fblk = fout ? reinterpret_cast<V*>(fout) + ((long)(grp * Y2 + ka) * NZ + kz) * TG::BLK : nullptr;
+  step2_fwd_op_inv<AX>(X, Y1 * VP * AX::N1, twx, map2, [&](int it, int kx, V v) -> V {
+    const int kb = (it / VP) / AX::N1;
+    if (fblk) fblk[(kx * Y1 + kb) * VP + it % VP] = flip(v);
     const int n0 = sym_freq(kx, NX);
     const T f0 = (T)n0;
     T k = fma(fma(kinA, f0, kinB[kb]), f0, kinC[kb]);
     if (kp.mask) k = outside_sphere(kp.nr, n0, sym_freq(ka + Y2 * kb, NY), n2) ? (T)0 : k - kp.shift;
     if (kp.pois != (T)0) k = ((T)2 * k < (T)1e-6) ? (T)0 : kp.pois / k;
-    return k * v;
+    const P ks = splat_of(k);
+    return {ks * v.x, ks * v.y};
   });
   __syncthreads();
-  step1_inv_transposed<AX>(X, Y1 * G * AX::N2, map1);
+  step1_inv_transposed<AX>(X, Y1 * VP * AX::N2, map1);
   __syncthreads();
 
   // inverse outer y stage kb -> y1, written straight back to HBM
-  for (int it = threadIdx.x; it < NX * G; it += blockDim.x) {
-    const int j = it % G, ix = it / G;
-    const int base = AX::slot(ix) * XS + j;
-    cplx<T> u[Y1];
+  for (int it = threadIdx.x; it < NX * VP; it += blockDim.x) {
+    const int v = it % VP, ix = it / VP;
+    const int base = AX::slot(ix) * XS + v;
+    V u[Y1];
 #pragma unroll
-    for (int y = 0; y < Y1; ++y) u[y] = X[base + y * G];
-    DFT<Y1, true, T>::run(u);
+    for (int y = 0; y < Y1; ++y) u[y] = X[base + y * VP];
+    DFT<Y1, true, P>::run(u);
 #pragma unroll
-    for (int y = 0; y < Y1; ++y) blk[(ix * Y1 + y) * G + j] = u[y];
+    for (int y = 0; y < Y1; ++y) blk[(ix * Y1 + y) * VP + v] = u[y];
   }
 }
 
 template <typename T, int NX, int NY, int NZ>
-__global__ void __launch_bounds__(256)
-    k_tile_x(cplx<T>* __restrict__ tmp, const cplx<T>* __restrict__ tw_x, KinParams<T> kp,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? TileGeom<T, NX, NY, NZ>::X_MIN_CTAS : 1)
+    k_tile_x(Lane<T>* __restrict__ tmp, const cplx<T>* __restrict__ tw_x, KinParams<T> kp,
              cplx<T>* __restrict__ fout, ProjView<T> fin, int fin_M, int fin_ysplit) {
   if (fin.slots) {
     const long n = (long)fin.nproj * fin.L * fin_M;
     const long stride = (long)gridDim.x * gridDim.y * blockDim.x;
-    for (long i = ((long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
-      proj_finish_item(fin, fin_M, fin_ysplit, i);
+    chain_wait();
+    for (long t = ((long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x; finish_item(t) < n; t += stride) {
+      const long i = finish_item(t + threadIdx.x);
+      proj_finish_item(fin, fin_M, fin_ysplit, i < n ? (unsigned)i : 0u, i < n);
+    }
   }
   tile_x_body<T, NX, NY, NZ>(blockIdx.x, blockIdx.y, tmp, tw_x, kp, fout);
 }
@@ -485,75 +553,69 @@ __global__ void __launch_bounds__(256)
 //   y stage -> block tmp[g][ka][kz]; pass C finishes with the inner y and z stages
 //   and the 1/N (transform.hpp:250-332).
 template <typename T, int NX, int NY, int NZ, int DIR>
-__global__ void __launch_bounds__(256)
-    k_tile_x_fft(cplx<T>* __restrict__ tmp, const cplx<T>* __restrict__ in, cplx<T>* __restrict__ out, long ld,
+__global__ void __launch_bounds__(256, TileGeom<T, NX, NY, NZ>::X_MIN_CTAS)
+    k_tile_x_fft(Lane<T>* __restrict__ tmp, const cplx<T>* __restrict__ in, cplx<T>* __restrict__ out, long ld,
                  int M, const cplx<T>* __restrict__ tw_x, int vec) {
   using TG = TileGeom<T, NX, NY, NZ>;
   using AX = typename TG::AX;
+  using V = Lane<T>;
+  using P = LaneP<T>;
   constexpr int G = TG::G, PV = TG::PV, VP = TG::VP, Y1 = TG::Y1, Y2 = TG::Y2, XS = TG::XS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<T>* X = reinterpret_cast<cplx<T>*>(smem_raw);
-  cplx<T>* twx = X + TG::XBLK;
+  V* X = reinterpret_cast<V*>(smem_raw);
+  V* twx = X + TG::XBLK;
 
   const int kz = blockIdx.x % NZ, ka = blockIdx.x / NZ, grp = blockIdx.y;
   const int m0 = grp * G;
   const int gcount = min(G, M - m0);
   const bool v16 = vec && gcount == G;
-  cplx<T>* blk = tmp + ((long)(grp * Y2 + ka) * NZ + kz) * TG::BLK;
+  V* blk = tmp + ((long)(grp * Y2 + ka) * NZ + kz) * TG::BLK;
   // point of frequency (kx, ka + Y2 kb, kz) in the orbital layout
   auto point = [&](int kx, int kb) { return ((long)kx * NY + ka + Y2 * kb) * NZ + kz; };
   auto map1 = [](int it, int& base, int& es, int& j2) {
-    const int j = it % G, rest = it / G;
+    const int v = it % VP, rest = it / VP;
     j2 = rest % AX::N2;
-    base = (rest / AX::N2) * G + j;
+    base = (rest / AX::N2) * VP + v;
     es = XS;
   };
   auto map2 = [](int it, int& base, int& es, int& k1) {
-    const int j = it % G, rest = it / G;
+    const int v = it % VP, rest = it / VP;
     k1 = rest % AX::N1;
-    base = (rest / AX::N1) * G + j;
+    base = (rest / AX::N1) * VP + v;
     es = XS;
   };
-  for (int i = threadIdx.x; i < NX; i += blockDim.x) twx[i] = tw_x[i];
+  for (int i = threadIdx.x; i < NX; i += blockDim.x) twx[i] = lane_splat(tw_x[i]);
+  chain_wait();
 
   if (DIR == 0) {
-    for (int q = threadIdx.x; q < NX * Y1 * VP; q += blockDim.x) {
-      const int v = q % VP, r = q / VP;
-      const int y1 = r % Y1, ix = r / Y1;
-      cp_async16(X + AX::slot(ix) * XS + y1 * G + v * PV, blk + (long)q * PV);
-    }
-    cp_async_commit();
-    cp_async_wait<0>();
-    __syncthreads();
-    // outer y stage: y1 -> kb
-    for (int it = threadIdx.x; it < NX * G; it += blockDim.x) {
-      const int j = it % G, ix = it / G;
-      const int base = AX::slot(ix) * XS + j;
-      cplx<T> u[Y1];
+    // outer y stage straight from HBM, as in the H pass: y1 -> kb
+    for (int it = threadIdx.x; it < NX * VP; it += blockDim.x) {
+      const int v = it % VP, ix = it / VP;
+      V u[Y1];
 #pragma unroll
-      for (int y = 0; y < Y1; ++y) u[y] = X[base + y * G];
-      DFT<Y1, false, T>::run(u);
+      for (int y = 0; y < Y1; ++y) u[y] = ld_l2(blk + (ix * Y1 + y) * VP + v);
+      DFT<Y1, false, P>::run(u);
+      const int base = AX::slot(ix) * XS + v;
 #pragma unroll
-      for (int y = 0; y < Y1; ++y) X[base + y * G] = u[y];
+      for (int y = 0; y < Y1; ++y) X[base + y * VP] = u[y];
     }
     __syncthreads();
-    step1<AX, false>(X, Y1 * G * AX::N2, twx, map1);
+    step1<AX, false>(X, Y1 * VP * AX::N2, twx, map1);
     __syncthreads();
-    step2<AX, false>(X, Y1 * G * AX::N1, map2);
+    step2<AX, false>(X, Y1 * VP * AX::N1, map2);
     __syncthreads();
     // kx sits in slot_of_freq(kx)
-    if (v16) {
-      for (int q = threadIdx.x; q < NX * Y1 * VP; q += blockDim.x) {
-        const int v = q % VP, r = q / VP;
-        const int kb = r % Y1, kx = r / Y1;
-        *reinterpret_cast<float4*>(out + point(kx, kb) * ld + m0 + v * PV) =
-            *reinterpret_cast<const float4*>(X + AX::slot_of_freq(kx) * XS + kb * G + v * PV);
-      }
-    } else {
-      for (int q = threadIdx.x; q < NX * Y1 * G; q += blockDim.x) {
-        const int j = q % G, r = q / G;
-        const int kb = r % Y1, kx = r / Y1;
-        if (j < gcount) out[point(kx, kb) * ld + m0 + j] = X[AX::slot_of_freq(kx) * XS + kb * G + j];
+    for (int q = threadIdx.x; q < NX * Y1 * VP; q += blockDim.x) {
+      const int v = q % VP, r = q / VP;
+      const int kb = r % Y1, kx = r / Y1;
+      const V w = X[AX::slot_of_freq(kx) * XS + kb * VP + v];
+      cplx<T>* dst = out + point(kx, kb) * ld + m0 + v * PV;
+      if (v16) {
+        *reinterpret_cast<V*>(dst) = flip(w);
+      } else {
+#pragma unroll
+        for (int k = 0; k < PV; ++k)
+          if (v * PV + k < gcount) dst[k] = lane_get(w, k);
       }
     }
   } else {
@@ -562,39 +624,33 @@ __global__ void __launch_bounds__(256)
       for (int q = threadIdx.x; q < NX * Y1 * VP; q += blockDim.x) {
         const int v = q % VP, r = q / VP;
         const int kb = r % Y1, kx = r / Y1;
-        cp_async16(X + AX::slot(kx) * XS + kb * G + v * PV, in + point(kx, kb) * ld + m0 + v * PV);
+        cp_async16(X + AX::slot(kx) * XS + kb * VP + v, in + point(kx, kb) * ld + m0 + v * PV);
       }
       cp_async_commit();
       cp_async_wait<0>();
     } else {
+      cplx<T>* Xj = reinterpret_cast<cplx<T>*>(X);
       for (int q = threadIdx.x; q < NX * Y1 * G; q += blockDim.x) {
         const int j = q % G, r = q / G;
         const int kb = r % Y1, kx = r / Y1;
-        X[AX::slot(kx) * XS + kb * G + j] = (j < gcount) ? in[point(kx, kb) * ld + m0 + j] : mk<T>(0, 0);
+        Xj[(AX::slot(kx) * XS + kb * VP) * PV + j] = (j < gcount) ? in[point(kx, kb) * ld + m0 + j] : mk<T>(0, 0);
       }
     }
     __syncthreads();
-    step1<AX, true>(X, Y1 * G * AX::N2, twx, map1);
+    step1<AX, true, true>(X, Y1 * VP * AX::N2, twx, map1);
     __syncthreads();
-    step2<AX, true>(X, Y1 * G * AX::N1, map2);
+    step2<AX, true>(X, Y1 * VP * AX::N1, map2);
     __syncthreads();
-    // inverse outer y stage: kb -> y1
-    for (int it = threadIdx.x; it < NX * G; it += blockDim.x) {
-      const int j = it % G, ix = it / G;
-      const int base = AX::slot_of_freq(ix) * XS + j;
-      cplx<T> u[Y1];
+    // inverse outer y stage kb -> y1, written straight to HBM
+    for (int it = threadIdx.x; it < NX * VP; it += blockDim.x) {
+      const int v = it % VP, ix = it / VP;
+      const int base = AX::slot_of_freq(ix) * XS + v;
+      V u[Y1];
 #pragma unroll
-      for (int y = 0; y < Y1; ++y) u[y] = X[base + y * G];
-      DFT<Y1, true, T>::run(u);
+      for (int y = 0; y < Y1; ++y) u[y] = X[base + y * VP];
+      DFT<Y1, true, P>::run(u);
 #pragma unroll
-      for (int y = 0; y < Y1; ++y) X[base + y * G] = u[y];
-    }
-    __syncthreads();
-    for (int q = threadIdx.x; q < NX * Y1 * VP; q += blockDim.x) {
-      const int v = q % VP, r = q / VP;
-      const int y1 = r % Y1, ix = r / Y1;
-      *reinterpret_cast<float4*>(blk + (long)q * PV) =
-          *reinterpret_cast<const float4*>(X + AX::slot_of_freq(ix) * XS + y1 * G + v * PV);
+      for (int y = 0; y < Y1; ++y) blk[(ix * Y1 + y) * VP + v] = u[y];
     }
   }
 }
@@ -605,175 +661,193 @@ __global__ void __launch_bounds__(256)
 // MODE_H = 1: the H epilogue; 0: out = alpha * (inverse transform), the second
 // half of to_real (alpha = 1/N), reading neither orbitals, V nor projectors.
 template <typename T, int NX, int NY, int NZ, int MODE_H>
-__device__ __forceinline__ void tile_inv_body(int bx, int by, const cplx<T>* __restrict__ tmp,
+__device__ __forceinline__ void tile_inv_body(int bx, int by, const Lane<T>* __restrict__ tmp,
                                               const cplx<T>* __restrict__ in, long ld_in, cplx<T>* __restrict__ out,
                                               long ld_out, int M, const cplx<T>* __restrict__ tw_y,
                                               const cplx<T>* __restrict__ tw_z, const ProjView<T>& pj,
-                                              const EpiParams<T>& ep, int rec_cap, int seg_cap, int vec) {
+                                              const EpiParams<T>& ep, int seg_cap, int vec) {
   using TG = TileGeom<T, NX, NY, NZ>;
   using AZ = typename TG::AZ;
+  using V = Lane<T>;
+  using P = LaneP<T>;
   constexpr int G = TG::G, PV = TG::PV, VP = TG::VP, Y1 = TG::Y1, Y2 = TG::Y2, ZS = TG::ZS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<T>* S = reinterpret_cast<cplx<T>*>(smem_raw);
-  cplx<T>* P = S + TG::TILE;  // [PTS][G] input orbitals of the tile (PREFETCH)
-  cplx<T>* twy = P + (TG::PREFETCH ? TG::PTS * G : 0);
-  cplx<T>* twz = twy + NY;
-  EntRec<T>* R = reinterpret_cast<EntRec<T>*>(twz + NZ);  // [rec_cap] records in point order
-  int* TP = reinterpret_cast<int*>(R + rec_cap);           // [PSTRIDE] point index of the tile
-  cplx<T>* PT = reinterpret_cast<cplx<T>*>(TP + TG::PSTRIDE);  // [seg_cap][PT_STRIDE] projections
+  V* S = reinterpret_cast<V*>(smem_raw);
+  V* twy = S + TG::TILE;
+  V* twz = twy + NY;
+  V* PT = twz + NZ;  // [seg_cap][PT_STRIDE] projections
 
   const int grp = bx, ix = by / Y1, y1 = by % Y1;
   const int m0 = grp * G;
   const int gcount = min(G, M - m0);
-  const bool v16 = vec && gcount == G;
+  // vec: bit 0, the input and output blocks take 16-byte accesses; bit 1, the base does
+  const bool v16 = (vec & 1) && gcount == G, b16 = (vec & 2) && gcount == G;
 
-  // group 0: the (ka, kz) runs of this tile, needed first; group 1: what only the
-  // epilogue reads (entry records, point index, and in FP64 the input orbitals).
-  // (Reading the runs into registers for the y stage measured slower than staging.)
+  for (int i = threadIdx.x; i < NY; i += blockDim.x) twy[i] = lane_splat(tw_y[i]);
+  for (int i = threadIdx.x; i < NZ; i += blockDim.x) twz[i] = lane_splat(tw_z[i]);
+  // where the tile's segments and records lie (set with the projectors, no pass writes it)
+  const bool proj_on = MODE_H && pj.nproj > 0;
+  const int tile = ix * Y1 + y1;
+  const int s0 = proj_on ? pj.seg_ptr[tile] : 0, nseg = proj_on ? pj.seg_ptr[tile + 1] - s0 : 0;
+  const int k0 = proj_on ? pj.rk_ptr[tile] : 0, k1 = proj_on ? pj.rk_ptr[tile + 1] : 0;
+  const int e_first = k0 < k1 ? pj.rk_start[k0] + (int)threadIdx.x / VP : 0;
+  chain_wait();
+  // the (ka, kz) runs of this tile
   for (int q = threadIdx.x; q < TG::PTS * VP; q += blockDim.x) {
     const int v = q % VP, pt = q / VP;
     const int kz = pt % NZ, ka = pt / NZ;
-    cp_async16(S + (ka * ZS + AZ::slot(kz)) * G + v * PV,
-               tmp + (((long)(grp * Y2 + ka) * NZ + kz) * NX + ix) * (Y1 * G) + y1 * G + v * PV);
+    cp_async16(S + (ka * ZS + AZ::slot(kz)) * VP + v,
+               tmp + (((long)(grp * Y2 + ka) * NZ + kz) * NX + ix) * (Y1 * VP) + y1 * VP + v);
   }
   cp_async_commit();
-  const bool proj_on = MODE_H && pj.nproj > 0;
-  const int tile = ix * Y1 + y1;
-  int roff = 0, s0 = 0, nseg = 0;
-  const EntRec<T>* rec = pj.ent_rec_pt;
-  if (proj_on) {
-    rec = stage_entries(pj, pj.ent_rec_pt, tile, rec_cap, R, roff);
-    const int* tp = pj.pt_ptr + (long)tile * TG::PSTRIDE;
-    for (int q = threadIdx.x; q < TG::PSTRIDE / 4; q += blockDim.x)
-      cp_async16(reinterpret_cast<int4*>(TP) + q, reinterpret_cast<const int4*>(tp) + q);
-    s0 = pj.seg_ptr[tile];
-    nseg = pj.seg_ptr[tile + 1] - s0;
-  }
-  // the point index counts from the tile's first record
-  const int rbase = (rec == R) ? 0 : roff_base(pj, s0, proj_on);
-  if (MODE_H && TG::PREFETCH && v16) {
-    for (int q = threadIdx.x; q < TG::PTS * VP; q += blockDim.x) {
-      const int v = q % VP, pt = q / VP;
-      const int z = pt % NZ, r = pt / NZ;
-      const long p = ((long)ix * NY + y1 + Y1 * r) * NZ + z;
-      cp_async16(P + pt * G + v * PV, in + p * ld_in + m0 + v * PV);
-    }
-  }
-  cp_async_commit();
-  for (int i = threadIdx.x; i < NY; i += blockDim.x) twy[i] = tw_y[i];
-  for (int i = threadIdx.x; i < NZ; i += blockDim.x) twz[i] = tw_z[i];
-  // the tile's atom projections, in the tile precision, as [segment][l][orbital] with
-  // a segment stride of PT_STRIDE: the lanes of one grid point read one contiguous run
-  // per l (a thread's PV orbitals as one 16-byte vector)
+  // the tile's atom projections, in the tile precision, as [segment][l][orbital lane]
+  // with a segment stride of PT_STRIDE: the lanes of one grid point read one contiguous
+  // run per l
   const bool pt_staged = nseg <= seg_cap;
-  if (proj_on && pt_staged) {
-    for (int i = threadIdx.x; i < nseg * LMAX * G; i += blockDim.x) {
-      const int j = i % G, l = (i / G) % LMAX, ts = i / (G * LMAX);
-      cplx<T> v = mk<T>(0, 0);
-      if (l < pj.L && j < gcount) {
-        const double2 d = ld_l2(pj.proj + ((long)pj.seg_atom[s0 + ts] * pj.L + l) * M + m0 + j);
-        v = mk<T>((T)d.x, (T)d.y);
+  // projection l of atom at, orbital lane v (two orbitals in FP32)
+  auto projection = [&](int at, int l, int v) -> V {
+    cplx<T> w[PV];
+#pragma unroll
+    for (int k = 0; k < PV; ++k) {
+      w[k] = mk<T>(0, 0);
+      if (l < pj.L && v * PV + k < gcount) {
+        const double2 d = ld_l2(pj.proj + ((long)at * pj.L + l) * M + m0 + v * PV + k);
+        w[k] = mk<T>((T)d.x, (T)d.y);
       }
-      PT[ts * TG::PT_STRIDE + l * G + j] = v;
+    }
+    V r;
+    memcpy(&r, w, 16);
+    return flip(r);
+  };
+  if (proj_on && pt_staged) {
+    for (int i = threadIdx.x; i < nseg * LMAX * VP; i += blockDim.x) {
+      const int v = i % VP, l = (i / VP) % LMAX, ts = i / (VP * LMAX);
+      PT[ts * TG::PT_STRIDE + l * VP + v] = projection(pj.seg_atom[s0 + ts], l, v);
     }
   }
-  cp_async_wait<1>();
+  cp_async_wait<0>();
   __syncthreads();
 
   // inverse inner y stage: conj twiddle, inverse DFT_Y2 over ka -> rows
-  for (int it = threadIdx.x; it < NZ * G; it += blockDim.x) {
-    const int j = it % G, zi = it / G;
-    const int base = AZ::slot(zi) * G + j;
-    cplx<T> u[Y2];
+  for (int it = threadIdx.x; it < NZ * VP; it += blockDim.x) {
+    const int v = it % VP, zi = it / VP;
+    const int base = AZ::slot(zi) * VP + v;
+    V u[Y2];
 #pragma unroll
-    for (int ka = 0; ka < Y2; ++ka) u[ka] = S[base + ka * ZS * G];
+    for (int ka = 0; ka < Y2; ++ka) u[ka] = S[base + ka * ZS * VP];
 #pragma unroll
-    for (int ka = 1; ka < Y2; ++ka) u[ka] = mul_conj(u[ka], twy[ka * Y1 + y1]);
-    DFT<Y2, true, T>::run(u);
+    for (int ka = 1; ka < Y2; ++ka) u[ka] = lmul_conj(u[ka], twy[ka * Y1 + y1]);
+    DFT<Y2, true, P>::run(u);
 #pragma unroll
-    for (int r = 0; r < Y2; ++r) S[base + r * ZS * G] = u[r];
+    for (int r = 0; r < Y2; ++r) S[base + r * ZS * VP] = u[r];
   }
   __syncthreads();
   // inverse z from natural order: element z ends in slot_of_freq(z)
-  step1<AZ, true>(S, Y2 * G * AZ::N2, twz, [](int it, int& base, int& es, int& j2) {
-    const int j = it % G, rest = it / G;
+  step1<AZ, true>(S, Y2 * VP * AZ::N2, twz, [](int it, int& base, int& es, int& j2) {
+    const int v = it % VP, rest = it / VP;
     j2 = rest % AZ::N2;
-    base = (rest / AZ::N2) * ZS * G + j;
-    es = G;
+    base = (rest / AZ::N2) * ZS * VP + v;
+    es = VP;
   });
   __syncthreads();
-  step2<AZ, true>(S, Y2 * G * AZ::N1, [](int it, int& base, int& es, int& k1) {
-    const int j = it % G, rest = it / G;
+  step2<AZ, true>(S, Y2 * VP * AZ::N1, [](int it, int& base, int& es, int& k1) {
+    const int v = it % VP, rest = it / VP;
     k1 = rest % AZ::N1;
-    base = (rest / AZ::N1) * ZS * G + j;
-    es = G;
+    base = (rest / AZ::N1) * ZS * VP + v;
+    es = VP;
   });
+
+  // nonlocal term, added to the tile in shared memory: V_nl psi(r) = sum over the entries
+  // at r of conj(exp(i (k+A).r_e)) sum_l beta_e[l] proj[a_e][l] (projector_all.hpp:182-232).
+  // A group of VP threads takes an entry.  The tile's records are in rank order (the first
+  // entry of every point, then the second ones, ...): within a rank no two entries share a
+  // point, and a barrier ends each rank, so every point adds its entries in a fixed order.
+  // A thread's next record, of this rank or the next one, is on its way while it works on
+  // the current (a dense shell of atoms has a dozen ranks of one or two records a thread).
+  if (proj_on) {
+    const int v = threadIdx.x % VP, eg = blockDim.x / VP, t0 = threadIdx.x / VP;
+    int e = e_first, e1 = k0 < k1 ? pj.rk_start[k0 + 1] : 0;
+    EntRec<T> re;
+    if (e < e1) re = pj.ent_rec_rk[e];
+    for (int k = k0; k < k1; ++k) {
+      const int next = e1 + t0, next_end = k + 1 < k1 ? pj.rk_start[k + 2] : e1;
+      __syncthreads();
+      if (e >= e1 && next < next_end) re = pj.ent_rec_rk[next];
+      while (e < e1) {
+        const EntRec<T> cur = re;
+        e += eg;
+        if (e < e1 || next < next_end) re = pj.ent_rec_rk[e < e1 ? e : next];
+        // t = sum over l in increasing order of beta[l] proj[l]
+        V t = {splat<P>(0.0), splat<P>(0.0)};
+        const V* pt = PT + cur.tseg * TG::PT_STRIDE + v;
+#pragma unroll
+        for (int l = 0; l < LMAX; ++l) {
+          // more atom segments in this tile than staged: projections from global memory
+          const V pv = pt_staged ? pt[l * VP] : projection(pj.seg_atom[s0 + cur.tseg], l, v);
+          const P b = splat_of(cur.beta[l]);
+          t.x = vfma(b, pv.x, t.x);
+          t.y = vfma(b, pv.y, t.y);
+        }
+        const P pr = splat_of(cur.ph[0]), pi = splat_of(cur.ph[1]), npi = splat_of(-cur.ph[1]);
+        V* dst = S + cur.off * VP + v;
+        const V h = *dst;
+        *dst = {h.x + vfma(t.x, pr, t.y * pi), h.y + vfma(t.y, pr, t.x * npi)};
+      }
+      e = next;
+      e1 = next_end;
+    }
+  }
   __syncthreads();
 
-  // epilogue: out = alpha (K psi + (V + vshift) psi + V_nl psi) + beta base, with
-  // V_nl psi(r) = sum over the entries at r of conj(exp(i (k+A).r_e)) sum_l
-  // beta_e[l] proj[a_e][l] (projector_all.hpp:182-232), summed by the point's owner.
-  // BE pieces of PV orbitals per thread, their loads issued together.
-  // pieces per thread whose loads are issued together: FP32 keeps four CTAs per SM
-  // within 64 registers a thread, FP64 (two CTAs per SM) takes more in flight
-  constexpr int BE = (TG::INV_MIN_CTAS == 4) ? 2 : 4;
-  cp_async_wait<0>();
-  __syncthreads();
-  if (!MODE_H) {
+  // epilogue: out = alpha (K psi + (V + vshift) psi + V_nl psi) + beta base
+  // BE lanes per thread whose loads are issued together
+  constexpr int BE = 4;
+  const P ar = splat_of(ep.alpha.x), ai = splat_of(ep.alpha.y), nai = splat_of(-ep.alpha.y);
+  // a lane of the output (orbital layout) at point p, orbitals m0 + jb ..
+  auto store = [&](long p, int jb, V w) {
+    cplx<T>* dst = out + p * ld_out + m0 + jb;
+    if (v16) {
+      *reinterpret_cast<V*>(dst) = flip(w);
+    } else {
+#pragma unroll
+      for (int k = 0; k < PV; ++k)
+        if (jb + k < gcount) dst[k] = lane_get(w, k);
+    }
+  };
+  // a lane of an orbital block at point p
+  auto load = [&](const cplx<T>* src, long ld, long p, int jb, bool wide) -> V {
+    V r;
+    if (wide) {
+      r = *reinterpret_cast<const V*>(src + p * ld + m0 + jb);
+    } else {
+      cplx<T> w[PV];
+#pragma unroll
+      for (int k = 0; k < PV; ++k) w[k] = (jb + k < gcount) ? src[p * ld + m0 + jb + k] : mk<T>(0, 0);
+      memcpy(&r, w, 16);
+    }
+    return r;
+  };
+  if constexpr (!MODE_H) {
     for (int q = threadIdx.x; q < TG::PTS * VP; q += blockDim.x) {
       const int v = q % VP, pt = q / VP;
       const int z = pt % NZ, r = pt / NZ;
       const long p = ((long)ix * NY + y1 + Y1 * r) * NZ + z;
-      const int jb = v * PV;
-      const int sl = (r * ZS + AZ::slot_of_freq(z)) * G + jb;
-      cplx<T> h[PV];
-#pragma unroll
-      for (int k = 0; k < PV; ++k) h[k] = ep.alpha * S[sl + k];
-      if (v16) {
-        float4 w;
-        memcpy(&w, h, 16);
-        *reinterpret_cast<float4*>(out + p * ld_out + m0 + jb) = w;
-      } else {
-#pragma unroll
-        for (int k = 0; k < PV; ++k)
-          if (jb + k < gcount) out[p * ld_out + m0 + jb + k] = h[k];
-      }
+      const V h = S[(r * ZS + AZ::slot_of_freq(z)) * VP + v];
+      store(p, v * PV, {vfma(h.x, ar, h.y * nai), vfma(h.x, ai, h.y * ar)});
     }
-    return;
-  }
+  } else
   for (int q0 = threadIdx.x; q0 < TG::PTS * VP; q0 += BE * blockDim.x) {
-    cplx<T> x[BE][PV];
+    V x[BE];
     T vp[BE];
-    // the first entry record of each point, fetched with the orbitals
-    EntRec<T> r0[BE];
-    int k0[BE], k1[BE];
 #pragma unroll
     for (int b = 0; b < BE; ++b) {
       const int q = q0 + b * blockDim.x;
-      k0[b] = k1[b] = 0;
       if (q >= TG::PTS * VP) continue;
       const int v = q % VP, pt = q / VP;
       const int z = pt % NZ, r = pt / NZ;
       const long p = ((long)ix * NY + y1 + Y1 * r) * NZ + z;
-      const int jb = v * PV;
-      if (proj_on) {
-        k0[b] = TP[pt];
-        k1[b] = TP[pt + 1];
-        // FP32 reads records from global memory: start the first one now; FP64 has
-        // them in shared memory already
-        if (!TG::PREFETCH && k1[b] > k0[b]) r0[b] = rec[k0[b] + rbase];
-      }
       vp[b] = ep.V[p] + ep.vshift;
-      if (TG::PREFETCH && v16) {
-#pragma unroll
-        for (int k = 0; k < PV; ++k) x[b][k] = P[pt * G + jb + k];
-      } else if (v16) {
-        const float4 w = *reinterpret_cast<const float4*>(in + p * ld_in + m0 + jb);
-        memcpy(x[b], &w, 16);
-      } else {
-#pragma unroll
-        for (int k = 0; k < PV; ++k) x[b][k] = (jb + k < gcount) ? in[p * ld_in + m0 + jb + k] : mk<T>(0, 0);
-      }
+      x[b] = load(in, ld_in, p, v * PV, v16);
     }
 #pragma unroll
     for (int b = 0; b < BE; ++b) {
@@ -782,86 +856,29 @@ __device__ __forceinline__ void tile_inv_body(int bx, int by, const cplx<T>* __r
       const int v = q % VP, pt = q / VP;
       const int z = pt % NZ, r = pt / NZ;
       const long p = ((long)ix * NY + y1 + Y1 * r) * NZ + z;
-      const int jb = v * PV;
-      const int sl = (r * ZS + AZ::slot_of_freq(z)) * G + jb;
-      cplx<T> h[PV];
-#pragma unroll
-      for (int k = 0; k < PV; ++k) h[k] = S[sl + k];
-      if (proj_on && pt_staged) {
-        for (int kk = k0[b]; kk < k1[b]; ++kk) {
-          const EntRec<T> re = (!TG::PREFETCH && kk == k0[b]) ? r0[b] : rec[kk + rbase];
-          const cplx<T> ph = mk<T>(re.ph[0], re.ph[1]);
-          const cplx<T>* pt = PT + re.tseg * TG::PT_STRIDE + jb;
-          // per orbital k, t_k = sum over l in increasing order; the PV orbitals of
-          // one l are adjacent (one 16-byte load)
-          cplx<T> t[PV];
-#pragma unroll
-          for (int k = 0; k < PV; ++k) t[k] = mk<T>(0, 0);
-#pragma unroll
-          for (int l = 0; l < LMAX; ++l) {
-#pragma unroll
-            for (int k = 0; k < PV; ++k) {
-              const cplx<T> pv = pt[l * G + k];
-              t[k].x = fma(re.beta[l], pv.x, t[k].x);
-              t[k].y = fma(re.beta[l], pv.y, t[k].y);
-            }
-          }
-#pragma unroll
-          for (int k = 0; k < PV; ++k) h[k] = h[k] + mul_conj(t[k], ph);
-        }
-      } else if (proj_on) {
-        // more atom segments in this tile than staged: projections from global memory
-        for (int kk = k0[b]; kk < k1[b]; ++kk) {
-          const EntRec<T> re = (!TG::PREFETCH && kk == k0[b]) ? r0[b] : rec[kk + rbase];
-          const cplx<T> ph = mk<T>(re.ph[0], re.ph[1]);
-#pragma unroll
-          for (int k = 0; k < PV; ++k) {
-            cplx<T> t = mk<T>(0, 0);
-#pragma unroll
-            for (int l = 0; l < LMAX; ++l) {
-              cplx<T> pv = mk<T>(0, 0);
-              if (l < pj.L && jb + k < gcount) {
-                const double2 d = ld_l2(pj.proj + ((long)pj.seg_atom[s0 + re.tseg] * pj.L + l) * M + m0 + jb + k);
-                pv = mk<T>((T)d.x, (T)d.y);
-              }
-              t.x = fma(re.beta[l], pv.x, t.x);
-              t.y = fma(re.beta[l], pv.y, t.y);
-            }
-            h[k] = h[k] + mul_conj(t, ph);
-          }
-        }
+      V h = S[(r * ZS + AZ::slot_of_freq(z)) * VP + v];
+      const V xv = flip(x[b]);
+      const P vs = splat_of(vp[b]);
+      h = {vfma(vs, xv.x, h.x), vfma(vs, xv.y, h.y)};
+      V o = {vfma(h.x, ar, h.y * nai), vfma(h.x, ai, h.y * ar)};
+      if (ep.base) {
+        const V bb = flip(load(ep.base, ep.ld_base, p, v * PV, b16));
+        const P br = splat_of(ep.beta.x), bi = splat_of(ep.beta.y), nbi = splat_of(-ep.beta.y);
+        o.x = o.x + vfma(bb.x, br, bb.y * nbi);
+        o.y = o.y + vfma(bb.x, bi, bb.y * br);
       }
-#pragma unroll
-      for (int k = 0; k < PV; ++k) {
-        h[k].x = fma(vp[b], x[b][k].x, h[k].x);
-        h[k].y = fma(vp[b], x[b][k].y, h[k].y);
-        h[k] = ep.alpha * h[k];
-        if (ep.base) {
-          const cplx<T> bb = (jb + k < gcount) ? ep.base[p * ep.ld_base + m0 + jb + k] : mk<T>(0, 0);
-          h[k] = h[k] + ep.beta * bb;
-        }
-      }
-      if (v16) {
-        float4 w;
-        memcpy(&w, h, 16);
-        *reinterpret_cast<float4*>(out + p * ld_out + m0 + jb) = w;
-      } else {
-#pragma unroll
-        for (int k = 0; k < PV; ++k)
-          if (jb + k < gcount) out[p * ld_out + m0 + jb + k] = h[k];
-      }
+      store(p, v * PV, o);
     }
   }
 }
 
 template <typename T, int NX, int NY, int NZ, int MODE_H = 1>
 __global__ void __launch_bounds__(256, TileGeom<T, NX, NY, NZ>::INV_MIN_CTAS)
-    k_tile_inv(const cplx<T>* __restrict__ tmp, const cplx<T>* __restrict__ in, long ld_in,
+    k_tile_inv(const Lane<T>* __restrict__ tmp, const cplx<T>* __restrict__ in, long ld_in,
                cplx<T>* __restrict__ out, long ld_out, int M, const cplx<T>* __restrict__ tw_y,
-               const cplx<T>* __restrict__ tw_z, ProjView<T> pj, EpiParams<T> ep, int rec_cap, int seg_cap,
-               int vec) {
+               const cplx<T>* __restrict__ tw_z, ProjView<T> pj, EpiParams<T> ep, int seg_cap, int vec) {
   tile_inv_body<T, NX, NY, NZ, MODE_H>(blockIdx.x, blockIdx.y, tmp, in, ld_in, out, ld_out, M, tw_y, tw_z, pj, ep,
-                                       rec_cap, seg_cap, vec);
+                                       seg_cap, vec);
 }
 
 }  // namespace inqb
