@@ -125,10 +125,10 @@ int set_kA(inqb_ctx* ctx, const double kA[3], void* stream) {
   return INQB_OK;
 }
 
-// One H application: out = alpha * H in + beta * base.
+// One H application: out = alpha * H in + beta * base - minus (minus optional).
 int apply(inqb_ctx* ctx, int mode, const void* in, long ld_in, void* out, long ld_out, int M, const void* base,
           long ld_base, const double alpha[2], const double beta[2], void* stream, void* fourier_out = nullptr,
-          BatchCellDesc* batch_cell = nullptr) {
+          BatchCellDesc* batch_cell = nullptr, const void* minus = nullptr, long ld_minus = 0) {
   INQB_TRY(reserve(ctx, M));
   if (!ctx->proj_phases_valid) {
     INQB_TRY(update_phases(ctx, stream));
@@ -146,6 +146,8 @@ int apply(inqb_ctx* ctx, int mode, const void* in, long ld_in, void* out, long l
   a.V = ctx->d_V.ptr;
   a.base = base;
   a.ld_base = ld_base;
+  a.minus = minus;
+  a.ld_minus = ld_minus;
   a.alpha[0] = alpha[0];
   a.alpha[1] = alpha[1];
   a.beta[0] = beta[0];
@@ -1327,13 +1329,13 @@ int inqb_crank_nicolson_step(inqb_ctx* ctx, void* psi, int M, int ld, double dt,
   INQB_TRY(reserve(ctx, M));
   const size_t blk = (size_t)ctx->N * M * ctx->elem_bytes();
   INQB_TRY(ctx->d_cn.ensure(3 * blk));
-  INQB_TRY(ctx->d_cnred.ensure(sizeof(double) * 5 * (size_t)M));
+  INQB_TRY(ctx->d_cnred.ensure(sizeof(double) * (sd_partial_doubles(M) + (size_t)M)));
   char* w = static_cast<char*>(ctx->d_cn.ptr);
   void* rhs = w;
   void* r = w + blk;
   void* hsd = w + 2 * blk;
-  double* acc = ctx->d_cnred.as<double>();
-  double* normres = acc + 4 * (size_t)M;
+  double* sums = ctx->d_cnred.as<double>();
+  double* normres = sums + sd_partial_doubles(M);
   const long Mi = M;
   cudaStream_t st = (cudaStream_t)stream;
   // rhs = (1 - i dt/2 H(t)) psi  (op_rhs, crank_nicolson.hpp:49-55)
@@ -1349,17 +1351,11 @@ int inqb_crank_nicolson_step(inqb_ctx* ctx, void* psi, int M, int ld, double dt,
     // steepest_descent (steepest_descent.hpp:22-80): five steps, no preconditioner
     for (int step = 0; step < 5; step++) {
       // r = (1 + i dt/2 H) phi - rhs
-      INQB_TRY(apply(ctx, LaunchArgs::H, psi, ld, r, Mi, M, psi, ld, fl, one, stream));
-      {
-        const double a[2][2] = {{1.0, 0.0}, {-1.0, 0.0}};
-        const void* x[2] = {r, rhs};
-        const long ldx[2] = {Mi, Mi};
-        INQB_TRY(launch_lincomb(ctx->precision, ctx->N, M, 2, a, x, ldx, r, Mi, stream));
-      }
+      INQB_TRY(apply(ctx, LaunchArgs::H, psi, ld, r, Mi, M, psi, ld, fl, one, stream, nullptr, nullptr, rhs, Mi));
       // hsd = (1 + i dt/2 H) r
       INQB_TRY(apply(ctx, LaunchArgs::H, r, Mi, hsd, Mi, M, r, Mi, fl, one, stream));
-      INQB_TRY(launch_sd_sums(ctx->precision, r, hsd, Mi, M, ctx->N, acc, stream));
-      INQB_TRY(launch_sd_update(ctx->precision, psi, ld, r, Mi, M, ctx->N, acc, ctx->dV, normres, stream));
+      INQB_TRY(launch_sd_sums(ctx->precision, r, hsd, Mi, M, ctx->N, sums, stream));
+      INQB_TRY(launch_sd_update(ctx->precision, psi, ld, r, Mi, M, ctx->N, sums, ctx->dV, normres, stream));
     }
     k++;
     INQB_CUDA_TRY(cudaMemcpyAsync(hres.data(), normres, sizeof(double) * M, cudaMemcpyDeviceToHost, st));
@@ -1389,13 +1385,13 @@ int inqb_crank_nicolson_scf_step(inqb_ctx* ctx, void* psi, int M, int ld, double
   const long N = ctx->N;
   const size_t blk = (size_t)N * M * ctx->elem_bytes();
   INQB_TRY(ctx->d_cn.ensure(3 * blk));
-  INQB_TRY(ctx->d_cnred.ensure(sizeof(double) * 5 * (size_t)M));
+  INQB_TRY(ctx->d_cnred.ensure(sizeof(double) * (sd_partial_doubles(M) + (size_t)M)));
   char* wb = static_cast<char*>(ctx->d_cn.ptr);
   void* rhs = wb;
   void* r = wb + blk;
   void* hsd = wb + 2 * blk;
-  double* acc = ctx->d_cnred.as<double>();
-  double* normres = acc + 4 * (size_t)M;
+  double* sums = ctx->d_cnred.as<double>();
+  double* normres = sums + sd_partial_doubles(M);
   PotWork pw;
   INQB_TRY(pot_work(ctx, pw));
   MixWork mw;
@@ -1420,16 +1416,10 @@ int inqb_crank_nicolson_scf_step(inqb_ctx* ctx, void* psi, int M, int ld, double
     // inqb_crank_nicolson_step) from the current psi
     INQB_TRY(ks_potential_dev(ctx, rho, vion, theory, pw, stream));
     for (int step = 0; step < 5; step++) {
-      INQB_TRY(apply(ctx, LaunchArgs::H, psi, ld, r, Mi, M, psi, ld, fl, one, stream));
-      {
-        const double a[2][2] = {{1.0, 0.0}, {-1.0, 0.0}};
-        const void* x[2] = {r, rhs};
-        const long ldx[2] = {Mi, Mi};
-        INQB_TRY(launch_lincomb(ctx->precision, N, M, 2, a, x, ldx, r, Mi, stream));
-      }
+      INQB_TRY(apply(ctx, LaunchArgs::H, psi, ld, r, Mi, M, psi, ld, fl, one, stream, nullptr, nullptr, rhs, Mi));
       INQB_TRY(apply(ctx, LaunchArgs::H, r, Mi, hsd, Mi, M, r, Mi, fl, one, stream));
-      INQB_TRY(launch_sd_sums(ctx->precision, r, hsd, Mi, M, N, acc, stream));
-      INQB_TRY(launch_sd_update(ctx->precision, psi, ld, r, Mi, M, N, acc, ctx->dV, normres, stream));
+      INQB_TRY(launch_sd_sums(ctx->precision, r, hsd, Mi, M, N, sums, stream));
+      INQB_TRY(launch_sd_update(ctx->precision, psi, ld, r, Mi, M, N, sums, ctx->dV, normres, stream));
     }
     // the new density and dV sum |rho - new| / nelec (crank_nicolson.hpp:98-99)
     INQB_TRY(sharded_density(ctx, psi, ld, M, occ, mw.fresh, stream));

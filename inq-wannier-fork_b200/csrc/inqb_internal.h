@@ -220,7 +220,7 @@ struct inqb_ctx {
   inqb::DevBuf d_nlpart;        // per-chunk nonlocal moments of the dH/dA inner products
   inqb::DevBuf d_adjL;          // adjoint step: H^j lambda (4 blocks), Xi, spare
   inqb::DevBuf d_cn;            // Crank-Nicolson: rhs, residual, (1 + i dt/2 H) residual
-  inqb::DevBuf d_cnred;         // Crank-Nicolson: 4 sums and the residual norm per orbital
+  inqb::DevBuf d_cnred;         // Crank-Nicolson: the sums' partials and the residual norm per orbital
   inqb::DevBuf d_scf;           // ETRS with self-consistency: the saved half step, H^k phi
   inqb_density_reduce_fn density_reduce = nullptr;  // cross-rank density sum (orbital sharding)
   void* density_reduce_user = nullptr;

@@ -74,7 +74,9 @@ struct EpiParams {
   T vshift;                 // added to V (1/2 |k+A|^2 when the Fourier mask is on)
   const cplx<T>* base;      // optional [N][ld_base]
   long ld_base;
-  cplx<T> alpha, beta;      // out = alpha * H in + beta * base
+  const cplx<T>* minus;     // optional [N][ld_minus]
+  long ld_minus;
+  cplx<T> alpha, beta;      // out = alpha * H in + beta * base - minus
 };
 
 // One cell of the persistent batch launch (batch.h): every argument the three tile
@@ -163,6 +165,7 @@ int launch_h_impl(const LaunchArgs& a) {
   const int vin = aligned16(a.in, a.ld_in, esz);
   const int vout = aligned16(a.out, a.ld_out, esz);
   const int vbase = a.base && aligned16(a.base, a.ld_base, esz);
+  const int vminus = a.minus && aligned16(a.minus, a.ld_minus, esz);
   int ysplit = a.ysplit > 0 ? a.ysplit : TG::YSPLIT;
   if (TG::Y1 % ysplit != 0) return fail(INQB_ERR_INVALID, "schedule: ysplit must divide the tiles per plane");
   const int thr_default[3] = {TG::THREADS, TG::X_THREADS, TG::Z_THREADS};
@@ -212,6 +215,8 @@ int launch_h_impl(const LaunchArgs& a) {
     ep.vshift = a.fourier_mask ? (T)(0.5 * kA2) : (T)0;
     ep.base = (const cplx<T>*)a.base;
     ep.ld_base = a.ld_base;
+    ep.minus = (const cplx<T>*)a.minus;
+    ep.ld_minus = a.ld_minus;
     ep.alpha = mk<T>((T)a.alpha[0], (T)a.alpha[1]);
     ep.beta = mk<T>((T)a.beta[0], (T)a.beta[1]);
     if (TG::smem_inv(seg_cap) > TG::SMEM_MAX)
@@ -221,7 +226,7 @@ int launch_h_impl(const LaunchArgs& a) {
       auto* d = reinterpret_cast<BatchCellDesc*>(a.batch_cell);
       d->kind = batch_kind(NX, NY, NZ);
       if (d->kind < 0) return fail(INQB_ERR_UNSUPPORTED, "grid not compiled into the persistent batch kernel");
-      if (sep || (pj.nproj > 0 && pj.slots == nullptr) || a.fourier_out || a.base)
+      if (sep || (pj.nproj > 0 && pj.slots == nullptr) || a.fourier_out || a.base || a.minus)
         return fail(INQB_ERR_UNSUPPORTED, "the persistent batch launch runs the fused projection only");
       BatchCell<T> c;
       c.in = (const cplx<T>*)a.in;
@@ -271,7 +276,7 @@ int launch_h_impl(const LaunchArgs& a) {
     if (a.events[4]) INQB_CUDA_TRY(cudaEventRecord((cudaEvent_t)a.events[4], st));
     INQB_TRY(launch_chained(k_tile_inv<T, NX, NY, NZ, 1>, ginv, thr[2], TG::smem_inv(seg_cap), st, tmp,
             (const cplx<T>*)a.in, a.ld_in, (cplx<T>*)a.out, a.ld_out, a.M, twy, twz, pj, ep, seg_cap,
-            (vin && vout) | (vbase << 1)));
+            (vin && vout) | (vbase << 1) | (vminus << 2)));
     if (a.events[5]) INQB_CUDA_TRY(cudaEventRecord((cudaEvent_t)a.events[5], st));
   } else if (a.mode == LaunchArgs::POISSON) {
     // solvers::poisson on M complex fields: forward z and inner y, then the outer y

@@ -19,6 +19,8 @@ struct LaunchArgs {
   double kA_cart[3] = {};           // cartesian k + A
   const void* base = nullptr;       // optional epilogue base (out = alpha H in + beta base)
   long ld_base = 0;
+  const void* minus = nullptr;      // optional block subtracted (out = alpha H in + beta base - minus)
+  long ld_minus = 0;
   double alpha[2] = {1.0, 0.0};
   double beta[2] = {0.0, 0.0};
   void* stream = nullptr;

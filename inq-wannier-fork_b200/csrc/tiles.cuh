@@ -680,8 +680,9 @@ __device__ __forceinline__ void tile_inv_body(int bx, int by, const Lane<T>* __r
   const int grp = bx, ix = by / Y1, y1 = by % Y1;
   const int m0 = grp * G;
   const int gcount = min(G, M - m0);
-  // vec: bit 0, the input and output blocks take 16-byte accesses; bit 1, the base does
-  const bool v16 = (vec & 1) && gcount == G, b16 = (vec & 2) && gcount == G;
+  // vec: bit 0, the input and output blocks take 16-byte accesses; bits 1 and 2, the base
+  // and the subtracted block do
+  const bool v16 = (vec & 1) && gcount == G, b16 = (vec & 2) && gcount == G, s16 = (vec & 4) && gcount == G;
 
   for (int i = threadIdx.x; i < NY; i += blockDim.x) twy[i] = lane_splat(tw_y[i]);
   for (int i = threadIdx.x; i < NZ; i += blockDim.x) twz[i] = lane_splat(tw_z[i]);
@@ -799,7 +800,7 @@ __device__ __forceinline__ void tile_inv_body(int bx, int by, const Lane<T>* __r
   }
   __syncthreads();
 
-  // epilogue: out = alpha (K psi + (V + vshift) psi + V_nl psi) + beta base
+  // epilogue: out = alpha (K psi + (V + vshift) psi + V_nl psi) + beta base - minus
   // BE lanes per thread whose loads are issued together
   constexpr int BE = 4;
   const P ar = splat_of(ep.alpha.x), ai = splat_of(ep.alpha.y), nai = splat_of(-ep.alpha.y);
@@ -867,6 +868,7 @@ __device__ __forceinline__ void tile_inv_body(int bx, int by, const Lane<T>* __r
         o.x = o.x + vfma(bb.x, br, bb.y * nbi);
         o.y = o.y + vfma(bb.x, bi, bb.y * br);
       }
+      if (ep.minus) o = o - flip(load(ep.minus, ep.ld_minus, p, v * PV, s16));
       store(p, v * PV, o);
     }
   }
