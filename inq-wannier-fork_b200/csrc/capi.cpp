@@ -208,10 +208,10 @@ int apply_events(inqb_ctx* ctx, const void* in, void* out, int M, const double a
   return st;
 }
 
-// psi <- sum_{k <= order} (f H)^k / k! psi by Horner's rule:
+// out = sum_{k <= order} (f H)^k / k! psi by Horner's rule (out may be psi; order >= 1):
 // y = psi; for k = order..1: y = psi + (f/k) H y.  (exponential.hpp:21-34)
-int exponential(inqb_ctx* ctx, void* psi, int M, long ld, double fre, double fim, int order, void* stream) {
-  if (order < 1) return INQB_OK;
+int exponential(inqb_ctx* ctx, const void* psi, long ld, void* out, long ld_out, int M, double fre, double fim, int order,
+                void* stream) {
   INQB_TRY(ctx->d_work.ensure((size_t)ctx->N * M * ctx->elem_bytes()));
   void* y = ctx->d_work.ptr;
   const double one[2] = {1.0, 0.0};
@@ -219,9 +219,7 @@ int exponential(inqb_ctx* ctx, void* psi, int M, long ld, double fre, double fim
     const double alpha[2] = {fre / k, fim / k};
     const void* in = (k == order) ? psi : y;
     const long ldi = (k == order) ? ld : M;
-    void* out = (k == 1) ? psi : y;
-    const long ldo = (k == 1) ? ld : M;
-    INQB_TRY(apply(ctx, LaunchArgs::H, in, ldi, out, ldo, M, psi, ld, alpha, one, stream));
+    INQB_TRY(apply(ctx, LaunchArgs::H, in, ldi, k == 1 ? out : y, k == 1 ? ld_out : M, M, psi, ld, alpha, one, stream));
   }
   return INQB_OK;
 }
@@ -1045,7 +1043,7 @@ int inqb_exponential(inqb_ctx* ctx, void* psi, int M, int ld, double f_re, doubl
   INQB_TRY(check_block(ctx, psi, M, ld));
   if (order < 0 || order > 64) return fail(INQB_ERR_INVALID, "order out of range");
   INQB_GUARD(ctx);
-  return exponential(ctx, psi, M, ld, f_re, f_im, order, stream);
+  return order < 1 ? INQB_OK : exponential(ctx, psi, ld, psi, ld, M, f_re, f_im, order, stream);
 }
 
 int inqb_etrs_step(inqb_ctx* ctx, void* psi, int M, int ld, double dt, const double kA_t_cov[3],
@@ -1055,9 +1053,9 @@ int inqb_etrs_step(inqb_ctx* ctx, void* psi, int M, int ld, double dt, const dou
   if (!kA_t_cov || !kA_tdt_cov || !std::isfinite(dt)) return fail(INQB_ERR_INVALID, "bad step arguments");
   INQB_GUARD(ctx);
   INQB_TRY(set_kA(ctx, kA_t_cov, stream));
-  INQB_TRY(exponential(ctx, psi, M, ld, 0.0, dt / 2.0, 4, stream));
+  INQB_TRY(exponential(ctx, psi, ld, psi, ld, M, 0.0, dt / 2.0, 4, stream));
   INQB_TRY(set_kA(ctx, kA_tdt_cov, stream));
-  INQB_TRY(exponential(ctx, psi, M, ld, 0.0, dt / 2.0, 4, stream));
+  INQB_TRY(exponential(ctx, psi, ld, psi, ld, M, 0.0, dt / 2.0, 4, stream));
   return INQB_OK;
 }
 
@@ -1166,8 +1164,7 @@ int inqb_etrs_scf_step(inqb_ctx* ctx, void* psi, int M, int ld, double dt, const
   double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   int done_iters = 0;
   for (int iscf = 0; iscf < nscf; iscf++) {
-    INQB_TRY(copy_block(save, M, psi, ld, M, N, esz, stream));
-    INQB_TRY(exponential(ctx, psi, M, ld, 0.0, 0.5 * dt, 4, stream));
+    INQB_TRY(exponential(ctx, save, M, psi, ld, M, 0.0, 0.5 * dt, 4, stream));
     INQB_CUDA_TRY(cudaMemcpyAsync(w.rho_old, rho, sizeof(double) * N, cudaMemcpyDeviceToDevice,
                                   (cudaStream_t)stream));
     INQB_TRY(sharded_density(ctx, psi, ld, M, occ, rho, stream));

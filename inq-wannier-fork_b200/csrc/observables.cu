@@ -16,21 +16,36 @@
 
 namespace inqb {
 
-template <typename T>
-__global__ void k_density(const cplx<T>* __restrict__ psi, long ld, int M, long N, const double* __restrict__ occ,
-                          double* __restrict__ rho) {
-  const int lane = threadIdx.x & 31;
-  const long warp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
-  for (long p = warp; p < N; p += nwarps) {
-    double acc = 0.0;
-    for (int m = lane; m < M; m += 32) {
-      const cplx<T> v = psi[p * ld + m];
-      acc += occ[m] * ((double)v.x * (double)v.x + (double)v.y * (double)v.y);
+// A group of LPP lanes per grid point (16 where M <= 16, so that no lane idles), four points
+// at a time: their loads are in flight together, which the one-point loop's reduction
+// chain prevented.
+template <typename T, int LPP>
+__global__ void __launch_bounds__(256)
+    k_density(const cplx<T>* __restrict__ psi, long ld, int M, long N, const double* __restrict__ occ,
+              double* __restrict__ rho) {
+  constexpr int PTS = 4;
+  const int lane = threadIdx.x & (LPP - 1);
+  const long grp = ((long)blockIdx.x * blockDim.x + threadIdx.x) / LPP;
+  const long ngrp = ((long)gridDim.x * blockDim.x) / LPP;
+  // every lane of a warp runs the same number of iterations (the shuffles below)
+  const long step = ngrp * PTS, pend = (N + step - 1) / step * step;
+  for (long p0 = grp * PTS; p0 < pend; p0 += step) {
+    double acc[PTS] = {0.0, 0.0, 0.0, 0.0};
+    for (int m = lane; m < M; m += LPP) {
+      cplx<T> v[PTS];
+#pragma unroll
+      for (int u = 0; u < PTS; ++u) v[u] = (p0 + u < N) ? psi[(p0 + u) * ld + m] : mk<T>(0, 0);
+      const double o = occ[m];
+#pragma unroll
+      for (int u = 0; u < PTS; ++u) acc[u] += o * ((double)v[u].x * (double)v[u].x + (double)v[u].y * (double)v[u].y);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) rho[p] = acc;
+    for (int o = LPP / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int u = 0; u < PTS; ++u) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], o);
+#pragma unroll
+    for (int u = 0; u < PTS; ++u)
+      if (lane == u && p0 + u < N) rho[p0 + u] = acc[u];
   }
 }
 
@@ -459,8 +474,12 @@ __global__ void __launch_bounds__(256, TN == 4 ? 2 : 3)
 // ---------------------------------------------------------------- launchers
 template <typename T>
 static int density_impl(const void* psi, long ld, int M, long N, const double* occ, double* rho, cudaStream_t st) {
-  const int blocks = (int)std::min<long>((N * 32 + 255) / 256, 148L * 16);
-  k_density<T><<<blocks, 256, 0, st>>>((const cplx<T>*)psi, ld, M, N, occ, rho);
+  const int lpp = M <= 16 ? 16 : 32;
+  const int blocks = (int)std::min<long>((N * lpp + 1023) / 1024, 148L * 8);
+  if (M <= 16)
+    k_density<T, 16><<<blocks, 256, 0, st>>>((const cplx<T>*)psi, ld, M, N, occ, rho);
+  else
+    k_density<T, 32><<<blocks, 256, 0, st>>>((const cplx<T>*)psi, ld, M, N, occ, rho);
   INQB_CUDA_TRY(cudaGetLastError());
   return INQB_OK;
 }
@@ -484,6 +503,7 @@ __global__ void __launch_bounds__(256)
   const long p0 = (long)blockIdx.x * pts_per_block, p1 = min(N, p0 + pts_per_block);
   double vr = 0.0, vi = 0.0, nn = 0.0;
   if (m < M) {
+#pragma unroll 4
     for (long p = p0 + tp; p < p1; p += 8) {
       const cplx<T> a = hpsi[p * ld + m], b = psi[p * ld + m];
       const double ax = a.x, ay = a.y, bx = b.x, by = b.y;

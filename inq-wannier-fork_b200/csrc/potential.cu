@@ -29,6 +29,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 
 #include "dft.cuh"
 #include "inqb_internal.h"
@@ -164,6 +165,32 @@ __global__ void k_shift2(const cplx<T>* __restrict__ y, long ldy, cplx<T>* __res
   }
 }
 
+// The same on blocks without padding (every ld = M, 16-byte aligned): one run of n 16-byte
+// pieces and no row index (a 64-bit division per element otherwise).
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+    k_shift2_flat(const cplx<T>* __restrict__ y, cplx<T>* __restrict__ a1, cplx<T>* __restrict__ a2, long n, double c1r,
+                  double c1i, double c2r, double c2i) {
+  constexpr int PV = 16 / (int)sizeof(cplx<T>);
+  struct alignas(16) Piece {
+    cplx<T> v[PV];
+  };
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    const Piece q = reinterpret_cast<const Piece*>(y)[i];
+    Piece u = reinterpret_cast<Piece*>(a1)[i], w = reinterpret_cast<Piece*>(a2)[i];
+#pragma unroll
+    for (int k = 0; k < PV; ++k) {
+      const double vx = q.v[k].x, vy = q.v[k].y;
+      u.v[k].x = (T)((double)u.v[k].x + c1r * vx - c1i * vy);
+      u.v[k].y = (T)((double)u.v[k].y + c1r * vy + c1i * vx);
+      w.v[k].x = (T)((double)w.v[k].x + c2r * vx - c2i * vy);
+      w.v[k].y = (T)((double)w.v[k].y + c2r * vy + c2i * vx);
+    }
+    reinterpret_cast<Piece*>(a1)[i] = u;
+    reinterpret_cast<Piece*>(a2)[i] = w;
+  }
+}
+
 // ---- Broyden density mixer (src/mixers/broyden.hpp:107-160), FP64 vectors of n values
 
 // ff = vout - vin, kept in f_old (the reference sets f_old = ff after using the old
@@ -264,19 +291,29 @@ int launch_absdiff(const double* a, const double* b, long N, double* partial, do
   return INQB_OK;
 }
 
+template <typename T>
+static int shift2_impl(const void* y, long ldy, void* a1, long ld1, void* a2, long ld2, int M, long N,
+                       const double c1[2], const double c2[2], cudaStream_t st) {
+  constexpr int PV = 16 / (int)sizeof(cplx<T>);
+  const bool flat = ldy == M && ld1 == M && ld2 == M && N * M % PV == 0 &&
+                    ((uintptr_t)y | (uintptr_t)a1 | (uintptr_t)a2) % 16 == 0;
+  const long total = flat ? N * M / PV : N * M;
+  const int nb = (int)std::max<long>(1, std::min<long>((total + kThreads - 1) / kThreads, 148L * 32));
+  if (flat)
+    k_shift2_flat<T><<<nb, kThreads, 0, st>>>((const cplx<T>*)y, (cplx<T>*)a1, (cplx<T>*)a2, total, c1[0], c1[1], c2[0],
+                                              c2[1]);
+  else
+    k_shift2<T><<<nb, kThreads, 0, st>>>((const cplx<T>*)y, ldy, (cplx<T>*)a1, ld1, (cplx<T>*)a2, ld2, M, N, c1[0],
+                                         c1[1], c2[0], c2[1]);
+  INQB_CUDA_TRY(cudaGetLastError());
+  return INQB_OK;
+}
+
 int launch_shift2(int precision, const void* y, long ldy, void* a1, long ld1, void* a2, long ld2, int M, long N,
                   const double c1[2], const double c2[2], void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
-  const long total = N * M;
-  const int nb = (int)std::max<long>(1, std::min<long>((total + kThreads - 1) / kThreads, 148L * 32));
-  if (precision == INQB_FP64)
-    k_shift2<double><<<nb, kThreads, 0, st>>>((const cplx<double>*)y, ldy, (cplx<double>*)a1, ld1,
-                                               (cplx<double>*)a2, ld2, M, N, c1[0], c1[1], c2[0], c2[1]);
-  else
-    k_shift2<float><<<nb, kThreads, 0, st>>>((const cplx<float>*)y, ldy, (cplx<float>*)a1, ld1,
-                                              (cplx<float>*)a2, ld2, M, N, c1[0], c1[1], c2[0], c2[1]);
-  INQB_CUDA_TRY(cudaGetLastError());
-  return INQB_OK;
+  return precision == INQB_FP64 ? shift2_impl<double>(y, ldy, a1, ld1, a2, ld2, M, N, c1, c2, st)
+                                : shift2_impl<float>(y, ldy, a1, ld1, a2, ld2, M, N, c1, c2, st);
 }
 
 int launch_broyden_diff(const double* vin, const double* vout, double* f_old, double* vin_old, double* df,

@@ -828,6 +828,7 @@ __device__ __forceinline__ void tile_inv_body(int bx, int by, const Lane<T>* __r
     }
     return r;
   };
+  const bool own = ep.base == in && ep.ld_base == ld_in;
   if constexpr (!MODE_H) {
     for (int q = threadIdx.x; q < TG::PTS * VP; q += blockDim.x) {
       const int v = q % VP, pt = q / VP;
@@ -863,7 +864,8 @@ __device__ __forceinline__ void tile_inv_body(int bx, int by, const Lane<T>* __r
       h = {vfma(vs, xv.x, h.x), vfma(vs, xv.y, h.y)};
       V o = {vfma(h.x, ar, h.y * nai), vfma(h.x, ai, h.y * ar)};
       if (ep.base) {
-        const V bb = flip(load(ep.base, ep.ld_base, p, v * PV, b16));
+        // base the input block itself (a Taylor series' first term, 1 + c H): already here
+        const V bb = own ? xv : flip(load(ep.base, ep.ld_base, p, v * PV, b16));
         const P br = splat_of(ep.beta.x), bi = splat_of(ep.beta.y), nbi = splat_of(-ep.beta.y);
         o.x = o.x + vfma(bb.x, br, bb.y * nbi);
         o.y = o.y + vfma(bb.x, bi, bb.y * br);
