@@ -437,25 +437,139 @@ __global__ void k_jade_change(const double* __restrict__ delta, int nsteps, int 
 }
 
 // ------------------------------------------------------------------ jade in one cluster
-// All sweeps in one launch of one thread-block cluster that holds the six matrices and u in
-// its shared memory (row r in CTA r % CL).  A rotation step is bound by latency, not by
-// bytes: the 3 x 3 eigenproblem is a serial chain, and the launch, the row gathers from L2
-// and the block reductions around it cost several times as much when every step is a launch
-// of its own.  Here a step is one cluster barrier, rows over distributed shared memory, and
-// a group of seven warps per pair: warp k sums and rotates matrix k (warp 6: u).
-//   kJG = 7 warps of a group; E: elements of a row per lane (M <= 32 E); GMAX: groups
-constexpr int kJG = 7 * 32;
+// jacobi3_top with its iteration in FP32 and the eigenvector then refined in FP64.  The
+// serial chain of FP64 roots and divisions made the Jacobi iteration the longest part of a
+// rotation step (5100 of 13200 cycles at 64 states).  The FP32 iteration makes the same
+// rotations, so it leaves the eigenvector in the same column with the same sign; three
+// steps of v += sum_i v_i (v_i . A v + lambda v_i . (v0 - v)) / (lambda - lambda_i) (the
+// column form of Ogita and Aishima's refinement, Japan J. Indust. Appl. Math. 35, 2018)
+// square its error each: 1e-4 -> 1e-8 -> 1e-16.  Where FP32 could choose differently (a
+// rotation near 45 degrees that involves a large eigenvalue) or the top eigenvalue is not
+// well separated, the FP64 iteration runs instead.
+__device__ void top3(const double G[3][3], double out[3]) {
+  const double scale = fmax(G[0][0], fmax(G[1][1], G[2][2]));
+  bool ok = scale > 0.0 && scale < 1e300;
+  const double inv = ok ? 1.0 / scale : 0.0;
+  double A[3][3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) A[i][j] = G[i][j] * inv;
+  float S[3][3], d[3], V[3][3] = {{1.f, 0.f, 0.f}, {0.f, 1.f, 0.f}, {0.f, 0.f, 1.f}};
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    d[i] = (float)A[i][i];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) S[i][j] = (float)A[i][j];
+  }
+  for (int pass = 0; pass < 8 && ok; ++pass) {
+    const float off = S[0][1] * S[0][1] + S[0][2] * S[0][2] + S[1][2] * S[1][2];
+    if (!(off > 1e-16f)) break;
+    const float thresh = sqrtf(off) * (1.f / 12.f);
+#pragma unroll
+    for (int p = 0; p < 3; p++)
+#pragma unroll
+      for (int q = p + 1; q < 3; q++) {
+        if (fabsf(S[p][q]) < thresh) continue;
+        const float h = d[q] - d[p], big = fmaxf(fabsf(d[p]), fabsf(d[q]));
+        if (fabsf(h) < 1e-3f * big && big > 0.05f) ok = false;
+        const float e2 = 2.f * fabsf(S[p][q]), dd = fabsf(h) + sqrtf(h * h + e2 * e2);
+        const float sg = (h != 0.f && (h < 0.f) != (S[p][q] < 0.f)) ? -1.f : 1.f;
+        const float rn = rsqrtf(dd * dd + e2 * e2);
+        const float t = sg * __fdividef(e2, dd), c = dd * rn, s = sg * (e2 * rn), tau = __fdividef(s, 1.f + c);
+        d[p] -= t * S[p][q];
+        d[q] += t * S[p][q];
+        S[p][q] = 0.f;
+#define INQB_FROT(x, y)                  \
+  {                                      \
+    const float g_ = (x), h_ = (y);      \
+    (x) = g_ - s * (h_ + g_ * tau);      \
+    (y) = h_ + s * (g_ - h_ * tau);      \
+  }
+#pragma unroll
+        for (int j = 0; j < p; j++) INQB_FROT(S[j][p], S[j][q])
+#pragma unroll
+        for (int j = p + 1; j < q; j++) INQB_FROT(S[p][j], S[j][q])
+#pragma unroll
+        for (int j = q + 1; j < 3; j++) INQB_FROT(S[p][j], S[q][j])
+#pragma unroll
+        for (int j = 0; j < 3; j++) INQB_FROT(V[j][p], V[j][q])
+#undef INQB_FROT
+      }
+  }
+  // the top column v and the other two, v1 and v2
+  const int m = (d[1] > d[0]) ? (d[2] > d[1] ? 2 : 1) : (d[2] > d[0] ? 2 : 0);
+  const float dm = m == 0 ? d[0] : m == 1 ? d[1] : d[2];
+  const float g1 = dm - (m == 0 ? d[1] : d[0]), g2 = dm - (m == 2 ? d[1] : d[2]);
+  if (!(ok && g1 > 0.02f * dm && g2 > 0.02f * dm)) {
+    double B[3][3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) B[i][j] = G[i][j];
+    jacobi3_top(B, out);
+    return;
+  }
+  const double i1 = (double)(1.f / g1), i2 = (double)(1.f / g2);
+  double v[3], v1[3], v2[3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    v[j] = m == 0 ? V[j][0] : m == 1 ? V[j][1] : V[j][2];
+    v1[j] = m == 0 ? V[j][1] : V[j][0];
+    v2[j] = m == 2 ? V[j][1] : V[j][2];
+  }
+#pragma unroll
+  for (int it = 0; it < 3; ++it) {
+    double w[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) w[j] = fma(A[j][0], v[0], fma(A[j][1], v[1], A[j][2] * v[2]));
+    const double vv = fma(v[0], v[0], fma(v[1], v[1], v[2] * v[2]));
+    const double lam = fma(v[0], w[0], fma(v[1], w[1], v[2] * w[2])) * (2.0 - vv);  // Rayleigh, |v| near 1
+    double e1 = 0.0, e2 = 0.0;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const double res = fma(-lam, v[j], w[j]);
+      e1 = fma(v1[j], res, e1);
+      e2 = fma(v2[j], res, e2);
+    }
+    e1 *= i1;
+    e2 *= i2;
+    const double em = 0.5 * (1.0 - vv);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) v[j] += fma(em, v[j], fma(e1, v1[j], e2 * v2[j]));
+  }
+#pragma unroll
+  for (int j = 0; j < 3; ++j) out[j] = v[j];
+}
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// All sweeps in one launch of one thread-block cluster whose shared memory holds the six
+// matrices and u.  A rotation step is bound by latency, not by bytes: as a launch of its
+// own it gathered rows from L2 and paid a launch around the serial eigenproblem.  Here the
+// rows sit where they are rotated: slot j of the tournament holds the rows (top[j], bot[j])
+// of the seven matrices, CTA r the slots r SP .. r SP + SP - 1, and a rotated row is stored
+// straight into the slot that has it in the next step (remote stores, no remote load: with
+// rows at home and read over distributed shared memory a step took 13200 cycles, 4800 of
+// them the reads).  Two cluster barriers a step: all rows are read before any is
+// overwritten (arrived at after the reads, waited for after the eigenproblem), and all are
+// written before the next step reads.  Seven warps a slot: warp k sums and rotates matrix
+// k (warp 6: u); E elements of a row per lane (M <= 32 E); GMAX slots per CTA at most.
+constexpr int kJG = 7 * 32;
 
 struct JadeShared {
-  double red[6][6];  // warp k: Re, Im of the pair elements (pq, pp, qq) of matrix k
+  double red[6][6];   // warp k: Re, Im of the pair elements (pq, pp, qq) of matrix k
   double diag[6][2];  // warp k: change of the two diagonal elements
-  double rot[3];     // c, Re s, Im s
+  double rot[3];      // c, Re s, Im s
+  int id[2];          // the rows of the slot (M and above: none)
 };
 
 template <int E, int GMAX>
@@ -464,122 +578,163 @@ __global__ void __launch_bounds__(GMAX * kJG)
                    int steps, int maxsweep, double tol, double* delta, double* __restrict__ out) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
-  const int CL = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
-  extern __shared__ __align__(16) double2 rows[];  // [rows of this CTA][7][M]
+  extern __shared__ __align__(16) double2 rows[];  // [slot of this CTA][top, bot][7][M]
   __shared__ JadeShared sh[GMAX];
   __shared__ double part[GMAX * kJG];
   const size_t MM = (size_t)M * M;
-  const int mine = (M - rank + CL - 1) / CL;  // rows r = rank, rank + CL, ...
-  for (int e = threadIdx.x; e < mine * 7 * M; e += blockDim.x) {
-    const int i = e % M, k = (e / M) % 7, r = rank + CL * (e / (7 * M));
-    rows[e] = k < 6 ? a[k * MM + (size_t)r * M + i] : make_double2(r == i ? 1.0 : 0.0, 0.0);
-  }
   const int g = threadIdx.x / kJG, k = (threadIdx.x % kJG) / 32, lane = threadIdx.x & 31;
-  const int PG = blockDim.x / kJG;
+  const int SP = blockDim.x / kJG, slot = (int)cluster.block_rank() * SP + g;
+  const bool on = slot < np, lead = threadIdx.x % kJG == 0;
   JadeShared& q = sh[g];
+  double2* rp = rows + ((size_t)(2 * g) * 7 + k) * M;
+  double2* rq = rp + (size_t)7 * M;
+  // the two rows of the first step; dummy rows (odd M) are zero
+  const int2 first = on ? pairs[slot] : make_int2(M, M);
+  if (lead) {
+    q.id[0] = first.x;
+    q.id[1] = first.y;
+  }
+  if (on)
+    for (int i = lane; i < M; i += 32) {
+      const double2* src = a + (size_t)min(k, 5) * MM;
+      rp[i] = first.x >= M ? make_double2(0, 0)
+              : k < 6      ? src[(size_t)first.x * M + i]
+                           : make_double2(first.x == i ? 1.0 : 0.0, 0.0);
+      rq[i] = first.y >= M ? make_double2(0, 0)
+              : k < 6      ? src[(size_t)first.y * M + i]
+                           : make_double2(first.y == i ? 1.0 : 0.0, 0.0);
+    }
+  // where the slot's rows go after a step: top 0 stays, the other tops move up one slot and
+  // the last one turns to the bottom row; the bottoms move down and the first turns up
+  const int ts = (slot == 0 || slot == np - 1) ? slot : slot + 1, tw = (slot > 0 && slot == np - 1) ? 1 : 0;
+  const int bs = np == 1 ? slot : slot == 0 ? 1 : slot - 1, bw = (np > 1 && slot == 0) ? 0 : 1;
+  double2* tdst = nullptr;
+  double2* bdst = nullptr;
+  int *tid_dst = nullptr, *bid_dst = nullptr;
+  if (on) {
+    tdst = cluster.map_shared_rank(rows, ts / SP) + ((size_t)(2 * (ts % SP) + tw) * 7 + k) * M;
+    bdst = cluster.map_shared_rank(rows, bs / SP) + ((size_t)(2 * (bs % SP) + bw) * 7 + k) * M;
+    tid_dst = cluster.map_shared_rank(&sh[0].id[0], ts / SP) + (sizeof(JadeShared) / sizeof(int)) * (ts % SP) + tw;
+    bid_dst = cluster.map_shared_rank(&sh[0].id[0], bs / SP) + (sizeof(JadeShared) / sizeof(int)) * (bs % SP) + bw;
+  }
+  cluster_arrive();
   int nsweep = 0;
   double change = 0.0;
   for (;;) {
     ++nsweep;
     for (int st = 0; st < steps; ++st) {
-      cluster.sync();  // the rows of the step before are in place
-      for (int pi = rank + CL * g; pi < np; pi += CL * PG) {
-        const int2 pq = pairs[(size_t)st * np + pi];
-        if (pq.x >= M || pq.y >= M) {
-          if (threadIdx.x % kJG == 0) delta[(size_t)st * np + pi] = 0.0;
-          continue;
+      cluster_wait();  // the rows of this step are in place
+      // the step before's change of the diagonal, complete since that barrier
+      if (on && lead && st > 0) {
+        double d = 0.0;
+        for (int kk = 0; kk < 6; ++kk) d += q.diag[kk][0] + q.diag[kk][1];
+        delta[(size_t)(st - 1) * np + slot] = d;
+      }
+      const int p0 = q.id[0], q0 = q.id[1];
+      const bool live = on && p0 < M && q0 < M;
+      double2 xp[E], xq[E];
+#pragma unroll
+      for (int t = 0; t < E; ++t) {
+        const int i = lane + 32 * t;
+        xp[t] = xq[t] = make_double2(0.0, 0.0);
+        if (on && i < M) {
+          xp[t] = rp[i];
+          xq[t] = rq[i];
         }
-        double2* rp = cluster.map_shared_rank(rows, pq.x % CL) + (size_t)(pq.x / CL) * 7 * M;
-        double2* rq = cluster.map_shared_rank(rows, pq.y % CL) + (size_t)(pq.y / CL) * 7 * M;
-        double2 xp[E], xq[E];
+      }
+      if (live && k < 6) {
+        // sums of conj(a_p) u_q, conj(a_p) u_p, conj(a_q) u_q
+        double s[6] = {0, 0, 0, 0, 0, 0};
+        const double2 *up = rows + ((size_t)(2 * g) * 7 + 6) * M, *uq = up + (size_t)7 * M;
 #pragma unroll
         for (int t = 0; t < E; ++t) {
           const int i = lane + 32 * t;
-          xp[t] = xq[t] = make_double2(0.0, 0.0);
           if (i < M) {
-            xp[t] = rp[k * M + i];
-            xq[t] = rq[k * M + i];
+            const double2 y = up[i], z = uq[i];
+            const double2 x0 = cmul(cconj(xp[t]), z), x1 = cmul(cconj(xp[t]), y), x2 = cmul(cconj(xq[t]), z);
+            s[0] += x0.x;
+            s[1] += x0.y;
+            s[2] += x1.x;
+            s[3] += x1.y;
+            s[4] += x2.x;
+            s[5] += x2.y;
           }
         }
-        if (k < 6) {
-          // sums of conj(a_p) u_q, conj(a_p) u_p, conj(a_q) u_q
-          double s[6] = {0, 0, 0, 0, 0, 0};
 #pragma unroll
-          for (int t = 0; t < E; ++t) {
-            const int i = lane + 32 * t;
-            if (i < M) {
-              const double2 up = rp[6 * M + i], uq = rq[6 * M + i];
-              const double2 x0 = cmul(cconj(xp[t]), uq), x1 = cmul(cconj(xp[t]), up), x2 = cmul(cconj(xq[t]), uq);
-              s[0] += x0.x;
-              s[1] += x0.y;
-              s[2] += x1.x;
-              s[3] += x1.y;
-              s[4] += x2.x;
-              s[5] += x2.y;
-            }
-          }
+        for (int v = 0; v < 6; ++v) s[v] = warp_sum(s[v]);
+        if (lane == 0) {
 #pragma unroll
-          for (int v = 0; v < 6; ++v) s[v] = warp_sum(s[v]);
-          if (lane == 0) {
-#pragma unroll
-            for (int v = 0; v < 6; ++v) q.red[k][v] = s[v];
-          }
+          for (int v = 0; v < 6; ++v) q.red[k][v] = s[v];
         }
-        asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(kJG) : "memory");
-        if (k == 0) {
-          double G[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+      }
+      __syncwarp();
+      cluster_arrive();  // this warp has read its rows
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(kJG) : "memory");
+      if (live && k == 0) {
+        double G[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
 #pragma unroll
-          for (int kk = 0; kk < 6; ++kk) {
-            const double* e = q.red[kk];
-            // h = (aii - ajj, aij + conj(aij), i (aij - conj(aij))), as in k_jade_step
-            const double h0 = e[2] - e[4], h0i = e[3] - e[5], h1 = 2.0 * e[0], h2 = -2.0 * e[1];
-            G[0][0] += h0 * h0 + h0i * h0i;
-            G[0][1] += h0 * h1;
-            G[0][2] += h0 * h2;
-            G[1][1] += h1 * h1;
-            G[1][2] += h1 * h2;
-            G[2][2] += h2 * h2;
-          }
-          G[1][0] = G[0][1];
-          G[2][0] = G[0][2];
-          G[2][1] = G[1][2];
-          double v[3];
-          jacobi3_top(G, v);
-          const double x = fabs(v[0]), y = v[0] < 0.0 ? -v[1] : v[1];
-          const double r = sqrt((x + 1.0) / 2.0);
-          if (lane == 0) {
-            q.rot[0] = r;
-            q.rot[1] = y / (2.0 * r);
-            q.rot[2] = -v[2] / (2.0 * r);
-          }
+        for (int kk = 0; kk < 6; ++kk) {
+          const double* e = q.red[kk];
+          // h = (aii - ajj, aij + conj(aij), i (aij - conj(aij))), as in k_jade_step
+          const double h0 = e[2] - e[4], h0i = e[3] - e[5], h1 = 2.0 * e[0], h2 = -2.0 * e[1];
+          G[0][0] += h0 * h0 + h0i * h0i;
+          G[0][1] += h0 * h1;
+          G[0][2] += h0 * h2;
+          G[1][1] += h1 * h1;
+          G[1][2] += h1 * h2;
+          G[2][2] += h2 * h2;
         }
-        asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(kJG) : "memory");
-        const double c = q.rot[0];
-        const double2 sv = make_double2(q.rot[1], q.rot[2]), sc = cconj(sv);
+        G[1][0] = G[0][1];
+        G[2][0] = G[0][2];
+        G[2][1] = G[1][2];
+        double v[3];
+        top3(G, v);
+        const double x = fabs(v[0]), y = v[0] < 0.0 ? -v[1] : v[1];
+        const double r = sqrt((x + 1.0) / 2.0), ir = 0.5 / r;
+        if (lane == 0) {
+          q.rot[0] = r;
+          q.rot[1] = y * ir;
+          q.rot[2] = -v[2] * ir;
+        }
+      }
+      __syncwarp();
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(kJG) : "memory");
+      cluster_wait();  // every row is read
+      if (on) {
+        const double c = live ? q.rot[0] : 1.0;
+        const double2 sv = live ? make_double2(q.rot[1], q.rot[2]) : make_double2(0.0, 0.0), sc = cconj(sv);
+        if (k < 6 && lane < 2 && !live) q.diag[k][lane] = 0.0;
 #pragma unroll
         for (int t = 0; t < E; ++t) {
           const int i = lane + 32 * t;
           if (i >= M) continue;
           const double2 t1 = cmul(sc, xq[t]), t2 = cmul(sv, xp[t]);
-          const double2 np_ = make_double2(c * xp[t].x + t1.x, c * xp[t].y + t1.y);
-          const double2 nq = make_double2(c * xq[t].x - t2.x, c * xq[t].y - t2.y);
-          rp[k * M + i] = np_;
-          rq[k * M + i] = nq;
-          if (k < 6 && i == pq.x) q.diag[k][0] = np_.x - xp[t].x;
-          if (k < 6 && i == pq.y) q.diag[k][1] = nq.x - xq[t].x;
+          const double2 yp = make_double2(c * xp[t].x + t1.x, c * xp[t].y + t1.y);
+          const double2 yq = make_double2(c * xq[t].x - t2.x, c * xq[t].y - t2.y);
+          tdst[i] = yp;
+          bdst[i] = yq;
+          if (live && k < 6 && i == p0) q.diag[k][0] = yp.x - xp[t].x;
+          if (live && k < 6 && i == q0) q.diag[k][1] = yq.x - xq[t].x;
         }
-        asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(kJG) : "memory");
-        if (threadIdx.x % kJG == 0) {
-          double d = 0.0;
-          for (int kk = 0; kk < 6; ++kk) d += q.diag[kk][0] + q.diag[kk][1];
-          delta[(size_t)st * np + pi] = d;
+        if (lead) {
+          *tid_dst = p0;
+          *bid_dst = q0;
         }
       }
+      __syncwarp();
+      cluster_arrive();
+    }
+    cluster_wait();
+    if (on && lead) {
+      double d = 0.0;
+      for (int kk = 0; kk < 6; ++kk) d += q.diag[kk][0] + q.diag[kk][1];
+      delta[(size_t)(steps - 1) * np + slot] = d;
     }
     // sum over the steps of 2 |sum over the pairs of the trace change|, in the same order
     // by every CTA, so all take the same decision
     __threadfence();
-    cluster.sync();
+    cluster_arrive();
+    cluster_wait();
     double acc = 0.0;
     for (int st = threadIdx.x; st < steps; st += blockDim.x) {
       double t = 0.0;
@@ -590,19 +745,21 @@ __global__ void __launch_bounds__(GMAX * kJG)
     __syncthreads();
     change = 0.0;
     for (int i = 0; i < min((int)blockDim.x, steps); ++i) change += part[i];
-    __syncthreads();
+    cluster_arrive();  // every CTA has read the deltas
     if (!isfinite(change) || fabs(change) < tol || nsweep >= maxsweep) break;
   }
-  for (int e = threadIdx.x; e < mine * 7 * M; e += blockDim.x) {
-    const int i = e % M, kk = (e / M) % 7, r = rank + CL * (e / (7 * M));
-    double2* dst = kk < 6 ? a + kk * MM : u;
-    dst[(size_t)r * M + i] = rows[e];
+  cluster_wait();
+  // a sweep's moves bring every row back to its first slot
+  for (int w = 0; w < 2 && on; ++w) {
+    const int r = q.id[w];
+    if (r >= M) continue;
+    double2* dst = (k < 6 ? a + (size_t)k * MM : u) + (size_t)r * M;
+    for (int i = lane; i < M; i += 32) dst[i] = (w ? rq : rp)[i];
   }
-  if (rank == 0 && threadIdx.x == 0) {
+  if (cluster.block_rank() == 0 && threadIdx.x == 0) {
     out[0] = change;
     out[1] = (double)nsweep;
   }
-  cluster.sync();  // no CTA leaves while another may still read its rows
 }
 
 __global__ void k_identity(double2* __restrict__ u, int M) {
@@ -812,14 +969,14 @@ int launch_jade_step(double2* a, double2* u, int M, const int2* pairs, int np, d
 template <int E, int GMAX>
 static int jade_cluster_launch(double2* a, double2* u, int M, const int2* pairs, int np, int steps, int maxsweep,
                                double tol, double* delta, double* out, bool* done, cudaStream_t st) {
-  // sixteen CTAs (fewer pairs each) where the GPU places such a cluster, else eight
+  // sixteen CTAs (fewer slots each) where the GPU places such a cluster, else eight
   for (const int cl : {16, 8}) {
-    const size_t smem = (size_t)((M + cl - 1) / cl) * 7 * M * sizeof(double2);
-    if (smem > 200 * 1024) continue;
-    const int groups = std::min(GMAX, (np + cl - 1) / cl);
+    const int slots = (np + cl - 1) / cl;
+    const size_t smem = (size_t)slots * 2 * 7 * M * sizeof(double2);
+    if (slots > GMAX || smem > 200 * 1024) continue;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cl);
-    cfg.blockDim = dim3(groups * kJG);
+    cfg.blockDim = dim3(slots * kJG);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
@@ -828,7 +985,8 @@ static int jade_cluster_launch(double2* a, double2* u, int M, const int2* pairs,
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    INQB_CUDA_TRY(cudaFuncSetAttribute(k_jade_cluster<E, GMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    INQB_CUDA_TRY(cudaFuncSetAttribute(k_jade_cluster<E, GMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       200 * 1024));
     if (cl > 8)
       INQB_CUDA_TRY(cudaFuncSetAttribute(k_jade_cluster<E, GMAX>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     int fit = 0;
@@ -836,7 +994,8 @@ static int jade_cluster_launch(double2* a, double2* u, int M, const int2* pairs,
       cudaGetLastError();
       continue;
     }
-    INQB_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_jade_cluster<E, GMAX>, a, u, M, pairs, np, steps, maxsweep, tol, delta, out));
+    INQB_CUDA_TRY(
+        cudaLaunchKernelEx(&cfg, k_jade_cluster<E, GMAX>, a, u, M, pairs, np, steps, maxsweep, tol, delta, out));
     *done = true;
     return INQB_OK;
   }
@@ -849,9 +1008,9 @@ int launch_jade_cluster(double2* a, double2* u, int M, const int2* pairs, int np
                         double* delta, double* out, bool* done, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   *done = false;
+  // a slot's seven warps must all be resident, so at most four slots per CTA: 128 states
   if (M <= 64) return jade_cluster_launch<2, 2>(a, u, M, pairs, np, steps, maxsweep, tol, delta, out, done, st);
   if (M <= 128) return jade_cluster_launch<4, 4>(a, u, M, pairs, np, steps, maxsweep, tol, delta, out, done, st);
-  if (M <= 192) return jade_cluster_launch<6, 4>(a, u, M, pairs, np, steps, maxsweep, tol, delta, out, done, st);
   return INQB_OK;
 }
 
