@@ -26,6 +26,7 @@ int split_of(int n, int* n1, int* n2);
 int build_proj_tables(const inqb_ctx& ctx, int nproj, int L, int smax, const int* counts, const int* coords,
                       const float* relpos, const double* beta, const double* coeff, ProjTables& t);
 int upload_proj_tables(const inqb_ctx& ctx, ProjTables& t);
+int build_proj_chunks(const inqb_ctx& ctx, ProjTables& t);
 int sphere_points(const CellGeom& cell, const int nr[3], const double center[3], double radius, int npts, int* coords,
                   float* dist, float* relpos, int* count_out);
 int gaussian_kb_beta(const CellGeom& cell, int npts, const float* dist, const float* relpos, double sigma,
@@ -106,13 +107,18 @@ int reserve(inqb_ctx* ctx, int M) {
   return INQB_OK;
 }
 
+// the projection kernels' coefficients at the current k + A (read in that form only)
+int update_project_table(inqb_ctx* ctx, void* stream) {
+  return launch_project_table(ctx->precision, ctx->proj.pc_chunks, ctx->proj.d_pc_relpos.as<float>(),
+                              ctx->proj.d_pc_beta.as<double>(), ctx->kA_cov, ctx->proj.d_pc_table.ptr, stream);
+}
+
 int update_phases(inqb_ctx* ctx, void* stream) {
   if (ctx->proj.nproj == 0 || ctx->proj.nent == 0) return INQB_OK;
   INQB_TRY(launch_phases(ctx->precision, ctx->proj.nent, ctx->proj.d_ent_relpos.as<float>(), ctx->kA_cov,
                          ctx->proj.d_ent_rec.ptr, ctx->proj.d_ent_rec_rk.ptr, ctx->proj.d_rk_pos.as<int>(),
                          ctx->proj.d_adj_rec.ptr, ctx->proj.d_atom_pos.as<int>(), stream));
-  return launch_project_table(ctx->precision, ctx->proj.pc_chunks, ctx->proj.d_pc_relpos.as<float>(),
-                              ctx->proj.d_pc_beta.as<double>(), ctx->kA_cov, ctx->proj.d_pc_table.ptr, stream);
+  return ctx->proj_mode == INQB_PROJECTION_KERNEL ? update_project_table(ctx, stream) : INQB_OK;
 }
 
 int set_kA(inqb_ctx* ctx, const double kA[3], void* stream) {
@@ -787,6 +793,12 @@ int inqb_set_projection_mode(inqb_ctx* ctx, int mode) {
   INQB_CHECK_CTX(ctx);
   if (mode != INQB_PROJECTION_FUSED && mode != INQB_PROJECTION_KERNEL)
     return fail(INQB_ERR_INVALID, "unknown projection mode");
+  INQB_GUARD(ctx);
+  if (mode == INQB_PROJECTION_KERNEL && ctx->proj_mode != mode && ctx->proj.nproj > 0) {
+    INQB_TRY(build_proj_chunks(*ctx, ctx->proj));
+    INQB_TRY(update_project_table(ctx, nullptr));
+    INQB_CUDA_TRY(cudaStreamSynchronize(nullptr));
+  }
   ctx->proj_mode = mode;
   return INQB_OK;
 }
@@ -942,6 +954,7 @@ int inqb_set_projectors(inqb_ctx* ctx, int nproj, int L, int smax, const int* co
     for (double b : fresh.ent_beta)
       if (!std::isfinite(b)) return fail(INQB_ERR_NONFINITE, "projector table has a non-finite value");
     INQB_TRY(upload_proj_tables(*ctx, fresh));
+    if (ctx->proj_mode == INQB_PROJECTION_KERNEL) INQB_TRY(build_proj_chunks(*ctx, fresh));
   }
   INQB_CUDA_TRY(cudaDeviceSynchronize());
   ctx->proj = std::move(fresh);
