@@ -440,10 +440,11 @@ int inqb_mlwf_centres(inqb_ctx* ctx, int M, const double* adiag, double* centres
  * (no counterpart in the reference; its kernels have fixed launch shapes).  A
  * schedule is {ysplit, threads of pass 1, of pass 2, of pass 3}: ysplit CTAs share
  * one x-plane in the first pass (a divisor of the tiles per plane), and each pass
- * runs 64..256 threads per CTA (multiples of 32).  Schedules are kept per orbital
+ * runs 64..256 threads per CTA (multiples of 32; the compiled default, 512 in the first
+ * and third pass of the longest axes, may be named too).  Schedules are kept per orbital
  * count M; counts without one use the compiled default. */
-/* Time the candidates (every ysplit with 128 and 256 threads for the first pass,
- * 128 and 256 threads for the others) on zeroed M-orbital blocks with CUDA events
+/* Time the candidates (every ysplit with 128, 256 and the compiled default's threads for
+ * the first pass, the same threads for the others) on zeroed M-orbital blocks with CUDA events
  * and keep the fastest for M; schedule (may be NULL) receives it.  Allocates two
  * scratch blocks for the duration of the call; synchronous. */
 int inqb_autotune(inqb_ctx* ctx, int M, void* stream, int schedule[4]);

@@ -2001,9 +2001,11 @@ int inqb_set_schedule(inqb_ctx* ctx, int M, const int schedule[4]) {
   }
   if (schedule[0] < 1 || ctx->plan->y1 % schedule[0] != 0)
     return fail(INQB_ERR_INVALID, "schedule: ysplit must divide " + std::to_string(ctx->plan->y1));
-  for (int k = 1; k < 4; k++)
-    if (schedule[k] < 64 || schedule[k] > 256 || schedule[k] % 32 != 0)
+  for (int k = 1; k < 4; k++) {
+    const bool compiled = schedule[k] == ctx->plan->threads[k - 1];  // may be 512
+    if (!compiled && (schedule[k] < 64 || schedule[k] > 256 || schedule[k] % 32 != 0))
       return fail(INQB_ERR_INVALID, "schedule: threads per CTA must be a multiple of 32 in [64, 256]");
+  }
   ctx->schedules[M] = {schedule[0], schedule[1], schedule[2], schedule[3]};
   return INQB_OK;
 }
@@ -2025,7 +2027,8 @@ int inqb_autotune(inqb_ctx* ctx, int M, void* stream, int schedule[4]) {
   const double one[2] = {1.0, 0.0}, zero[2] = {0.0, 0.0};
   const bool saved_timing = ctx->timing_on;
   ctx->timing_on = false;
-  std::array<int, 4> best = {ctx->plan->ysplit, 256, 256, 256};
+  const Plan& plan = *ctx->plan;
+  std::array<int, 4> best = {plan.ysplit, plan.threads[0], plan.threads[1], plan.threads[2]};
   // pass times (ms) of one schedule: the best of three applications after a warm-up
   auto pass_ms = [&](const std::array<int, 4>& s, float out_ms[3]) -> int {
     ctx->schedules[M] = s;
@@ -2048,7 +2051,7 @@ int inqb_autotune(inqb_ctx* ctx, int M, void* stream, int schedule[4]) {
   // pass A: every divisor of Y1 times every thread count; passes B and C: thread counts
   for (int ys = 1; ys <= ctx->plan->y1 && status == INQB_OK; ys++) {
     if (ctx->plan->y1 % ys != 0) continue;
-    for (int thr : kScheduleThreads) {
+    for (int thr : {plan.threads[0], kScheduleThreads[0], kScheduleThreads[1]}) {
       std::array<int, 4> s = best;
       s[0] = ys;
       s[1] = thr;
@@ -2061,7 +2064,7 @@ int inqb_autotune(inqb_ctx* ctx, int M, void* stream, int schedule[4]) {
     }
   }
   for (int k = 1; k < 3 && status == INQB_OK; k++)
-    for (int thr : kScheduleThreads) {
+    for (int thr : {plan.threads[k], kScheduleThreads[0], kScheduleThreads[1]}) {
       std::array<int, 4> s = best;
       s[1 + k] = thr;
       if ((status = pass_ms(s, t)) != INQB_OK) break;

@@ -49,9 +49,9 @@ __device__ __forceinline__ void fma_acc(cplx<T>& acc, cplx<T> a, cplx<T> b) {
 }
 
 // ---------------------------------------------------------------- lanes
-// The transforms work on 16-byte lanes: one complex128 value (cplx<double>), or the
-// complex64 values of two neighbouring orbitals as (re, re | im, im) in two packed FP32
-// pairs (cplx<F2>).  Every operation of the transforms is the same for both orbitals, so
+// The transforms work on lanes, usually of 16 bytes: one complex128 value (cplx<double>), or
+// the complex64 values of two neighbouring orbitals as (re, re | im, im) in two packed FP32
+// pairs (cplx<F2>); long FP32 axes use one complex64 (cplx<float>, TileGeom in tiles.cuh).  Every operation of the transforms is the same for both orbitals, so
 // a packed f32x2 instruction (sm_100: add, sub, mul, fma; each half rounded to nearest
 // like the scalar form) does the work of two, and shared memory, HBM and the index
 // arithmetic see one 16-byte access per lane in both precisions.
@@ -89,6 +89,7 @@ __device__ __forceinline__ F2 vfma(F2 a, F2 b, F2 c) {
   return r;
 }
 __device__ __forceinline__ double vfma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float vfma(float a, float b, float c) { return fmaf(a, b, c); }
 
 // the value c in every part of a lane component
 template <typename P>
@@ -97,12 +98,19 @@ template <>
 __device__ __forceinline__ double splat<double>(double c) { return c; }
 template <>
 __device__ __forceinline__ F2 splat<F2>(double c) { return f2((float)c, (float)c); }
-__device__ __forceinline__ F2 splat_of(float c) { return f2(c, c); }
-__device__ __forceinline__ double splat_of(double c) { return c; }
+template <>
+__device__ __forceinline__ float splat<float>(double c) { return (float)c; }
+// the same of a value in the tile precision
+template <typename P, typename T>
+__device__ __forceinline__ P splat_of(T c) { return c; }
+template <>
+__device__ __forceinline__ F2 splat_of<F2, float>(float c) { return f2(c, c); }
 template <typename P>
 __device__ __forceinline__ P vneg(P a) { return splat<P>(-1.0) * a; }
 template <>
 __device__ __forceinline__ double vneg<double>(double a) { return -a; }
+template <>
+__device__ __forceinline__ float vneg<float>(float a) { return -a; }
 
 template <typename T>
 struct LaneOf;
@@ -122,18 +130,21 @@ __device__ __forceinline__ cplx<F2> flip(cplx<F2> a) {
   return {f2(p.x, q.x), f2(p.y, q.y)};
 }
 __device__ __forceinline__ cplx<double> flip(cplx<double> a) { return a; }
+__device__ __forceinline__ cplx<float> flip(cplx<float> a) { return a; }
 // value of orbital k of a lane
 __device__ __forceinline__ cplx<float> lane_get(cplx<F2> a, int k) {
   const float2 p = f2_get(a.x), q = f2_get(a.y);
   return k ? mk<float>(p.y, q.y) : mk<float>(p.x, q.x);
 }
 __device__ __forceinline__ cplx<double> lane_get(cplx<double> a, int) { return a; }
-__device__ __forceinline__ cplx<F2> lane_splat(cplx<float> a) { return {f2(a.x, a.x), f2(a.y, a.y)}; }
-__device__ __forceinline__ cplx<double> lane_splat(cplx<double> a) { return a; }
+__device__ __forceinline__ cplx<float> lane_get(cplx<float> a, int) { return a; }
+template <typename P, typename T>
+__device__ __forceinline__ cplx<P> lane_splat(cplx<T> a) { return {splat_of<P>(a.x), splat_of<P>(a.y)}; }
 __device__ __forceinline__ cplx<F2> lane_shfl_xor(cplx<F2> a, int o) {
   return {F2{__shfl_xor_sync(0xffffffffu, a.x.v, o)}, F2{__shfl_xor_sync(0xffffffffu, a.y.v, o)}};
 }
-__device__ __forceinline__ cplx<double> lane_shfl_xor(cplx<double> a, int o) {
+template <typename P>
+__device__ __forceinline__ cplx<P> lane_shfl_xor(cplx<P> a, int o) {
   return {__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o)};
 }
 

@@ -157,7 +157,7 @@ int launch_h_impl(const LaunchArgs& a) {
   const cplx<T>* twx = tw;
   const cplx<T>* twy = tw + NX;
   const cplx<T>* twz = tw + NX + NY;
-  Lane<T>* tmp = reinterpret_cast<Lane<T>*>(a.tmp);
+  auto* tmp = reinterpret_cast<typename TG::V*>(a.tmp);
   cudaStream_t st = (cudaStream_t)a.stream;
   const size_t esz = sizeof(cplx<T>);
   const int tgroups = (a.M + GT - 1) / GT;
@@ -168,12 +168,12 @@ int launch_h_impl(const LaunchArgs& a) {
   const int vminus = a.minus && aligned16(a.minus, a.ld_minus, esz);
   int ysplit = a.ysplit > 0 ? a.ysplit : TG::YSPLIT;
   if (TG::Y1 % ysplit != 0) return fail(INQB_ERR_INVALID, "schedule: ysplit must divide the tiles per plane");
-  const int thr_default[3] = {TG::THREADS, TG::X_THREADS, TG::Z_THREADS};
+  const int thr_default[3] = {TG::ZT, TG::X_THREADS, TG::Z_THREADS};
   int thr[3];
   for (int k = 0; k < 3; k++) {
     thr[k] = a.threads[k] > 0 ? a.threads[k] : thr_default[k];
-    if (thr[k] % 32 != 0 || thr[k] < 64 || thr[k] > TG::THREADS)
-      return fail(INQB_ERR_INVALID, "schedule: threads per CTA must be a multiple of 32 in [64, 256]");
+    if (thr[k] % 32 != 0 || thr[k] < 64 || thr[k] > (k == 1 ? TG::THREADS : TG::ZT))
+      return fail(INQB_ERR_INVALID, "schedule: threads per CTA must be a multiple of 32 from 64 to the pass's most");
   }
   const dim3 gfwd(tgroups, NX * ysplit), gx(TG::Y2 * NZ, tgroups), ginv(tgroups, NX * TG::Y1);
 
@@ -240,7 +240,7 @@ int launch_h_impl(const LaunchArgs& a) {
       c.seg_cap = seg_cap;
       c.vin = vin;
       c.vio = vin && vout;
-      c.tmp = tmp;
+      c.tmp = reinterpret_cast<Lane<T>*>(a.tmp);
       c.tw = tw;
       c.pj = pj;
       c.kp = kp;
@@ -329,6 +329,9 @@ inline Plan make_plan() {
   p.y1 = TileGeom<T, NX, NY, NZ>::Y1;
   p.y2 = TileGeom<T, NX, NY, NZ>::Y2;
   p.ysplit = TileGeom<T, NX, NY, NZ>::YSPLIT;
+  using TG = TileGeom<T, NX, NY, NZ>;
+  const int def[3] = {TG::ZT, TG::X_THREADS, TG::Z_THREADS};
+  for (int k = 0; k < 3; k++) p.threads[k] = def[k];
   p.launch = &launch_h_impl<T, NX, NY, NZ>;
   return p;
 }

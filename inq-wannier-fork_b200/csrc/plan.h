@@ -40,7 +40,7 @@ struct LaunchArgs {
   void* batch_cell = nullptr;
 };
 
-// Candidate values the autotuner tries.
+// Candidate values the autotuner tries, beside the compiled default.
 constexpr int kScheduleThreads[2] = {128, 256};
 
 struct Plan {
@@ -49,6 +49,7 @@ struct Plan {
   int y1 = 1;      // tiles per x-plane (the divisors of y1 are the first pass's splits)
   int y2 = 1;      // rows per tile (the y split is NY = y2 * y1)
   int ysplit = 1;  // default split
+  int threads[3] = {256, 256, 256};  // compiled defaults of the three passes
   int (*launch)(const LaunchArgs&) = nullptr;
 };
 

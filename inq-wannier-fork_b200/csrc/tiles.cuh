@@ -54,6 +54,10 @@ __device__ __forceinline__ cplx<double> ld_l2(const cplx<double>* p) {
   const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
   return mk<double>(v.x, v.y);
 }
+__device__ __forceinline__ cplx<float> ld_l2(const cplx<float>* p) {
+  const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
+  return mk<float>(v.x, v.y);
+}
 __device__ __forceinline__ double2 ld_l2(const double2* p) { return __ldcg(p); }
 
 // ---------------------------------------------------------------- geometry
@@ -70,44 +74,54 @@ struct TileGeom {
   // per SM (measured: FP32 144^3 apply 75 -> 65 ms; FP64 is faster with 64 bytes)
   static constexpr int RUN = (sizeof(T) == 4 && Y2 * ZS * 64 > 80 * 1024) ? 32 : 64;
   static constexpr int G = RUN / (int)sizeof(cplx<T>);
-  static constexpr int PV = 16 / (int)sizeof(cplx<T>);  // orbitals per 16-byte lane
-  static constexpr int VP = G / PV;                      // lanes per point
-  // the sizes below count 16-byte lanes
+  // A lane holds 16 bytes, except in FP32 where a transform step is longer than 12 values:
+  // 16 lanes of two orbitals take 64 registers, which leaves two CTAs of 256 threads per SM;
+  // with one orbital per lane twice the threads fit (144^3 x 64 orbitals, two orbitals ->
+  // one: pass A 1964 -> 1777 us, B 1176 -> 1099 us, C 2487 -> 2273 us).
+  static constexpr int cmin(int a, int b) { return a < b ? a : b; }
+  static constexpr int cmax(int a, int b) { return a > b ? a : b; }
+  static constexpr int RZ = cmax(AZ::N1, AZ::N2), RX = cmax(AX::N1, AX::N2);
+  static constexpr bool NARROW = sizeof(T) == 4 && cmax(cmax(RZ, RX), cmax(Y1, Y2)) > 12;
+  using P = std::conditional_t<NARROW, T, LaneP<T>>;
+  using V = cplx<P>;
+  static constexpr int PV = (int)(sizeof(V) / sizeof(cplx<T>));  // orbitals per lane
+  static constexpr int VP = G / PV;                               // lanes per point
+  static constexpr int CH = RUN / 16, LC = 16 / (int)sizeof(V);   // 16-byte copies of a point, lanes of one
+  // the sizes below count lanes
   static constexpr int TILE = Y2 * ZS * VP;  // a tile in shared memory
   static constexpr int PTS = Y2 * NZ;        // grid points of a tile
   static constexpr int XS = (Y1 + 1) * VP;   // x-slot stride of the x-line block (one point of padding)
   static constexpr int XBLK = AX::SLOTS * XS;
   static constexpr int BLK = NX * Y1 * VP;   // one tmp block [ix][y1][G]
-  static constexpr int THREADS = 256;
   static constexpr size_t SMEM_MAX = 227 * 1024;  // dynamic shared memory a CTA may have
   static constexpr size_t smem_fwd(int acc_atoms, int rec_cap) {
-    return sizeof(Lane<T>) * ((size_t)TILE + NY + NZ) + sizeof(double2) * (size_t)acc_atoms * LMAX * G +
+    return sizeof(V) * ((size_t)TILE + NY + NZ) + sizeof(double2) * (size_t)acc_atoms * LMAX * G +
            sizeof(EntRec<T>) * (size_t)rec_cap;
   }
-  static constexpr size_t SMEM_X = sizeof(Lane<T>) * ((size_t)XBLK + NX) + sizeof(T) * 2 * Y1;
-  static constexpr size_t TILE_BYTES = sizeof(Lane<T>) * (size_t)TILE;
+  static constexpr size_t SMEM_X = sizeof(V) * ((size_t)XBLK + NX) + sizeof(T) * 2 * Y1;
+  static constexpr size_t TILE_BYTES = sizeof(V) * (size_t)TILE;
   // CTAs of 256 threads per SM that a pass asks the compiler for: four where the radices
   // fit 64 registers a thread (up to 8 lanes of a transform), three (80 registers) up to
   // 12, two (128) beyond, and no more than the tiles in shared memory allow
-  static constexpr int radix_ctas(int r) { return r <= 8 ? 4 : r <= 12 ? 3 : 2; }
-  static constexpr int cmin(int a, int b) { return a < b ? a : b; }
-  static constexpr int cmax(int a, int b) { return a > b ? a : b; }
+  static constexpr int radix_ctas(int r) { return r * (int)sizeof(V) <= 128 ? 4 : r * (int)sizeof(V) <= 192 ? 3 : 2; }
   static constexpr int fit(size_t bytes) { return (int)(SMEM_MAX / (bytes + 1024)); }
-  static constexpr int RZ = cmax(AZ::N1, AZ::N2), RX = cmax(AX::N1, AX::N2);
-  static constexpr int FWD_MIN_CTAS = cmax(1, cmin(cmin(3, radix_ctas(cmax(RZ, Y2))), fit(TILE_BYTES)));
+  // 512 threads in the z passes where the tile lets one CTA on an SM, or two of narrow lanes
+  // (144^3 x 16 orbitals FP64, 256 -> 512 threads: pass A 885 -> 537 us, C 2149 -> 924 us)
+  static constexpr int THREADS = 256, ZT = (NARROW || fit(TILE_BYTES) < 2) ? 512 : 256;
+  static constexpr int FWD_MIN_CTAS = NARROW ? 2 : cmax(1, cmin(cmin(3, radix_ctas(cmax(RZ, Y2))), fit(TILE_BYTES)));
   static constexpr int X_MIN_CTAS = cmax(1, cmin(radix_ctas(cmax(RX, Y1)), fit(SMEM_X)));
-  static constexpr int INV_MIN_CTAS = cmax(1, cmin(radix_ctas(cmax(RZ, Y2)), fit(TILE_BYTES)));
+  static constexpr int INV_MIN_CTAS = NARROW ? 2 : cmax(1, cmin(radix_ctas(cmax(RZ, Y2)), fit(TILE_BYTES)));
   // lanes per atom segment of pass C's staged projections [l][orbital]: 64 bytes of
   // padding, so that consecutive segments start in opposite halves of the
   // shared-memory banks
-  static constexpr int PT_STRIDE = LMAX * VP + 4;
+  static constexpr int PT_STRIDE = LMAX * VP + 64 / (int)sizeof(V);
   static constexpr size_t smem_inv(int seg_cap) {
-    return sizeof(Lane<T>) * ((size_t)TILE + NY + NZ + (size_t)seg_cap * PT_STRIDE);
+    return sizeof(V) * ((size_t)TILE + NY + NZ + (size_t)seg_cap * PT_STRIDE);
   }
   // Pass A default: the CTAs that share an x-plane.  Each walks its tiles one after the
   // other, so fewer tiles per CTA end the launch more evenly; more CTAs add partial sums of
   // the projection.  Measured (mixed; CTAs per plane: us of the pass): 144^3 1: 2487,
-  // 3: 2223, 9: 2104; 128^3 2: 735, 4: 608, 8: 626; 96^3 2: 315, 4: 275, 8: 280; 60^3 1: 118,
+  // 3: 2223, 9: 2104 (two-orbital lanes); 128^3 2: 735, 4: 608, 8: 626; 96^3 2: 315, 4: 275, 8: 280; 60^3 1: 118,
   // 5: 95; 40^3 1: 25.8, 5: 18.7; 32^3 2: 14.1, 4: 10.7; 24^3 1: 18.7, 3: 12.3; but 64^3 2: 184,
   // 4: 193, 8: 187 and 72^3 2: 135, 8: 136.
   static constexpr int YSPLIT = (Y1 % 2 == 1 || Y1 <= 4) ? Y1 : Y1 == 6 ? 3 : (TILE_BYTES > 40 * 1024) ? 4 : 2;
@@ -122,7 +136,7 @@ struct TileGeom {
   }
   static constexpr int X_THREADS =
       round_threads(NX * VP, sizeof(T) == 8 ? 192 : (cmax(RX, Y1) > 8 || NX * VP > 256) ? 192 : 256);
-  static constexpr int Z_THREADS = (NZ * VP > 128 && NZ * VP <= 192) ? round_threads(NZ * VP, 192) : THREADS;
+  static constexpr int Z_THREADS = (NZ * VP > 128 && NZ * VP <= 192) ? round_threads(NZ * VP, 192) : ZT;
 };
 
 // Entry records staged in shared memory per tile; a tile with more entries
@@ -160,13 +174,13 @@ constexpr int kSegMax = 320;
 // blockIdx.y), the persistent batch kernel at the coordinates of a work item.
 template <typename T, int NX, int NY, int NZ>
 __device__ __forceinline__ void tile_fwd_body(int bx, int by, const cplx<T>* __restrict__ in, long ld, int M,
-                                              Lane<T>* __restrict__ tmp, const cplx<T>* __restrict__ tw_y,
+                                              typename TileGeom<T, NX, NY, NZ>::V* __restrict__ tmp, const cplx<T>* __restrict__ tw_y,
                                               const cplx<T>* __restrict__ tw_z, ProjView<T> pj, int acc_cap,
                                               int rec_cap, int ysplit, int vec) {
   using TG = TileGeom<T, NX, NY, NZ>;
   using AZ = typename TG::AZ;
-  using V = Lane<T>;
-  using P = LaneP<T>;
+  using V = typename TG::V;
+  using P = typename TG::P;
   constexpr int G = TG::G, PV = TG::PV, VP = TG::VP, Y1 = TG::Y1, Y2 = TG::Y2, ZS = TG::ZS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V* S = reinterpret_cast<V*>(smem_raw);
@@ -183,8 +197,8 @@ __device__ __forceinline__ void tile_fwd_body(int bx, int by, const cplx<T>* __r
   const bool v16 = vec && gcount == G;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const bool proj_on = pj.nproj > 0;
-  for (int i = threadIdx.x; i < NY; i += blockDim.x) twy[i] = lane_splat(tw_y[i]);
-  for (int i = threadIdx.x; i < NZ; i += blockDim.x) twz[i] = lane_splat(tw_z[i]);
+  for (int i = threadIdx.x; i < NY; i += blockDim.x) twy[i] = lane_splat<P>(tw_y[i]);
+  for (int i = threadIdx.x; i < NZ; i += blockDim.x) twz[i] = lane_splat<P>(tw_z[i]);
   if (proj_on)
     for (int i = threadIdx.x; i < acc_cap * LMAX * G; i += blockDim.x) acc[i] = make_double2(0.0, 0.0);
   chain_wait();
@@ -204,11 +218,11 @@ __device__ __forceinline__ void tile_fwd_body(int bx, int by, const cplx<T>* __r
   auto load_tile = [&](int y1) {
     if (v16) {
 #pragma unroll 1
-      for (int q = threadIdx.x; q < TG::PTS * VP; q += blockDim.x) {
-        const int v = q % VP, pt = q / VP;
+      for (int q = threadIdx.x; q < TG::PTS * TG::CH; q += blockDim.x) {
+        const int c = q % TG::CH * TG::LC, pt = q / TG::CH;
         const int z = pt % NZ, r = pt / NZ;
         const long p = ((long)ix * NY + y1 + Y1 * r) * NZ + z;
-        cp_async16(S + (r * ZS + AZ::slot(z)) * VP + v, in + p * ld + m0 + v * PV);
+        cp_async16(S + (r * ZS + AZ::slot(z)) * VP + c, in + p * ld + m0 + c * PV);
       }
     } else {
       cplx<T>* Sj = reinterpret_cast<cplx<T>*>(S);
@@ -246,11 +260,11 @@ __device__ __forceinline__ void tile_fwd_body(int bx, int by, const cplx<T>* __r
         for (int l = 0; l < LMAX; ++l) a[l] = {splat<P>(0.0), splat<P>(0.0)};
         auto add = [&](const EntRec<T>& re) {
           const V u = flip(S[re.off * VP + v]);
-          const P pr = splat_of(re.ph[0]), pi = splat_of(re.ph[1]), npi = splat_of(-re.ph[1]);
+          const P pr = splat_of<P>(re.ph[0]), pi = splat_of<P>(re.ph[1]), npi = splat_of<P>(-re.ph[1]);
           const V x = {vfma(u.x, pr, u.y * npi), vfma(u.x, pi, u.y * pr)};
 #pragma unroll
           for (int l = 0; l < LMAX; ++l) {
-            const P b = splat_of(re.beta[l]);
+            const P b = splat_of<P>(re.beta[l]);
             a[l].x = vfma(b, x.x, a[l].x);
             a[l].y = vfma(b, x.y, a[l].y);
           }
@@ -371,8 +385,8 @@ __device__ __forceinline__ void tile_fwd_body(int bx, int by, const cplx<T>* __r
 }
 
 template <typename T, int NX, int NY, int NZ>
-__global__ void __launch_bounds__(256, TileGeom<T, NX, NY, NZ>::FWD_MIN_CTAS)
-    k_tile_fwd(const cplx<T>* __restrict__ in, long ld, int M, Lane<T>* __restrict__ tmp,
+__global__ void __launch_bounds__(TileGeom<T, NX, NY, NZ>::ZT, TileGeom<T, NX, NY, NZ>::FWD_MIN_CTAS)
+    k_tile_fwd(const cplx<T>* __restrict__ in, long ld, int M, typename TileGeom<T, NX, NY, NZ>::V* __restrict__ tmp,
                const cplx<T>* __restrict__ tw_y, const cplx<T>* __restrict__ tw_z, ProjView<T> pj, int acc_cap,
                int rec_cap, int ysplit, int vec) {
   tile_fwd_body<T, NX, NY, NZ>(blockIdx.x, blockIdx.y, in, ld, M, tmp, tw_y, tw_z, pj, acc_cap, rec_cap, ysplit,
@@ -433,13 +447,13 @@ __device__ __forceinline__ long finish_item(long t) { return t / 32 * (32 / kFin
 // thread t of CTA b handles item b * blockDim + t, so the few CTAs that carry the
 // finish run beside thousands that do not.
 template <typename T, int NX, int NY, int NZ>
-__device__ __forceinline__ void tile_x_body(int bx, int by, Lane<T>* __restrict__ tmp,
+__device__ __forceinline__ void tile_x_body(int bx, int by, typename TileGeom<T, NX, NY, NZ>::V* __restrict__ tmp,
                                             const cplx<T>* __restrict__ tw_x, KinParams<T> kp,
                                             cplx<T>* __restrict__ fout) {
   using TG = TileGeom<T, NX, NY, NZ>;
   using AX = typename TG::AX;
-  using V = Lane<T>;
-  using P = LaneP<T>;
+  using V = typename TG::V;
+  using P = typename TG::P;
   constexpr int VP = TG::VP, Y1 = TG::Y1, Y2 = TG::Y2, XS = TG::XS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V* X = reinterpret_cast<V*>(smem_raw);
@@ -449,7 +463,7 @@ __device__ __forceinline__ void tile_x_body(int bx, int by, Lane<T>* __restrict_
 
   const int kz = bx % NZ, ka = bx / NZ, grp = by;
   V* blk = tmp + ((long)(grp * Y2 + ka) * NZ + kz) * TG::BLK;
-  for (int i = threadIdx.x; i < NX; i += blockDim.x) twx[i] = lane_splat(tw_x[i]);
+  for (int i = threadIdx.x; i < NX; i += blockDim.x) twx[i] = lane_splat<P>(tw_x[i]);
   // Along an x line 1/2 |G + k + A|^2 / N = kA2 n0^2 + kinB n0 + kinC with
   // q = n1 b1 + n2 b2 + k + A:  kA2 = |b0|^2 / 2N, kinB = b0.q / N, kinC = |q|^2 / 2N
   if (threadIdx.x < Y1) {
@@ -510,7 +524,7 @@ __device__ __forceinline__ void tile_x_body(int bx, int by, Lane<T>* __restrict_
     T k = fma(fma(kinA, f0, kinB[kb]), f0, kinC[kb]);
     if (kp.mask) k = outside_sphere(kp.nr, n0, sym_freq(ka + Y2 * kb, NY), n2) ? (T)0 : k - kp.shift;
     if (kp.pois != (T)0) k = ((T)2 * k < (T)1e-6) ? (T)0 : kp.pois / k;
-    const P ks = splat_of(k);
+    const P ks = splat_of<P>(k);
     return {ks * v.x, ks * v.y};
   });
   __syncthreads();
@@ -532,7 +546,7 @@ __device__ __forceinline__ void tile_x_body(int bx, int by, Lane<T>* __restrict_
 
 template <typename T, int NX, int NY, int NZ>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? TileGeom<T, NX, NY, NZ>::X_MIN_CTAS : 1)
-    k_tile_x(Lane<T>* __restrict__ tmp, const cplx<T>* __restrict__ tw_x, KinParams<T> kp,
+    k_tile_x(typename TileGeom<T, NX, NY, NZ>::V* __restrict__ tmp, const cplx<T>* __restrict__ tw_x, KinParams<T> kp,
              cplx<T>* __restrict__ fout, ProjView<T> fin, int fin_M, int fin_ysplit) {
   if (fin.slots) {
     const long n = (long)fin.nproj * fin.L * fin_M;
@@ -554,12 +568,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? TileGeom<T, NX, NY, NZ>:
 //   and the 1/N (transform.hpp:250-332).
 template <typename T, int NX, int NY, int NZ, int DIR>
 __global__ void __launch_bounds__(256, TileGeom<T, NX, NY, NZ>::X_MIN_CTAS)
-    k_tile_x_fft(Lane<T>* __restrict__ tmp, const cplx<T>* __restrict__ in, cplx<T>* __restrict__ out, long ld,
+    k_tile_x_fft(typename TileGeom<T, NX, NY, NZ>::V* __restrict__ tmp, const cplx<T>* __restrict__ in, cplx<T>* __restrict__ out, long ld,
                  int M, const cplx<T>* __restrict__ tw_x, int vec) {
   using TG = TileGeom<T, NX, NY, NZ>;
   using AX = typename TG::AX;
-  using V = Lane<T>;
-  using P = LaneP<T>;
+  using V = typename TG::V;
+  using P = typename TG::P;
   constexpr int G = TG::G, PV = TG::PV, VP = TG::VP, Y1 = TG::Y1, Y2 = TG::Y2, XS = TG::XS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V* X = reinterpret_cast<V*>(smem_raw);
@@ -584,7 +598,7 @@ __global__ void __launch_bounds__(256, TileGeom<T, NX, NY, NZ>::X_MIN_CTAS)
     base = (rest / AX::N1) * VP + v;
     es = XS;
   };
-  for (int i = threadIdx.x; i < NX; i += blockDim.x) twx[i] = lane_splat(tw_x[i]);
+  for (int i = threadIdx.x; i < NX; i += blockDim.x) twx[i] = lane_splat<P>(tw_x[i]);
   chain_wait();
 
   if (DIR == 0) {
@@ -621,10 +635,10 @@ __global__ void __launch_bounds__(256, TileGeom<T, NX, NY, NZ>::X_MIN_CTAS)
   } else {
     // natural kx into slot(kx); the inverse from natural order leaves ix in slot_of_freq(ix)
     if (v16) {
-      for (int q = threadIdx.x; q < NX * Y1 * VP; q += blockDim.x) {
-        const int v = q % VP, r = q / VP;
+      for (int q = threadIdx.x; q < NX * Y1 * TG::CH; q += blockDim.x) {
+        const int c = q % TG::CH * TG::LC, r = q / TG::CH;
         const int kb = r % Y1, kx = r / Y1;
-        cp_async16(X + AX::slot(kx) * XS + kb * VP + v, in + point(kx, kb) * ld + m0 + v * PV);
+        cp_async16(X + AX::slot(kx) * XS + kb * VP + c, in + point(kx, kb) * ld + m0 + c * PV);
       }
       cp_async_commit();
       cp_async_wait<0>();
@@ -661,15 +675,15 @@ __global__ void __launch_bounds__(256, TileGeom<T, NX, NY, NZ>::X_MIN_CTAS)
 // MODE_H = 1: the H epilogue; 0: out = alpha * (inverse transform), the second
 // half of to_real (alpha = 1/N), reading neither orbitals, V nor projectors.
 template <typename T, int NX, int NY, int NZ, int MODE_H>
-__device__ __forceinline__ void tile_inv_body(int bx, int by, const Lane<T>* __restrict__ tmp,
+__device__ __forceinline__ void tile_inv_body(int bx, int by, const typename TileGeom<T, NX, NY, NZ>::V* __restrict__ tmp,
                                               const cplx<T>* __restrict__ in, long ld_in, cplx<T>* __restrict__ out,
                                               long ld_out, int M, const cplx<T>* __restrict__ tw_y,
                                               const cplx<T>* __restrict__ tw_z, const ProjView<T>& pj,
                                               const EpiParams<T>& ep, int seg_cap, int vec) {
   using TG = TileGeom<T, NX, NY, NZ>;
   using AZ = typename TG::AZ;
-  using V = Lane<T>;
-  using P = LaneP<T>;
+  using V = typename TG::V;
+  using P = typename TG::P;
   constexpr int G = TG::G, PV = TG::PV, VP = TG::VP, Y1 = TG::Y1, Y2 = TG::Y2, ZS = TG::ZS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V* S = reinterpret_cast<V*>(smem_raw);
@@ -684,8 +698,8 @@ __device__ __forceinline__ void tile_inv_body(int bx, int by, const Lane<T>* __r
   // and the subtracted block do
   const bool v16 = (vec & 1) && gcount == G, b16 = (vec & 2) && gcount == G, s16 = (vec & 4) && gcount == G;
 
-  for (int i = threadIdx.x; i < NY; i += blockDim.x) twy[i] = lane_splat(tw_y[i]);
-  for (int i = threadIdx.x; i < NZ; i += blockDim.x) twz[i] = lane_splat(tw_z[i]);
+  for (int i = threadIdx.x; i < NY; i += blockDim.x) twy[i] = lane_splat<P>(tw_y[i]);
+  for (int i = threadIdx.x; i < NZ; i += blockDim.x) twz[i] = lane_splat<P>(tw_z[i]);
   // where the tile's segments and records lie (set with the projectors, no pass writes it)
   const bool proj_on = MODE_H && pj.nproj > 0;
   const int tile = ix * Y1 + y1;
@@ -694,11 +708,11 @@ __device__ __forceinline__ void tile_inv_body(int bx, int by, const Lane<T>* __r
   const int e_first = k0 < k1 ? pj.rk_start[k0] + (int)threadIdx.x / VP : 0;
   chain_wait();
   // the (ka, kz) runs of this tile
-  for (int q = threadIdx.x; q < TG::PTS * VP; q += blockDim.x) {
-    const int v = q % VP, pt = q / VP;
+  for (int q = threadIdx.x; q < TG::PTS * TG::CH; q += blockDim.x) {
+    const int c = q % TG::CH * TG::LC, pt = q / TG::CH;
     const int kz = pt % NZ, ka = pt / NZ;
-    cp_async16(S + (ka * ZS + AZ::slot(kz)) * VP + v,
-               tmp + (((long)(grp * Y2 + ka) * NZ + kz) * NX + ix) * (Y1 * VP) + y1 * VP + v);
+    cp_async16(S + (ka * ZS + AZ::slot(kz)) * VP + c,
+               tmp + (((long)(grp * Y2 + ka) * NZ + kz) * NX + ix) * (Y1 * VP) + y1 * VP + c);
   }
   cp_async_commit();
   // the tile's atom projections, in the tile precision, as [segment][l][orbital lane]
@@ -717,7 +731,7 @@ __device__ __forceinline__ void tile_inv_body(int bx, int by, const Lane<T>* __r
       }
     }
     V r;
-    memcpy(&r, w, 16);
+    memcpy(&r, w, sizeof(V));
     return flip(r);
   };
   if (proj_on && pt_staged) {
@@ -785,11 +799,11 @@ __device__ __forceinline__ void tile_inv_body(int bx, int by, const Lane<T>* __r
         for (int l = 0; l < LMAX; ++l) {
           // more atom segments in this tile than staged: projections from global memory
           const V pv = pt_staged ? pt[l * VP] : projection(pj.seg_atom[s0 + cur.tseg], l, v);
-          const P b = splat_of(cur.beta[l]);
+          const P b = splat_of<P>(cur.beta[l]);
           t.x = vfma(b, pv.x, t.x);
           t.y = vfma(b, pv.y, t.y);
         }
-        const P pr = splat_of(cur.ph[0]), pi = splat_of(cur.ph[1]), npi = splat_of(-cur.ph[1]);
+        const P pr = splat_of<P>(cur.ph[0]), pi = splat_of<P>(cur.ph[1]), npi = splat_of<P>(-cur.ph[1]);
         V* dst = S + cur.off * VP + v;
         const V h = *dst;
         *dst = {h.x + vfma(t.x, pr, t.y * pi), h.y + vfma(t.y, pr, t.x * npi)};
@@ -803,7 +817,7 @@ __device__ __forceinline__ void tile_inv_body(int bx, int by, const Lane<T>* __r
   // epilogue: out = alpha (K psi + (V + vshift) psi + V_nl psi) + beta base - minus
   // BE lanes per thread whose loads are issued together
   constexpr int BE = 4;
-  const P ar = splat_of(ep.alpha.x), ai = splat_of(ep.alpha.y), nai = splat_of(-ep.alpha.y);
+  const P ar = splat_of<P>(ep.alpha.x), ai = splat_of<P>(ep.alpha.y), nai = splat_of<P>(-ep.alpha.y);
   // a lane of the output (orbital layout) at point p, orbitals m0 + jb ..
   auto store = [&](long p, int jb, V w) {
     cplx<T>* dst = out + p * ld_out + m0 + jb;
@@ -824,7 +838,7 @@ __device__ __forceinline__ void tile_inv_body(int bx, int by, const Lane<T>* __r
       cplx<T> w[PV];
 #pragma unroll
       for (int k = 0; k < PV; ++k) w[k] = (jb + k < gcount) ? src[p * ld + m0 + jb + k] : mk<T>(0, 0);
-      memcpy(&r, w, 16);
+      memcpy(&r, w, sizeof(V));
     }
     return r;
   };
@@ -860,13 +874,13 @@ __device__ __forceinline__ void tile_inv_body(int bx, int by, const Lane<T>* __r
       const long p = ((long)ix * NY + y1 + Y1 * r) * NZ + z;
       V h = S[(r * ZS + AZ::slot_of_freq(z)) * VP + v];
       const V xv = flip(x[b]);
-      const P vs = splat_of(vp[b]);
+      const P vs = splat_of<P>(vp[b]);
       h = {vfma(vs, xv.x, h.x), vfma(vs, xv.y, h.y)};
       V o = {vfma(h.x, ar, h.y * nai), vfma(h.x, ai, h.y * ar)};
       if (ep.base) {
         // base the input block itself (a Taylor series' first term, 1 + c H): already here
         const V bb = own ? xv : flip(load(ep.base, ep.ld_base, p, v * PV, b16));
-        const P br = splat_of(ep.beta.x), bi = splat_of(ep.beta.y), nbi = splat_of(-ep.beta.y);
+        const P br = splat_of<P>(ep.beta.x), bi = splat_of<P>(ep.beta.y), nbi = splat_of<P>(-ep.beta.y);
         o.x = o.x + vfma(bb.x, br, bb.y * nbi);
         o.y = o.y + vfma(bb.x, bi, bb.y * br);
       }
@@ -877,8 +891,8 @@ __device__ __forceinline__ void tile_inv_body(int bx, int by, const Lane<T>* __r
 }
 
 template <typename T, int NX, int NY, int NZ, int MODE_H = 1>
-__global__ void __launch_bounds__(256, TileGeom<T, NX, NY, NZ>::INV_MIN_CTAS)
-    k_tile_inv(const Lane<T>* __restrict__ tmp, const cplx<T>* __restrict__ in, long ld_in,
+__global__ void __launch_bounds__(TileGeom<T, NX, NY, NZ>::ZT, TileGeom<T, NX, NY, NZ>::INV_MIN_CTAS)
+    k_tile_inv(const typename TileGeom<T, NX, NY, NZ>::V* __restrict__ tmp, const cplx<T>* __restrict__ in, long ld_in,
                cplx<T>* __restrict__ out, long ld_out, int M, const cplx<T>* __restrict__ tw_y,
                const cplx<T>* __restrict__ tw_z, ProjView<T> pj, EpiParams<T> ep, int seg_cap, int vec) {
   tile_inv_body<T, NX, NY, NZ, MODE_H>(blockIdx.x, blockIdx.y, tmp, in, ld_in, out, ld_out, M, tw_y, tw_z, pj, ep,

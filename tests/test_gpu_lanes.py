@@ -78,3 +78,23 @@ def test_more_atoms_than_a_tile_stages(pb, oracle_mod, precision, tol, atoms):
     # up to 360 entries a point: their FP32 sum is within about sqrt(360) 6e-8 of its terms' norm
     assert rel_max(h(x).cpu().numpy(), o.apply_h(x.cpu().numpy().astype(np.complex128))) < tol
     assert torch.equal(h(x), h(x))
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-13), ("mixed", 1e-6)])
+@pytest.mark.parametrize("n,M", [(80, 1), (80, 7), (80, 17), (128, 5)])
+def test_long_axes(pb, precision, tol, n, M):
+    """Axes whose transforms are longer than 12 values: one orbital a lane in FP32, 512
+    threads in the first and third pass, against the same passes with 64 and 256 threads
+    (sums of the projections in another order), in rows of both alignments."""
+    sysd = small_system(pb, n=n, a=0.3 * n, M=1)
+    h = make_product(pb, sysd, precision, (0.02, 0.0, 0.01))
+    x, _, view = _pair(h, M, 1)
+    y = h(x)
+    assert torch.isfinite(torch.view_as_real(y)).all()
+    assert torch.equal(y, h(view))
+    for threads in (64, 256):
+        h.set_schedule(M, (1, threads, threads, threads))
+        assert float((h(x) - y).norm() / y.norm()) < tol
+    picked = h.autotune(M)
+    h.set_schedule(M, picked)  # what the tuner picks can be set again
+    assert float((h(x) - y).norm() / y.norm()) < tol
