@@ -11,6 +11,7 @@
 #include <mutex>
 
 #include "dft.cuh"
+#include "dmma.cuh"
 #include "inqb_internal.h"
 #include "observables.h"
 
@@ -100,17 +101,30 @@ __global__ void k_dipole(const double* __restrict__ rho, long N, LatticeView g, 
 __device__ __forceinline__ int grid_row() { return (threadIdx.x / 32) % 4 * 4 + threadIdx.x % 32 / 8; }
 __device__ __forceinline__ int grid_col() { return threadIdx.x / 128 * 8 + threadIdx.x % 8; }
 
-// S[i][j] += dV sum_{p in slab} conj(a[p][i]) b[p][j], FP64 products and sums.  256
-// threads as 16 x 16, TM x TM outputs a thread (outputs ti + 16 a, tj + 16 b), so a CTA
-// holds a (16 TM)^2 tile in registers over its slab of points; KP points are staged at a
-// time, the next ones fetched into registers meanwhile.  The pass is bound by the FP64
-// units: a thread's TM^2 complex products take 4 TM^2 DFMA for 2 TM 16-byte shared loads.
+// tile t of the tiles on and above the diagonal: (0, 0..), (1, 1..), ...
+__device__ __forceinline__ void overlap_tile(int t, int tiles_j, bool upper, int& bi, int& bj) {
+  if (upper) {
+    bi = 0;
+    while (t >= tiles_j - bi) t -= tiles_j - bi++;
+    bj = bi + t;
+  } else {
+    bi = t / tiles_j;
+    bj = t % tiles_j;
+  }
+}
+
+// S[i][j] += dV sum_{p in slab} conj(a[p][i]) b[p][j], FP64 products and sums.
 // The square overlap (upper) computes the tiles on and above the diagonal only, which is
 // all the Cholesky factorisation reads.
+//
+// Tiles of 16 and 32 outputs a side (TM = 1, 2), for blocks of at most 32 orbitals: 256
+// threads as 16 x 16, TM x TM outputs a thread (outputs ti + 16 a, tj + 16 b) over the
+// CTA's slab of points; KP points are staged at a time, the next ones fetched into
+// registers meanwhile.
 template <int TM>
 struct OverlapCfg {
-  static constexpr int KP = TM == 4 ? 8 : TM == 2 ? 16 : 32;
-  static constexpr int CTAS = TM == 4 ? 2 : 4;  // per SM
+  static constexpr int KP = TM == 2 ? 16 : 32;
+  static constexpr int CTAS = 4;  // per SM
 };
 
 template <typename T, int TM>
@@ -121,15 +135,7 @@ __global__ void __launch_bounds__(256, OverlapCfg<TM>::CTAS)
   __shared__ double2 sa[KP][TILE], sb[KP][TILE];
   const int tiles_j = (Mb + TILE - 1) / TILE;
   int bi, bj;
-  if (upper) {  // tile blockIdx.x of the rows (0, 0..), (1, 1..), ...
-    int t = blockIdx.x;
-    bi = 0;
-    while (t >= tiles_j - bi) t -= tiles_j - bi++;
-    bj = bi + t;
-  } else {
-    bi = blockIdx.x / tiles_j;
-    bj = blockIdx.x % tiles_j;
-  }
+  overlap_tile(blockIdx.x, tiles_j, upper, bi, bj);
   const int i0 = bi * TILE, j0 = bj * TILE;
   const bool diag = upper && bi == bj;  // one block serves both sides
   const int ti = grid_row(), tj = grid_col();
@@ -188,6 +194,88 @@ __global__ void __launch_bounds__(256, OverlapCfg<TM>::CTAS)
         atomicAdd(&S[(long)i * lds + j].x, dV * re[a][b]);
         atomicAdd(&S[(long)i * lds + j].y, dV * im[a][b]);
       }
+    }
+}
+
+// Slabs of points per tile in proportion to its work, so that the CTAs of a wave end
+// together: a tile takes the time of its busiest warp (8-wide blocks: 16, on the diagonal 9,
+// less at the edges) and one more for the chunk's loads and barrier.
+struct OverlapShare {
+  long ctas, total, most;  // CTAs of the launch, sum of the weights, slabs a tile may have
+  __host__ __device__ static int weight(int bi, int bj, int Ma, int Mb, bool upper) {
+    const int ra = (Ma - bi * kDT + 7) / 8, rb = (Mb - bj * kDT + 7) / 8;
+    const int rows = ra < 8 ? ra : 8, cols = rb < 8 ? rb : 8;
+    if (upper && bi == bj) return (cols < 8 ? cols : 9) + 1;
+    return cols * (rows > 4 ? 2 : 1) + 1;
+  }
+  __host__ __device__ int slabs(int bi, int bj, int Ma, int Mb, bool upper) const {
+    const long n = ctas * weight(bi, bj, Ma, Mb, upper) / total;
+    return (int)(n < 1 ? 1 : n < most ? n : most);
+  }
+};
+
+// The same overlap with tiles of 64 on the FP64 tensor instruction: a warp's 64 products of
+// a staged quad of points take 10 shared loads, where 4 x 4 outputs a thread on FMAs took 8
+// loads for 64 FMAs and waited for them (64^3 points x 128 orbitals complex128: 1.19 ->
+// 0.69 ms).  Bound by the FP64 pipe, 81% busy.
+template <typename T>
+__global__ void __launch_bounds__(kDThreads, 2)
+    k_overlap_dmma(const cplx<T>* __restrict__ pa, long lda, int Ma, const cplx<T>* __restrict__ pb, long ldb, int Mb,
+                   long N, OverlapShare share, double dV, double2* __restrict__ S, long lds, int upper) {
+  __shared__ DmmaBuf sa[2], sb[2];
+  int bi = 0, bj = 0, first = 0, slabs = share.slabs(0, 0, Ma, Mb, upper);
+  while ((int)blockIdx.x >= first + slabs) {  // the tile whose slabs hold this CTA
+    first += slabs;
+    if (++bj * kDT >= Mb) bj = upper ? ++bi : (++bi, 0);
+    slabs = share.slabs(bi, bj, Ma, Mb, upper);
+  }
+  const long slab = ((N + slabs - 1) / slabs + kDK - 1) / kDK * kDK;
+  const int i0 = bi * kDT, j0 = bj * kDT;
+  const bool diag = upper && bi == bj;  // one block serves both sides
+  const long p0 = (blockIdx.x - first) * slab, p1 = min(N, p0 + slab);
+  if (p0 >= N) return;
+  DmmaTile t;
+  t.clear();
+  const int rows = min(8, (Ma - i0 + 7) / 8), hi = min(8, (Mb - j0 + 7) / 8);
+  DmmaOperand<T, false> oa, ob;
+  auto load = [&](long pc, int buf) {
+    oa.load(sa[buf], pa, [&](int q, int j) { return pc + q < p1 && i0 + j < Ma ? (pc + q) * lda + i0 + j : -1L; });
+    if (!diag)
+      ob.load(sb[buf], pb, [&](int q, int j) { return pc + q < p1 && j0 + j < Mb ? (pc + q) * ldb + j0 + j : -1L; });
+    dmma_commit();
+  };
+  auto store = [&](int buf) {
+    oa.store(sa[buf]);
+    if (!diag) ob.store(sb[buf]);
+  };
+  load(p0, 0);
+  store(0);
+  int buf = 0;
+  for (long pc = p0; pc < p1; pc += kDK, buf ^= 1) {
+    dmma_arrived();
+    __syncthreads();  // chunk pc is complete, and every warp has left the other buffer
+    const bool more = pc + kDK < p1;
+    if (more) load(pc + kDK, buf ^ 1);
+    if (diag)
+      t.mul_upper<kConjX>(sa[buf], sa[buf], hi, DmmaNoWeight());
+    else
+      t.mul_block<kConjX>(sa[buf], sb[buf], rows, hi, DmmaNoWeight());
+    if (more) store(buf ^ 1);
+  }
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int i = i0 + 8 * DmmaTile::row_block(a) + (lane >> 2), j = j0 + 8 * c + 2 * (lane & 3);
+      auto add = [&](int jj, double x, double y) {
+        if (i < Ma && jj < Mb && !(upper && i > jj)) {
+          atomicAdd(&S[(long)i * lds + jj].x, dV * x);
+          atomicAdd(&S[(long)i * lds + jj].y, dV * y);
+        }
+      };
+      add(j, t.re[a][c].x, t.im[a][c].x);
+      add(j + 1, t.re[a][c].y, t.im[a][c].y);
     }
 }
 
@@ -384,14 +472,16 @@ __global__ void __launch_bounds__(256) k_chol_inverse(double2* S, long lds, cons
 }
 
 // ---------------------------------------------------------------- rotation
-// out[p][j] = sum_i a[p][i] R[i][j], FP64 arithmetic.  A CTA owns 64 points and (16 TN)
-// columns at a time, 256 threads as 16 x 16 with 4 x TN outputs each; eight orbitals i are
-// staged at a time, the next ones fetched into registers meanwhile.
+// out[p][j] = sum_i a[p][i] R[i][j], FP64 arithmetic.  A CTA owns 64 points and a block of
+// columns at a time; eight orbitals i are staged at a time, the next ones fetched into
+// registers meanwhile.
 // UPPER: R is upper triangular and out may be a.  The CTA walks its columns from the last
 // block down: a block of outputs reads only the input columns up to itself, so it may
 // overwrite its own input columns once they are read.
+//
+// At most 32 columns: (16 TN) of them, 256 threads as 16 x 16 with 4 x TN outputs each.
 template <typename T, int TN, bool UPPER>
-__global__ void __launch_bounds__(256, TN == 4 ? 2 : 3)
+__global__ void __launch_bounds__(256, 3)
     k_rotate(const cplx<T>* a, long lda, int Ma, const double2* __restrict__ R, long ldr, int Mo, cplx<T>* out,
              long ldo, long N) {
   constexpr int TP = 4, PTS = 16 * TP, COLS = 16 * TN, KP = 8;
@@ -467,6 +557,62 @@ __global__ void __launch_bounds__(256, TN == 4 ? 2 : 3)
         const long p = p0 + tp + 16 * u;
         const int j = j0 + tj + 16 * v;
         if (p < N && j < Mo) out[p * ldo + j] = mk<T>((T)re[u][v], (T)im[u][v]);
+      }
+  }
+}
+
+// More columns: 64 at a time on the FP64 tensor instruction, a warp 16 points x 64 columns
+// (64^3 points x 128 orbitals complex128, triangular: 1.00 -> 0.77 ms; FP64 pipe 69% busy).
+// The chunks of all column blocks are one pipeline.
+// ADJ: the factor is R^H instead.
+template <typename T, bool UPPER, bool ADJ>
+__global__ void __launch_bounds__(kDThreads, 2)
+    k_rotate_dmma(const cplx<T>* a, long lda, int Ma, const double2* __restrict__ R, long ldr, int Mo, cplx<T>* out,
+                  long ldo, long N) {
+  __shared__ DmmaBuf sa[2], sr[2];  // [i][point], [i][column]
+  const cplx<double>* Rc = reinterpret_cast<const cplx<double>*>(R);
+  const long p0 = (long)blockIdx.x * kDT;
+  const int nblk = (Mo + kDT - 1) / kDT;
+  const int b_hi = UPPER ? nblk - 1 : (int)blockIdx.y, b_lo = UPPER ? 0 : (int)blockIdx.y;
+  DmmaOperand<T, true> oa;
+  DmmaOperand<double, ADJ> orr;
+  auto depth = [&](int jb) { return UPPER ? min(Ma, (jb + 1) * kDT) : Ma; };  // input columns of block jb
+  auto load = [&](int jb, int k0, int buf) {
+    const int j0 = jb * kDT, kend = depth(jb);
+    oa.load(sa[buf], a, [&](int q, int p) { return p0 + p < N && k0 + q < kend ? (p0 + p) * lda + k0 + q : -1L; });
+    orr.load(sr[buf], Rc, [&](int q, int j) {
+      return k0 + q < kend && j0 + j < Mo ? (ADJ ? (j0 + j) * ldr + k0 + q : (k0 + q) * ldr + j0 + j) : -1L;
+    });
+    dmma_commit();
+  };
+  load(b_hi, 0, 0);
+  oa.store(sa[0]);
+  int buf = 0;
+  for (int jb = b_hi; jb >= b_lo; --jb) {
+    const int j0 = jb * kDT, kend = depth(jb);
+    const int hi = min(8, (Mo - j0 + 7) / 8);
+    DmmaTile t;
+    t.clear();
+    for (int k0 = 0; k0 < kend; k0 += kDK, buf ^= 1) {
+      dmma_arrived();
+      __syncthreads();  // chunk k0 is complete, and every warp has left the other buffer
+      // the next chunk, or the first of the next block: columns that this block does not write
+      const bool last = k0 + kDK >= kend, more = !last || jb > b_lo;
+      if (more) load(last ? jb - 1 : jb, last ? 0 : k0 + kDK, buf ^ 1);
+      // UPPER: R[i][j] = 0 for the 8-wide column blocks left of row i
+      const int first = UPPER ? max(0, (k0 - j0) / 8) : 0;
+      t.mul_right<ADJ ? kConjY : kConjNone>(sa[buf], sr[buf], first, hi, DmmaNoWeight());
+      if (more) oa.store(sa[buf ^ 1]);
+    }
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const long p = p0 + 8 * DmmaTile::row_block(r) + (lane >> 2);
+        const int j = j0 + 8 * c + 2 * (lane & 3);
+        if (p < N && j < Mo) out[p * ldo + j] = mk<T>((T)t.re[r][c].x, (T)t.im[r][c].x);
+        if (p < N && j + 1 < Mo) out[p * ldo + j + 1] = mk<T>((T)t.re[r][c].y, (T)t.im[r][c].y);
       }
   }
 }
@@ -557,8 +703,7 @@ int launch_dipole(const double* rho, long N, const double lat[3][3], const int n
   return INQB_OK;
 }
 
-// tiles of the output at TM outputs a side per thread; slabs of points so that the CTAs
-// fill the GPU (at least 512 points a slab)
+// tiles of the output and slabs of points (at least 512 each) so that the CTAs fill the GPU
 template <typename T, int TM>
 static int overlap_launch(const void* a, long lda, int Ma, const void* b, long ldb, int Mb, long N, double dV,
                           double2* S, long lds, bool upper, cudaStream_t st) {
@@ -574,6 +719,24 @@ static int overlap_launch(const void* a, long lda, int Ma, const void* b, long l
   return INQB_OK;
 }
 
+template <typename T>
+static int overlap_dmma_launch(const void* a, long lda, int Ma, const void* b, long ldb, int Mb, long N, double dV,
+                               double2* S, long lds, bool upper, cudaStream_t st) {
+  const int ti = (Ma + kDT - 1) / kDT, tj = (Mb + kDT - 1) / kDT;
+  // one wave of CTAs for one tile, else two (64^3 x 64, 128, 256 orbitals, whole call: one wave
+  // 529, 1542, 5327 us, two 560, 1531, 5224)
+  OverlapShare share = {ti * tj == 1 ? 148 * 2 : 148 * 4, 0, std::max<long>(1, N / 512)};
+  for (int i = 0; i < ti; i++)
+    for (int j = upper ? i : 0; j < tj; j++) share.total += OverlapShare::weight(i, j, Ma, Mb, upper);
+  unsigned blocks = 0;
+  for (int i = 0; i < ti; i++)
+    for (int j = upper ? i : 0; j < tj; j++) blocks += share.slabs(i, j, Ma, Mb, upper);
+  k_overlap_dmma<T><<<blocks, kDThreads, 0, st>>>((const cplx<T>*)a, lda, Ma, (const cplx<T>*)b, ldb, Mb, N, share, dV,
+                                                  S, lds, upper);
+  INQB_CUDA_TRY(cudaGetLastError());
+  return INQB_OK;
+}
+
 // the tile follows the larger block: a 16- or 32-wide tile where a 64-wide one would be
 // mostly padding
 template <typename T>
@@ -582,7 +745,7 @@ static int overlap_any(const void* a, long lda, int Ma, const void* b, long ldb,
   const int M = std::max(Ma, Mb);
   if (M <= 16) return overlap_launch<T, 1>(a, lda, Ma, b, ldb, Mb, N, dV, S, lds, upper, st);
   if (M <= 32) return overlap_launch<T, 2>(a, lda, Ma, b, ldb, Mb, N, dV, S, lds, upper, st);
-  return overlap_launch<T, 4>(a, lda, Ma, b, ldb, Mb, N, dV, S, lds, upper, st);
+  return overlap_dmma_launch<T>(a, lda, Ma, b, ldb, Mb, N, dV, S, lds, upper, st);
 }
 
 // S (upper triangle of a Hermitian matrix) <- U^-1; X: M x M scratch (receives U)
@@ -618,7 +781,10 @@ static int rotate_any(const void* a, long lda, int Ma, const double2* R, long ld
                       cudaStream_t st) {
   if (Mo <= 16) return rotate_launch<T, 1, UPPER>(a, lda, Ma, R, ldr, Mo, out, ldo, N, st);
   if (Mo <= 32) return rotate_launch<T, 2, UPPER>(a, lda, Ma, R, ldr, Mo, out, ldo, N, st);
-  return rotate_launch<T, 4, UPPER>(a, lda, Ma, R, ldr, Mo, out, ldo, N, st);
+  const dim3 grid((unsigned)((N + kDT - 1) / kDT), UPPER ? 1u : (unsigned)((Mo + kDT - 1) / kDT));
+  k_rotate_dmma<T, UPPER, false><<<grid, kDThreads, 0, st>>>((const cplx<T>*)a, lda, Ma, R, ldr, Mo, (cplx<T>*)out, ldo, N);
+  INQB_CUDA_TRY(cudaGetLastError());
+  return INQB_OK;
 }
 
 template <typename T>
@@ -666,6 +832,16 @@ int launch_rotate_block(int precision, const void* a, long lda, int Ma, const do
   return precision == INQB_FP64
              ? rotate_any<double, false>(a, lda, Ma, R, ldr, Mo, out, ldo, N, (cudaStream_t)stream)
              : rotate_any<float, false>(a, lda, Ma, R, ldr, Mo, out, ldo, N, (cudaStream_t)stream);
+}
+
+// out[p][j] = sum_i psi[p][i] conj(u[j][i]) for complex128 orbitals, u M x M
+int launch_rotate_adjoint(const void* psi, long ld, int M, const double2* u, void* out, long ldo, long N,
+                          void* stream) {
+  const dim3 grid((unsigned)((N + kDT - 1) / kDT), (unsigned)((M + kDT - 1) / kDT));
+  k_rotate_dmma<double, false, true><<<grid, kDThreads, 0, (cudaStream_t)stream>>>(
+      (const cplx<double>*)psi, ld, M, u, M, M, (cplx<double>*)out, ldo, N);
+  INQB_CUDA_TRY(cudaGetLastError());
+  return INQB_OK;
 }
 
 // ---------------------------------------------------------------- orthonormalisation without allocation

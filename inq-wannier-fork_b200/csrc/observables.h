@@ -18,6 +18,8 @@ int launch_orthonormalize(int precision, void* psi, long ld, int M, long N, doub
 int launch_overlap_block(int precision, const void* a, long lda, int Ma, const void* b, long ldb, int Mb, long N,
                          double dV, double2* S, long lds, void* stream);
 int launch_cholesky_inverse(double2* S, int M, long lds, double2* X, int* info, void* stream);
+int launch_rotate_adjoint(const void* psi, long ld, int M, const double2* u, void* out, long ldo, long N,
+                          void* stream);
 int launch_rotate_block(int precision, const void* a, long lda, int Ma, const double2* R, long ldr, int Mo,
                         void* out, long ldo, long N, void* stream);
 // Largest orbital count of the allocation-free orthonormalisation (fixed device scratch).

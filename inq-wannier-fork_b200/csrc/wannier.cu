@@ -13,7 +13,8 @@
 //            multiplies dense M x M rotation matrices (7 GEMMs per step); the pairs are
 //            disjoint, so rotating two rows per pair is the same product in O(M) per pair.
 //   adiag    adiag[k][i] = sum_j conj(a_k[i][j]) u[i][j]
-//   rotate   psi <- psi u^H (operations::rotate), tiled through shared memory
+//   rotate   psi <- psi u^H (operations::rotate), tiled through shared memory; complex128
+//            orbitals by the rotation kernel of observables.cu
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -21,7 +22,9 @@
 #include <cmath>
 
 #include "dft.cuh"
+#include "dmma.cuh"
 #include "inqb_internal.h"
+#include "observables.h"
 #include "wannier.h"
 
 namespace inqb {
@@ -34,14 +37,12 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
 __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
 
 // ------------------------------------------------------------------ gram
-// 256 threads as 16 x 16; thread (tm, tn) holds outputs m = m0 + tm + 16 a (a < TMX),
-// n = n0 + tn + 16 b (b < TNX) for the three directions; CTA tile (16 TMX) x (16 TNX).
 // Axis lengths are those of the FFT size table, N below 2^31.
 // FP64 contexts accumulate in FP64 over the CTA's slab (few slabs).  The mixed context
 // accumulates FP32 products in FP32 over a slab of at most kSlabF32 points and keeps one
 // FP32 partial per slab; the finish kernel adds the slabs in FP64 (the FP32 rounding of
 // a slab sum is about 6e-8 sqrt(kSlabF32) of its size, about 1e-7 of the total after the
-// FP64 sum over slabs).  Freeing the FP64 registers lets the FP32 tile be 4 x 2.
+// FP64 sum over slabs).
 constexpr long kSlabF32 = 1024;    // points per slab in the mixed precision
 
 struct GramGeom {
@@ -53,17 +54,14 @@ template <typename T>
 struct GramCfg;
 template <>
 struct GramCfg<double> {
-  static constexpr int TMX = 4, TNX = 2, GP = 16, MINB = 1;  // GP: points per staged chunk
-  using P = double2;                                         // partial type
+  static constexpr int TILE_M = kDT, TILE_N = kDT, GP = kDK;  // GP: points per staged chunk
+  using P = double2;                                          // partial type
 };
 template <>
 struct GramCfg<float> {
-  static constexpr int TMX = 4, TNX = 2, GP = 16, MINB = 3;
+  static constexpr int TMX = 4, TNX = 2, TILE_M = 16 * TMX, TILE_N = 16 * TNX, GP = 16;
   using P = float2;
 };
-
-__device__ __forceinline__ void store_partial(double2* p, double x, double y) { *p = make_double2(x, y); }
-__device__ __forceinline__ void store_partial(float2* p, float x, float y) { *p = make_float2(x, y); }
 
 // e^{i theta_d} factorises over the axes: axis table entry [d][j][n] = exp(i pi
 // frac_to_theta[d][j] f_j(n)), n a grid index of axis j (at most kAxisMax of them).
@@ -78,18 +76,70 @@ __global__ void k_mlwf_axis(GramGeom geo, double2* __restrict__ tab) {
   }
 }
 
-// grid (tiles_m * tiles_n, nslab).  Bound by the FP64 (FP32) units: 4 x 2 outputs of three
-// directions take 96 fused multiply-adds for 10 shared loads.  The next chunk's orbitals
-// are fetched into registers and its weights formed from the axis tables while the current
-// chunk is summed.
-template <typename T>
-__global__ void __launch_bounds__(256, GramCfg<T>::MINB)
-    k_mlwf_gram(const cplx<T>* __restrict__ pa, long lda, int Ma, const cplx<T>* __restrict__ pb, long ldb, int Mb,
-                long N, GramGeom geo, const double2* __restrict__ tab, long pts_per_slab,
-                typename GramCfg<T>::P* __restrict__ partial) {
-  using R = T;
-  constexpr int TMX = GramCfg<T>::TMX, TNX = GramCfg<T>::TNX, kGP = GramCfg<T>::GP;
-  constexpr int TILE_M = 16 * TMX, TILE_N = 16 * TNX;
+__device__ __forceinline__ double2 gram_weight(const GramGeom& geo, const double2* tab, int d, long point) {
+  const unsigned p = (unsigned)point;
+  const unsigned iz = p % geo.nr[2], r = p / geo.nr[2], iy = r % geo.nr[1], ix = r / geo.nr[1];
+  const double2* t = tab + d * 3 * kAxisMax;
+  return cmul(cmul(t[ix], t[kAxisMax + iy]), t[2 * kAxisMax + iz]);
+}
+
+// FP64: grid (tiles_m * tiles_n, nslab, 3), a 64 x 64 tile of one direction on the FP64
+// tensor instruction (DmmaTile), the weight multiplied into the left operand as it is read
+// (conj(a) w = conj(a conj(w))).  4 x 2 outputs a thread of the three directions on FMAs
+// waited for their shared loads and did a narrow tile's padding (whole TD-MLWF step at 48^3:
+// 8 states 463 -> 319 us, 64 states 1905 -> 1790 us).
+__global__ void __launch_bounds__(kDThreads, 2)
+    k_mlwf_gram_dmma(const cplx<double>* __restrict__ pa, long lda, int Ma, const cplx<double>* __restrict__ pb,
+                     long ldb, int Mb, long N, GramGeom geo, const double2* __restrict__ tab, long pts_per_slab,
+                     double2* __restrict__ partial) {
+  __shared__ DmmaBuf sa[2], sb[2];
+  __shared__ double2 sw[2][kDK];
+  const int tiles_m = (Ma + kDT - 1) / kDT, d = blockIdx.z;
+  const int m0 = (blockIdx.x % tiles_m) * kDT, n0 = (blockIdx.x / tiles_m) * kDT;
+  const long p_beg = (long)blockIdx.y * pts_per_slab, p_end = min(N, p_beg + pts_per_slab);
+  DmmaTile t;
+  t.clear();
+  const int rows = min(8, (Ma - m0 + 7) / 8), hi = min(8, (Mb - n0 + 7) / 8);
+  DmmaOperand<double, false> oa, ob;
+  auto load = [&](long pc, int buf) {
+    oa.load(sa[buf], pa, [&](int q, int j) { return pc + q < p_end && m0 + j < Ma ? (pc + q) * lda + m0 + j : -1L; });
+    ob.load(sb[buf], pb, [&](int q, int j) { return pc + q < p_end && n0 + j < Mb ? (pc + q) * ldb + n0 + j : -1L; });
+    dmma_commit();
+    if (threadIdx.x < kDK) sw[buf][threadIdx.x] = gram_weight(geo, tab, d, min(pc + (long)threadIdx.x, N - 1));
+  };
+  load(p_beg, 0);
+  int buf = 0;
+  for (long pc = p_beg; pc < p_end; pc += kDK, buf ^= 1) {
+    dmma_arrived();
+    __syncthreads();  // chunk pc is complete, and every warp has left the other buffer
+    if (pc + kDK < p_end) load(pc + kDK, buf ^ 1);
+    t.mul_block<kConjX>(sa[buf], sb[buf], rows, hi, [&](double2 u, int k) { return cmul(u, cconj(sw[buf][k])); });
+  }
+  // partial[slab][d][m][n], m < Ma, n < Mb
+  double2* out = partial + ((size_t)blockIdx.y * 3 + d) * Ma * Mb;
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int m = m0 + 8 * DmmaTile::row_block(a) + (lane >> 2), n = n0 + 8 * c + 2 * (lane & 3);
+      if (m < Ma && n < Mb) out[(size_t)m * Mb + n] = make_double2(t.re[a][c].x, t.im[a][c].x);
+      if (m < Ma && n + 1 < Mb) out[(size_t)m * Mb + n + 1] = make_double2(t.re[a][c].y, t.im[a][c].y);
+    }
+}
+
+// FP32: grid (tiles_m * tiles_n, nslab), 256 threads as 16 x 16; thread (tm, tn) holds outputs
+// m = m0 + tm + 16 a (a < TMX), n = n0 + tn + 16 b (b < TNX) for the three directions.  Bound
+// by the FP32 units: 4 x 2 outputs of three directions take 96 fused multiply-adds for 10
+// shared loads.  The next chunk's orbitals are fetched into registers and its weights formed
+// from the axis tables while the current chunk is summed.
+__global__ void __launch_bounds__(256, 3)
+    k_mlwf_gram(const cplx<float>* __restrict__ pa, long lda, int Ma, const cplx<float>* __restrict__ pb, long ldb,
+                int Mb, long N, GramGeom geo, const double2* __restrict__ tab, long pts_per_slab,
+                float2* __restrict__ partial) {
+  using R = float;
+  constexpr int TMX = GramCfg<R>::TMX, TNX = GramCfg<R>::TNX, kGP = GramCfg<R>::GP;
+  constexpr int TILE_M = GramCfg<R>::TILE_M, TILE_N = GramCfg<R>::TILE_N;
   constexpr int PA = kGP * TILE_M / 256, PB = kGP * TILE_N / 256;
   __shared__ cplx<R> sA[kGP][TILE_M];
   __shared__ cplx<R> sB[3][kGP][TILE_N];
@@ -123,10 +173,7 @@ __global__ void __launch_bounds__(256, GramCfg<T>::MINB)
   auto weights = [&](long pc, int buf) {
     if (threadIdx.x >= 3 * kGP) return;
     const int d = threadIdx.x / kGP, q = threadIdx.x % kGP;
-    const unsigned p = (unsigned)min(pc + q, N - 1);
-    const unsigned iz = p % geo.nr[2], r = p / geo.nr[2], iy = r % geo.nr[1], ix = r / geo.nr[1];
-    const double2* t = tab + d * 3 * kAxisMax;
-    const double2 w = cmul(cmul(t[ix], t[kAxisMax + iy]), t[2 * kAxisMax + iz]);
+    const double2 w = gram_weight(geo, tab, d, min(pc + q, N - 1));
     sW[buf][d][q] = mk<R>((R)w.x, (R)w.y);
   };
   fetch(p_beg);
@@ -182,8 +229,8 @@ __global__ void __launch_bounds__(256, GramCfg<T>::MINB)
       for (int b = 0; b < TNX; ++b) {
         const int m = m0 + tm + 16 * a, n = n0 + tn + 16 * b;
         if (m < Ma && n < Mb)
-          store_partial(&partial[((size_t)blockIdx.y * 3 + d) * MM + (size_t)m * Mb + n], acc[d][a][b][0],
-                        acc[d][a][b][1]);
+          partial[((size_t)blockIdx.y * 3 + d) * MM + (size_t)m * Mb + n] =
+              make_float2(acc[d][a][b][0], acc[d][a][b][1]);
       }
 }
 
@@ -799,17 +846,15 @@ __global__ void __launch_bounds__(128)
 }
 
 // ------------------------------------------------------------------ rotate
-// out[p][i] = sum_j psi[p][j] conj(u[i][j]); 64 x 64 output tiles, 256 threads with
-// 4 x 4 outputs each, j in chunks of 8 through shared memory.
+// out[p][i] = sum_j psi[p][j] conj(u[i][j]) in FP32 (complex128 orbitals: launch_rotate_adjoint);
+// 64 x 64 output tiles, 256 threads with 4 x 4 outputs each, j in chunks of 8 through shared
+// memory.
 constexpr int kRT = 64, kRK = 8;
 
-// FP64: 128 registers for two CTAs per SM (136 unbounded, one CTA: 2.98 -> 2.09 ms at
-// 64^3 x 128 states); FP32 runs best unbounded
-template <typename T>
-__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 1)
-    k_mlwf_rotate(const cplx<T>* __restrict__ psi, long ld, int M, long N, const double2* __restrict__ u,
-                  cplx<T>* __restrict__ out, long ldo) {
-  using R = T;
+__global__ void __launch_bounds__(256)
+    k_mlwf_rotate(const cplx<float>* __restrict__ psi, long ld, int M, long N, const double2* __restrict__ u,
+                  cplx<float>* __restrict__ out, long ldo) {
+  using R = float;
   __shared__ cplx<R> sP[kRK][kRT + 1];  // [j][point]
   __shared__ cplx<R> sU[kRK][kRT];      // [j][i] = conj(u[i][j])
   const long p0 = (long)blockIdx.x * kRT;
@@ -868,11 +913,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 1)
 namespace {
 template <typename T>
 long gram_slabs(long N, int Ma, int Mb) {
-  constexpr int TM = 16 * GramCfg<T>::TMX, TN = 16 * GramCfg<T>::TNX, kGP = GramCfg<T>::GP;
-  const long tiles = (long)((Ma + TM - 1) / TM) * ((Mb + TN - 1) / TN);
-  const long chunks = (N + kGP - 1) / kGP;
   if (sizeof(T) == 4) return std::max<long>(1, (N + kSlabF32 - 1) / kSlabF32);
-  return std::max<long>(1, std::min<long>(chunks, (148L * 2 + tiles - 1) / tiles));
+  constexpr int TM = GramCfg<T>::TILE_M, TN = GramCfg<T>::TILE_N;
+  const long tiles = 3L * ((Ma + TM - 1) / TM) * ((Mb + TN - 1) / TN);
+  const long chunks = (N + GramCfg<T>::GP - 1) / GramCfg<T>::GP;
+  return std::max<long>(1, std::min<long>(chunks, 148L * 4 / tiles));  // two waves of 2 CTAs an SM
 }
 size_t slab_bytes(long N, int Ma, int Mb) {
   const size_t MM = (size_t)Ma * Mb;
@@ -894,16 +939,20 @@ template <typename T>
 static int gram_impl(const void* pa, long lda, int Ma, const void* pb, long ldb, int Mb, long N, const GramGeom& g,
                      void* partial, double2** Zout, cudaStream_t st) {
   using P = typename GramCfg<T>::P;
-  constexpr int TM = 16 * GramCfg<T>::TMX, TN = 16 * GramCfg<T>::TNX, kGP = GramCfg<T>::GP;
+  constexpr int TM = GramCfg<T>::TILE_M, TN = GramCfg<T>::TILE_N, kGP = GramCfg<T>::GP;
   const long slabs = gram_slabs<T>(N, Ma, Mb);
   const long per = ((N + slabs - 1) / slabs + kGP - 1) / kGP * kGP;
   const long nslab = (N + per - 1) / per;
-  const dim3 grid((unsigned)(((Ma + TM - 1) / TM) * ((Mb + TN - 1) / TN)), (unsigned)nslab);
+  const unsigned tiles = (unsigned)(((Ma + TM - 1) / TM) * ((Mb + TN - 1) / TN));
   double2* Z = reinterpret_cast<double2*>(static_cast<char*>(partial) + (slab_bytes(N, Ma, Mb) + 255) / 256 * 256);
   double2* tab = Z + 3 * (size_t)Ma * Mb;
   k_mlwf_axis<<<9, 128, 0, st>>>(g, tab);
-  k_mlwf_gram<T><<<grid, 256, 0, st>>>((const cplx<T>*)pa, lda, Ma, (const cplx<T>*)pb, ldb, Mb, N, g, tab, per,
-                                       (P*)partial);
+  if constexpr (sizeof(T) == 8)
+    k_mlwf_gram_dmma<<<dim3(tiles, (unsigned)nslab, 3), kDThreads, 0, st>>>(
+        (const cplx<T>*)pa, lda, Ma, (const cplx<T>*)pb, ldb, Mb, N, g, tab, per, (P*)partial);
+  else
+    k_mlwf_gram<<<dim3(tiles, (unsigned)nslab), 256, 0, st>>>((const cplx<T>*)pa, lda, Ma, (const cplx<T>*)pb, ldb,
+                                                              Mb, N, g, tab, per, (P*)partial);
   INQB_CUDA_TRY(cudaGetLastError());
   const long work = 3L * Ma * Mb;
   k_mlwf_slab_sum<P><<<(unsigned)((work + 31) / 32), 256, 0, st>>>((const P*)partial, (int)nslab, work, Z);
@@ -1028,13 +1077,9 @@ int launch_jade_adiag(const double2* a, const double2* u, int M, double2* adiag,
 
 int launch_mlwf_rotate(int precision, const void* psi, long ld, int M, long N, const double2* u, void* out, long ldo,
                        void* stream) {
+  if (precision == INQB_FP64) return launch_rotate_adjoint(psi, ld, M, u, out, ldo, N, stream);
   const dim3 grid((unsigned)((N + kRT - 1) / kRT), (unsigned)((M + kRT - 1) / kRT));
-  if (precision == INQB_FP64)
-    k_mlwf_rotate<double><<<grid, 256, 0, (cudaStream_t)stream>>>((const cplx<double>*)psi, ld, M, N, u,
-                                                                   (cplx<double>*)out, ldo);
-  else
-    k_mlwf_rotate<float><<<grid, 256, 0, (cudaStream_t)stream>>>((const cplx<float>*)psi, ld, M, N, u,
-                                                                  (cplx<float>*)out, ldo);
+  k_mlwf_rotate<<<grid, 256, 0, (cudaStream_t)stream>>>((const cplx<float>*)psi, ld, M, N, u, (cplx<float>*)out, ldo);
   INQB_CUDA_TRY(cudaGetLastError());
   return INQB_OK;
 }

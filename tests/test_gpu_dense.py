@@ -90,3 +90,38 @@ def test_jade_sizes(pb, oracle_mod, M):
     assert sweeps == sw_ref
     assert np.abs(u.cpu().numpy() - u_ref).max() < 1e-10
     assert np.abs(adiag.cpu().numpy() - d_ref).max() < 1e-10
+
+
+@pytest.mark.parametrize("Ma,Mb,n", [(33, 33, 16), (40, 72, 16), (136, 41, 16), (70, 200, 32)])
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-13), ("mixed", 1e-13)])
+def test_wide_tiles_of_ragged_blocks(pb, Ma, Mb, n, precision, tol):
+    """64-wide tiles whose row blocks, column blocks or both end inside the tile, from
+    complex128 and complex64 orbitals; one slab of points to many."""
+    h = _ham(pb, n, precision)
+    a, b = _block(h, Ma, Ma + 1, 1, h.dtype), _block(h, Mb, Mb + 2, 2, h.dtype)
+    wa, wb = a.to(torch.complex128), b.to(torch.complex128)
+    ref = h.volume_element * (wa.conj().T @ wb)
+    assert float((h.overlap_block(a, b) - ref).norm() / ref.norm()) < tol
+    rot = _block(h, Mb, Mb, 3, torch.complex128)[:Ma].contiguous()
+    ref = wa @ rot
+    # complex64 results are rounded once to 6e-8
+    assert float((h.rotate_block(a, rot) - ref).norm() / ref.norm()) < (1e-14 if precision == "fp64" else 1e-7)
+
+
+@pytest.mark.parametrize("Ma,Mb", [(1, 1), (7, 9), (33, 8), (31, 33), (64, 65), (70, 100)])
+def test_gram_and_adjoint_rotation(pb, Ma, Mb):
+    """The weighted Gram matrices and psi u^H of complex128 orbitals at the edges of their
+    64-wide tiles."""
+    h = _ham(pb, 18)
+    a, b = _block(h, Ma, Ma + 1, 1, h.dtype), _block(h, Mb, Mb, 2, h.dtype)
+    i = torch.arange(18, device="cuda", dtype=torch.float64)
+    f = torch.where(i >= 9, i - 18, i) / 18
+    for d, Z in enumerate(h.mlwf_gram_block(a, b)):
+        shape = [1, 1, 1]
+        shape[d] = 18
+        w = torch.exp(2j * np.pi * f).reshape(shape).expand(18, 18, 18).reshape(-1, 1)
+        ref = a.conj().T @ (w * b)
+        assert float((Z - ref).norm() / ref.norm()) < 1e-13
+    u = _block(h, Mb, Mb, 4, torch.complex128)[:Mb].contiguous()
+    ref = b @ u.conj().T
+    assert float((h.mlwf_rotate_(b.clone(), u) - ref).norm() / ref.norm()) < 1e-14
