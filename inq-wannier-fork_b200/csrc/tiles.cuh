@@ -98,6 +98,15 @@ struct TileGeom {
     return sizeof(V) * ((size_t)TILE + NY + NZ) + sizeof(double2) * (size_t)acc_atoms * LMAX * G +
            sizeof(EntRec<T>) * (size_t)rec_cap;
   }
+  // The second pass copies a block of 32 KB or more to shared memory before its first stage
+  // (outer_y_load), the H pass only with at most 8 row classes.
+  // Measured (straight -> staged, us): H pass 64^3 x 128 mixed 144 -> 137, FP64 313 -> 259;
+  // 72^3 mixed 218 -> 211, 128^3 x 64 821 -> 613, FP64 x 16 330 -> 313; 96^3 even; 144^3
+  // (9 classes) 1104 -> 1115, FP64 549 -> 596.  Forward FFT (two passes) 64^3 x 128 232 -> 226,
+  // FP64 517 -> 444; 128^3 x 16 418 -> 384, 663 -> 620; 144^3 554 -> 534, 982 -> 925; below
+  // 32 KB 48^3 x 64 60 -> 62, 60^3 x 37 127 -> 130, 40^3 x 24 FP64 27 -> 29.
+  static constexpr bool FFT_STAGED = sizeof(V) * (size_t)BLK >= 32 * 1024;
+  static constexpr bool H_STAGED = FFT_STAGED && Y1 <= 8;
   static constexpr size_t SMEM_X = sizeof(V) * ((size_t)XBLK + NX) + sizeof(T) * 2 * Y1;
   static constexpr size_t TILE_BYTES = sizeof(V) * (size_t)TILE;
   // CTAs of 256 threads per SM that a pass asks the compiler for: four where the radices
@@ -440,6 +449,35 @@ __device__ __forceinline__ void proj_finish_item(const ProjView<T>& pj, int M, i
 // handles item (t / 32) * 4 + t % 4
 __device__ __forceinline__ long finish_item(long t) { return t / 32 * (32 / kFinParts) + t % (32 / kFinParts); }
 
+// The forward outer y stage y1 -> kb of one block [ix][y1][G] into the x slots.  Straight
+// from HBM a thread loads the Y1 lanes of its (ix, v) column (neighbouring threads read
+// whole runs) and writes it to shared memory once; STAGED copies the block to shared memory
+// first, with more bytes in flight a thread.
+template <typename TG, bool STAGED>
+__device__ __forceinline__ void outer_y_load(typename TG::V* X, const typename TG::V* blk) {
+  using AX = typename TG::AX;
+  constexpr int NX = TG::AX::N, Y1 = TG::Y1, VP = TG::VP, XS = TG::XS;
+  if (STAGED) {
+    for (int q = threadIdx.x; q < NX * Y1 * TG::CH; q += blockDim.x) {
+      const int c = q % TG::CH * TG::LC, r = q / TG::CH;
+      cp_async16(X + AX::slot(r / Y1) * XS + r % Y1 * VP + c, blk + r * VP + c);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+  }
+  for (int it = threadIdx.x; it < NX * VP; it += blockDim.x) {
+    const int v = it % VP, ix = it / VP;
+    const int base = AX::slot(ix) * XS + v;
+    typename TG::V u[Y1];
+#pragma unroll
+    for (int y = 0; y < Y1; ++y) u[y] = STAGED ? X[base + y * VP] : ld_l2(blk + (ix * Y1 + y) * VP + v);
+    DFT<Y1, false, typename TG::P>::run(u);
+#pragma unroll
+    for (int y = 0; y < Y1; ++y) X[base + y * VP] = u[y];
+  }
+}
+
 // ---------------------------------------------------------------- pass B
 // One contiguous block tmp[g][ka][kz] = [ix][y1][G]; in shared memory the x
 // index goes to padded slots of stride XS and (y1, j) stays contiguous.  With
@@ -483,19 +521,7 @@ __device__ __forceinline__ void tile_x_body(int bx, int by, typename TileGeom<T,
                  (kp.b[0][0] * kp.b[0][0] + kp.b[0][1] * kp.b[0][1] + kp.b[0][2] * kp.b[0][2]);
 
   chain_wait();
-  // outer y stage straight from HBM: a thread loads the Y1 lanes of its (ix, v)
-  // column (neighbouring threads read whole 64-byte runs), DFT_Y1 over y1 -> kb, and
-  // writes the column to shared memory once
-  for (int it = threadIdx.x; it < NX * VP; it += blockDim.x) {
-    const int v = it % VP, ix = it / VP;
-    V u[Y1];
-#pragma unroll
-    for (int y = 0; y < Y1; ++y) u[y] = ld_l2(blk + (ix * Y1 + y) * VP + v);
-    DFT<Y1, false, P>::run(u);
-    const int base = AX::slot(ix) * XS + v;
-#pragma unroll
-    for (int y = 0; y < Y1; ++y) X[base + y * VP] = u[y];
-  }
+  outer_y_load<TG, TG::H_STAGED>(X, blk);
   __syncthreads();
 
   auto map1 = [](int it, int& base, int& es, int& j2) {
@@ -602,17 +628,7 @@ __global__ void __launch_bounds__(256, TileGeom<T, NX, NY, NZ>::X_MIN_CTAS)
   chain_wait();
 
   if (DIR == 0) {
-    // outer y stage straight from HBM, as in the H pass: y1 -> kb
-    for (int it = threadIdx.x; it < NX * VP; it += blockDim.x) {
-      const int v = it % VP, ix = it / VP;
-      V u[Y1];
-#pragma unroll
-      for (int y = 0; y < Y1; ++y) u[y] = ld_l2(blk + (ix * Y1 + y) * VP + v);
-      DFT<Y1, false, P>::run(u);
-      const int base = AX::slot(ix) * XS + v;
-#pragma unroll
-      for (int y = 0; y < Y1; ++y) X[base + y * VP] = u[y];
-    }
+    outer_y_load<TG, TG::FFT_STAGED>(X, blk);
     __syncthreads();
     step1<AX, false>(X, Y1 * VP * AX::N2, twx, map1);
     __syncthreads();
