@@ -51,7 +51,8 @@ __device__ __forceinline__ void fma_acc(cplx<T>& acc, cplx<T> a, cplx<T> b) {
 // ---------------------------------------------------------------- lanes
 // The transforms work on lanes, usually of 16 bytes: one complex128 value (cplx<double>), or
 // the complex64 values of two neighbouring orbitals as (re, re | im, im) in two packed FP32
-// pairs (cplx<F2>); long FP32 axes use one complex64 (cplx<float>, TileGeom in tiles.cuh).  Every operation of the transforms is the same for both orbitals, so
+// pairs (cplx<F2>); long FP32 axes use one complex64 (cplx<float>, TileGeom in tiles.cuh).
+// Every operation of the transforms is the same for the orbitals of a lane, so
 // a packed f32x2 instruction (sm_100: add, sub, mul, fma; each half rounded to nearest
 // like the scalar form) does the work of two, and shared memory, HBM and the index
 // arithmetic see one 16-byte access per lane in both precisions.
