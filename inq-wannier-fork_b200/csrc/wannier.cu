@@ -594,10 +594,16 @@ __device__ __forceinline__ double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+// The aligned forms want every lane of the warp at the instruction together, which loops over
+// the lanes' rows and branches on one lane do not leave by themselves.
 __device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
 // All sweeps in one launch of one thread-block cluster whose shared memory holds the six
 // matrices and u.  A rotation step is bound by latency, not by bytes: as a launch of its
@@ -714,7 +720,6 @@ __global__ void __launch_bounds__(GMAX * kJG)
           for (int v = 0; v < 6; ++v) q.red[k][v] = s[v];
         }
       }
-      __syncwarp();
       cluster_arrive();  // this warp has read its rows
       asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(kJG) : "memory");
       if (live && k == 0) {
@@ -768,7 +773,6 @@ __global__ void __launch_bounds__(GMAX * kJG)
           *bid_dst = q0;
         }
       }
-      __syncwarp();
       cluster_arrive();
     }
     cluster_wait();
