@@ -76,14 +76,12 @@ ProjView<T> proj_view(inqb_ctx* ctx) {
   v.seg_ent = t.d_seg_ent.as<int>();
   v.seg_local = t.d_seg_local.as<int>();
   v.plane_ptr = t.d_plane_ptr.as<int>();
-  v.plane_atom = t.d_plane_atom.as<int>();
   v.scale = t.d_scale.as<double>();
   v.proj = ctx->d_projacc.as<double2>();
   v.pc_ptr = t.d_pc_ptr.as<int>();
   v.pc_pt = t.d_pc_pt.as<int>();
-  v.pc_table = t.pc_chunks > 0 ? t.d_pc_table.ptr : nullptr;
+  v.pc_table = t.d_pc_table.ptr;
   v.err = ctx->d_err.as<int>();
-  v.proj_mode = ctx->proj_mode;
   v.slots = ctx->d_slots.as<double2>();
   v.aslot_ptr = t.d_aslot_ptr.as<int>();
   v.aslot = t.d_aslot.as<int>();
@@ -171,8 +169,12 @@ int apply(inqb_ctx* ctx, int mode, const void* in, long ld_in, void* out, long l
     for (int k = 0; k < 3; k++) a.threads[k] = sched->second[1 + k];
   }
   if (a.ysplit <= 0) a.ysplit = ctx->plan->ysplit;
-  // the fused projection's partial sums: one [4][M] slot per (plane, atom, CTA of the plane)
-  if (mode == LaunchArgs::H && ctx->proj.nproj > 0 && ctx->proj_mode == INQB_PROJECTION_FUSED)
+  // the projection runs as its own kernel where that form is chosen and takes this block's
+  // rows; else it is fused into the first pass, with one [4][M] slot of partial sums per
+  // (plane, atom, CTA of the plane)
+  a.project_first = mode == LaunchArgs::H && ctx->proj.pc_chunks > 0 && ctx->proj_mode == INQB_PROJECTION_KERNEL &&
+                    project_supported(ctx->precision, in, ld_in);
+  if (mode == LaunchArgs::H && ctx->proj.nproj > 0 && !a.project_first)
     INQB_TRY(ctx->d_slots.ensure(sizeof(double2) * (size_t)ctx->proj.aslot.size() * a.ysplit * 4 * M));
   if (ctx->timing_on && mode == LaunchArgs::H && !batch_cell && ctx->timing_count < ctx->timing_capacity) {
     for (int i = 0; i < 6; i++) a.events[i] = ctx->timing_events[6 * ctx->timing_count + i];

@@ -132,7 +132,7 @@ struct ProjTables {
   DevBuf d_aslot_ptr, d_aslot;
   DevBuf d_adj_rec, d_atom_pos;     // [nent] AdjRec<T> in atom-major order
   // device copies
-  DevBuf d_seg_ptr, d_seg_atom, d_seg_ent, d_seg_local, d_plane_ptr, d_plane_atom;
+  DevBuf d_seg_ptr, d_seg_atom, d_seg_ent, d_seg_local, d_plane_ptr;
   DevBuf d_ent_relpos;              // [nent][3] float
   DevBuf d_ent_rec;                 // [nent] EntRec<T>, phases filled for each k + A
   // point order inside each tile: pt_pos[e] is the place of entry e, and
@@ -159,7 +159,6 @@ struct ProjView {
   const int* seg_ent;     // [nseg + 1] entry ranges
   const int* seg_local;   // plane-local atom index of a segment
   const int* plane_ptr;   // [NX + 1] atoms of plane ix
-  const int* plane_atom;
   const EntRec<T>* ent_rec;     // segment (atom) order
   const EntRec<T>* ent_rec_rk;  // rank order inside each tile
   const int* rk_ptr;            // [NX * Y1 + 1] ranks of a tile
@@ -171,7 +170,6 @@ struct ProjView {
   const int* pc_pt;
   const void* pc_table;
   int* err;               // device error word (a device-side wait gave up)
-  int proj_mode;          // 0: fused into the first tile pass; 1: projection kernel
   // the fused projection's partial sums: slot (plane_ptr[ix] + local atom) * ysplit + half
   // holds [LMAX][M]; aslot_ptr / aslot list each atom's slots in plane order
   double2* slots;         // null: flush with atomics instead

@@ -193,10 +193,9 @@ int launch_h_impl(const LaunchArgs& a) {
   kp.pois = (T)0;
 
   if (a.mode == LaunchArgs::H) {
-    // the KB projection: its own deterministic kernel (project.cu) where the tables and
-    // the block's alignment allow, else fused into the first tile pass with FP64 atomics
-    const bool sep = pj.nproj > 0 && pj.proj_mode == 1 && pj.pc_table != nullptr &&
-                     project_supported(sizeof(T) == 8 ? INQB_FP64 : INQB_MIXED, a.in, a.ld_in);
+    // the KB projection: its own kernel (project.cu), or fused into the first tile pass with
+    // one partial sum per (plane, atom, CTA of the plane), which the second pass adds
+    const bool sep = a.project_first;
     ProjView<T> pjA = pj;
     if (sep) pjA.nproj = 0;
     // accumulators for as many of a plane's atoms as fit beside the tile
@@ -259,8 +258,6 @@ int launch_h_impl(const LaunchArgs& a) {
     if (sep) {
       INQB_TRY(launch_project(sizeof(T) == 8 ? INQB_FP64 : INQB_MIXED, a.in, a.ld_in, a.M, pj.nproj, pj.L,
                               pj.pc_ptr, pj.pc_pt, pj.pc_table, pj.scale, pj.proj, pj.err, st));
-    } else if (pj.nproj > 0 && pj.slots == nullptr) {
-      INQB_CUDA_TRY(cudaMemsetAsync(pj.proj, 0, sizeof(double2) * (size_t)pj.nproj * pj.L * a.M, st));
     }
     if (a.events[1]) INQB_CUDA_TRY(cudaEventRecord((cudaEvent_t)a.events[1], st));
     if (a.events[2]) INQB_CUDA_TRY(cudaEventRecord((cudaEvent_t)a.events[2], st));

@@ -38,6 +38,8 @@ struct LaunchArgs {
   // H mode: when set (a BatchCellDesc*, batch.h), describe the apply for the
   // persistent batch launch instead of launching it
   void* batch_cell = nullptr;
+  // the projection runs as its own kernel before the passes (else fused into the first)
+  bool project_first = false;
 };
 
 // Candidate values the autotuner tries, beside the compiled default.

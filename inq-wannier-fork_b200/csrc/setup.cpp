@@ -445,7 +445,6 @@ int upload_proj_tables(const inqb_ctx& ctx, ProjTables& t) {
   INQB_TRY(upload(t.d_seg_ent, t.seg_ent));
   INQB_TRY(upload(t.d_seg_local, t.seg_local));
   INQB_TRY(upload(t.d_plane_ptr, t.plane_ptr));
-  INQB_TRY(upload(t.d_plane_atom, t.plane_atom));
   INQB_TRY(upload(t.d_ent_relpos, t.ent_relpos));
   INQB_TRY(upload(t.d_scale, t.scale));
   INQB_TRY(upload(t.d_atom_ptr, t.atom_ptr));

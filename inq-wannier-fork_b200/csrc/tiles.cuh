@@ -212,7 +212,7 @@ __device__ __forceinline__ void tile_fwd_body(int bx, int by, const cplx<T>* __r
     for (int i = threadIdx.x; i < acc_cap * LMAX * G; i += blockDim.x) acc[i] = make_double2(0.0, 0.0);
   chain_wait();
   // slots of the plane's atoms beyond the shared-memory accumulators start at zero
-  if (proj_on && pj.slots) {
+  if (proj_on) {
     const int a0 = pj.plane_ptr[ix], na = pj.plane_ptr[ix + 1] - a0;
     for (int i = threadIdx.x; i < max(0, na - acc_cap) * LMAX * G; i += blockDim.x) {
       const int j = i % G, l = (i / G) % LMAX, sl = acc_cap + i / (G * LMAX);
@@ -310,7 +310,7 @@ __device__ __forceinline__ void tile_fwd_body(int bx, int by, const cplx<T>* __r
               double2& d = acc[(sl * LMAX + l) * G + j];
               d.x += (double)w.x;
               d.y += (double)w.y;
-            } else if (pj.slots) {
+            } else {
               // beyond the shared-memory accumulators: this CTA's own slot in global
               // memory (zeroed at the start), the same ownership
               double2* d = pj.slots + (((long)(pj.plane_ptr[ix] + sl) * YS + yh) * LMAX + l) * M + m0 + j;
@@ -318,12 +318,6 @@ __device__ __forceinline__ void tile_fwd_body(int bx, int by, const cplx<T>* __r
               o.x += (double)w.x;
               o.y += (double)w.y;
               *d = o;
-            } else if (l < pj.L) {
-              const int at = pj.seg_atom[s];
-              const double sc = pj.scale[at * pj.L + l];
-              double2* dst = &pj.proj[((long)at * pj.L + l) * M + m0 + j];
-              atomicAdd(&dst->x, sc * (double)w.x);
-              atomicAdd(&dst->y, sc * (double)w.y);
             }
           }
         }
@@ -370,25 +364,15 @@ __device__ __forceinline__ void tile_fwd_body(int bx, int by, const cplx<T>* __r
     if (y1 + 1 < (yh + 1) * YPER) load_tile(y1 + 1);
   }
 
-  // -- flush the plane accumulators: into this CTA's (plane, half) slots, which the
-  // finish kernel adds per atom in a fixed order; without slots, proj[a][l][m] +=
-  // dV ekb * sum with atomics
+  // -- flush the plane accumulators into this CTA's slots, which the second pass adds per
+  // atom in a fixed order
   if (proj_on) {
     const int a0 = pj.plane_ptr[ix];
     const int na = min(pj.plane_ptr[ix + 1] - a0, acc_cap);
     for (int i = threadIdx.x; i < na * LMAX * G; i += blockDim.x) {
       const int j = i % G, l = (i / G) % LMAX, sl = i / (G * LMAX);
       if (j >= gcount) continue;
-      const double2 v = acc[i];
-      if (pj.slots) {
-        pj.slots[(((long)(a0 + sl) * YS + yh) * LMAX + l) * M + m0 + j] = v;
-      } else if (l < pj.L) {
-        const int at = pj.plane_atom[a0 + sl];
-        const double sc = pj.scale[at * pj.L + l];
-        double2* dst = &pj.proj[((long)at * pj.L + l) * M + m0 + j];
-        atomicAdd(&dst->x, sc * v.x);
-        atomicAdd(&dst->y, sc * v.y);
-      }
+      pj.slots[(((long)(a0 + sl) * YS + yh) * LMAX + l) * M + m0 + j] = acc[i];
     }
   }
 }

@@ -11,7 +11,8 @@ src/hamiltonian/projector_all.hpp:98-216) against the oracle, through the C ABI:
   * both forms are deterministic: two applies agree bit for bit;
   * an odd leading dimension (complex64 rows not 16-byte aligned) takes the fused form
     and is still right;
-  * no device-side wait gave up (inqb_device_status).
+  * no device-side wait gave up (inqb_device_status);
+  * that fused form's partial sums have the room of their own block, whatever ran before.
 """
 import numpy as np
 import pytest
@@ -103,3 +104,20 @@ def test_output_takes_the_input_row_stride(pb, sys70):
     assert out.shape == view.shape and out.stride(0) == view.stride(0)
     with pytest.raises(ValueError):
         h.apply(view, out=torch.empty_like(view.contiguous()))
+
+
+@pytest.mark.parametrize("before", [0, 8])
+def test_kernel_mode_on_odd_rows_has_its_own_partial_sums(pb, oracle_mod, sys70, before):
+    """Kernel mode on complex64 rows of odd length runs the fused form: 37 orbitals after no
+    fused apply, and after one of 8 orbitals."""
+    s = sys70
+    h = make_product(pb, s, "mixed")
+    full = torch.as_tensor(s["psi"]).to("cuda", torch.complex64)
+    if before:
+        h(full[:, :before].contiguous())
+    h.set_projection_mode("kernel")
+    x = full[:, :37].contiguous()
+    out = h(x)
+    assert torch.equal(out, h(x))
+    h.device_status()
+    assert rel_norm(out.cpu().numpy(), make_oracle(oracle_mod, s).apply_h(s["psi"][:, :37])) < TOL["mixed"]
