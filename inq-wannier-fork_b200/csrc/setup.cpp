@@ -72,6 +72,7 @@ int DevBuf::ensure(size_t nbytes) {
   if (nbytes == 0) return INQB_OK;
   cudaError_t e = cudaMalloc(&ptr, nbytes);
   if (e != cudaSuccess) {
+    cudaGetLastError();  // a caller that frees memory and tries again must not meet it at its next launch
     ptr = nullptr;
     bytes = 0;
     return fail(INQB_ERR_NOMEM, std::string("cudaMalloc(") + std::to_string(nbytes) + "): " + cudaGetErrorString(e));
@@ -477,7 +478,8 @@ int upload_proj_tables(const inqb_ctx& ctx, ProjTables& t) {
 
 // The projection kernels' chunk tables, made when that form is chosen (the fused form, the
 // default, does not read them): built from the host tables, uploaded, and room for the
-// coefficient table.
+// coefficient table.  pc_chunks > 0 says that all of it is there, so it is set last: a build
+// that ran out of device memory is made again by the next call.
 int build_proj_chunks(const inqb_ctx& ctx, ProjTables& t) {
   if (t.nproj == 0 || t.pc_chunks > 0) return INQB_OK;
   const int nproj = t.nproj, L = t.L;
@@ -485,8 +487,8 @@ int build_proj_chunks(const inqb_ctx& ctx, ProjTables& t) {
   t.pc_ptr.assign(nproj + 1, 0);
   for (int a = 0; a < nproj; a++)
     t.pc_ptr[a + 1] = t.pc_ptr[a] + (t.atom_ptr[a + 1] - t.atom_ptr[a] + kProjChunk - 1) / kProjChunk;
-  t.pc_chunks = t.pc_ptr[nproj];
-  const size_t pcn = (size_t)t.pc_chunks * kProjChunk;
+  const int chunks = t.pc_ptr[nproj];
+  const size_t pcn = (size_t)chunks * kProjChunk;
   t.pc_pt.assign(pcn, -1);
   t.pc_beta.assign(pcn * 4, 0.0);
   t.pc_relpos.assign(pcn * 3, 0.0f);
@@ -502,7 +504,8 @@ int build_proj_chunks(const inqb_ctx& ctx, ProjTables& t) {
   INQB_TRY(upload(t.d_pc_pt, t.pc_pt));
   INQB_TRY(upload(t.d_pc_beta, t.pc_beta));
   INQB_TRY(upload(t.d_pc_relpos, t.pc_relpos));
-  INQB_TRY(t.d_pc_table.ensure(std::max<size_t>(project_table_bytes(ctx.precision, t.pc_chunks), 16)));
+  INQB_TRY(t.d_pc_table.ensure(std::max<size_t>(project_table_bytes(ctx.precision, chunks), 16)));
+  t.pc_chunks = chunks;
   return INQB_OK;
 }
 
