@@ -107,12 +107,15 @@ int reserve(inqb_ctx* ctx, int M) {
 
 // the projection kernels' coefficients at the current k + A (read in that form only)
 int update_project_table(inqb_ctx* ctx, void* stream) {
-  return launch_project_table(ctx->precision, ctx->proj.pc_chunks, ctx->proj.d_pc_relpos.as<float>(),
-                              ctx->proj.d_pc_beta.as<double>(), ctx->kA_cov, ctx->proj.d_pc_table.ptr, stream);
+  INQB_TRY(launch_project_table(ctx->precision, ctx->proj.pc_chunks, ctx->proj.d_pc_relpos.as<float>(),
+                                ctx->proj.d_pc_beta.as<double>(), ctx->kA_cov, ctx->proj.d_pc_table.ptr, stream));
+  ctx->proj_table_valid = true;
+  return INQB_OK;
 }
 
 int update_phases(inqb_ctx* ctx, void* stream) {
   if (ctx->proj.nproj == 0 || ctx->proj.nent == 0) return INQB_OK;
+  ctx->proj_table_valid = false;
   INQB_TRY(launch_phases(ctx->precision, ctx->proj.nent, ctx->proj.d_ent_relpos.as<float>(), ctx->kA_cov,
                          ctx->proj.d_ent_rec.ptr, ctx->proj.d_ent_rec_rk.ptr, ctx->proj.d_rk_pos.as<int>(),
                          ctx->proj.d_adj_rec.ptr, ctx->proj.d_atom_pos.as<int>(), stream));
@@ -796,10 +799,15 @@ int inqb_set_projection_mode(inqb_ctx* ctx, int mode) {
   if (mode != INQB_PROJECTION_FUSED && mode != INQB_PROJECTION_KERNEL)
     return fail(INQB_ERR_INVALID, "unknown projection mode");
   INQB_GUARD(ctx);
-  if (mode == INQB_PROJECTION_KERNEL && ctx->proj_mode != mode && ctx->proj.nproj > 0) {
+  if (mode == INQB_PROJECTION_KERNEL && ctx->proj_mode != mode && ctx->proj.nent > 0) {
     INQB_TRY(build_proj_chunks(*ctx, ctx->proj));
-    INQB_TRY(update_project_table(ctx, nullptr));
-    INQB_CUDA_TRY(cudaStreamSynchronize(nullptr));
+    // k + A has moved on since the table was filled: no apply of this form may still read it,
+    // on whichever stream it was queued
+    if (!ctx->proj_table_valid) {
+      INQB_CUDA_TRY(cudaDeviceSynchronize());
+      INQB_TRY(update_project_table(ctx, nullptr));
+      INQB_CUDA_TRY(cudaStreamSynchronize(nullptr));
+    }
   }
   ctx->proj_mode = mode;
   return INQB_OK;

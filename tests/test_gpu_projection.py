@@ -121,3 +121,38 @@ def test_kernel_mode_on_odd_rows_has_its_own_partial_sums(pb, oracle_mod, sys70,
     assert torch.equal(out, h(x))
     h.device_status()
     assert rel_norm(out.cpu().numpy(), make_oracle(oracle_mod, s).apply_h(s["psi"][:, :37])) < TOL["mixed"]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_mode_switches_follow_the_vector_potential(pb, oracle_mod, sys70, precision):
+    """Back to kernel mode after k + A changed in fused mode: the coefficient table is that of
+    the new k + A; and an apply of kernel mode still queued on a stream that does not wait for
+    the default one reads the table of its own."""
+    s = sys70
+    h = make_product(pb, s, precision)
+    o = oracle_mod.System(s["lattice"], s["nr"])
+    x = torch.as_tensor(s["psi"]).to("cuda", DT[precision])[:, :8].contiguous()
+    kA = [o.cart_to_cov(np.array(v)) for v in ([0.0, 0.0, 0.0], [0.3, -0.2, 0.1], [-0.2, 0.1, 0.4])]
+    ref = [make_oracle(oracle_mod, s, k).apply_h(s["psi"][:, :8]) for k in kA]
+    for k, r in zip(kA, ref):
+        h.set_projection_mode("fused")
+        h.set_vector_potential_cov(k)
+        h.set_projection_mode("kernel")
+        assert _err(precision, h(x).cpu().numpy(), r) < TOL[precision]
+    side = torch.cuda.Stream()
+    y, scratch = torch.empty_like(x), x.clone()
+    h.set_projection_mode("fused")
+    h.etrs_step_(x.clone(), 0.01, kA[0], kA[2])  # its workspaces: no allocation holds the host up below
+    h.set_projection_mode("kernel")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(200_000_000)  # the host is ahead of the stream by about 0.1 s
+        h.apply(x, y)
+        h.set_projection_mode("fused")
+        h.etrs_step_(scratch, 0.01, kA[0], kA[1])
+        h.set_projection_mode("kernel")
+        z = h(x)
+    torch.cuda.synchronize()
+    h.device_status()
+    assert _err(precision, y.cpu().numpy(), ref[2]) < TOL[precision]
+    assert _err(precision, z.cpu().numpy(), ref[1]) < TOL[precision]
