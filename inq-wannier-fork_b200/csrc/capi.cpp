@@ -57,8 +57,38 @@ struct DeviceGuard {
   DeviceGuard guard_((ctx)->device);     \
   if (guard_.status != INQB_OK) return guard_.status
 
+// The workspace of an application to M orbitals: the Fourier intermediate, then the projections
+// and, for the fused projection (ysplit > 0), one [4][M] slot of partial sums per (plane, atom,
+// CTA of the plane).  One allocation: with three, a context's first call waited for each of
+// them (first batched call on 16 cells of 24^3 to 48^3: 10.2 -> 7.5 ms).
+struct HWork {
+  size_t proj = 0, slots = 0, bytes = 0;  // offsets (0: none) and the whole
+};
+HWork h_work(const inqb_ctx* ctx, int M, int ysplit) {
+  const size_t G = ctx->plan->G, Gt = ctx->plan->G_tile;
+  const size_t padded = std::max((M + G - 1) / G * G, (M + Gt - 1) / Gt * Gt);
+  const auto up = [](size_t n) { return (n + 255) / 256 * 256; };
+  HWork w;
+  w.bytes = padded * (size_t)ctx->N * ctx->elem_bytes();
+  if (ctx->proj.nproj > 0) {
+    w.proj = up(w.bytes);
+    w.bytes = w.proj + sizeof(double2) * (size_t)ctx->proj.nproj * ctx->proj.L * M;
+    if (ysplit > 0 && !ctx->proj.aslot.empty()) {
+      w.slots = up(w.bytes);
+      w.bytes = w.slots + sizeof(double2) * ctx->proj.aslot.size() * ysplit * 4 * M;
+    }
+  }
+  return w;
+}
+
+// CTAs per x-plane of the first pass for M orbitals
+int ysplit_of(const inqb_ctx* ctx, int M) {
+  const auto s = ctx->schedules.find(M);
+  return s != ctx->schedules.end() ? s->second[0] : ctx->plan->ysplit;
+}
+
 template <typename T>
-ProjView<T> proj_view(inqb_ctx* ctx) {
+ProjView<T> proj_view(inqb_ctx* ctx, const HWork& w) {
   ProjView<T> v{};
   const ProjTables& t = ctx->proj;
   v.nproj = t.nproj;
@@ -77,12 +107,12 @@ ProjView<T> proj_view(inqb_ctx* ctx) {
   v.seg_local = t.d_seg_local.as<int>();
   v.plane_ptr = t.d_plane_ptr.as<int>();
   v.scale = t.d_scale.as<double>();
-  v.proj = ctx->d_projacc.as<double2>();
+  v.proj = reinterpret_cast<double2*>(ctx->d_tmp.as<char>() + w.proj);
   v.pc_ptr = t.d_pc_ptr.as<int>();
   v.pc_pt = t.d_pc_pt.as<int>();
   v.pc_table = t.d_pc_table.ptr;
   v.err = ctx->d_err.as<int>();
-  v.slots = ctx->d_slots.as<double2>();
+  v.slots = w.slots > 0 ? reinterpret_cast<double2*>(ctx->d_tmp.as<char>() + w.slots) : nullptr;
   v.aslot_ptr = t.d_aslot_ptr.as<int>();
   v.aslot = t.d_aslot.as<int>();
   return v;
@@ -98,11 +128,7 @@ int check_block(const inqb_ctx* ctx, const void* a, int M, long ld) {
 }
 
 int reserve(inqb_ctx* ctx, int M) {
-  const int G = ctx->plan->G, Gt = ctx->plan->G_tile;
-  const size_t padded = std::max((size_t)(M + G - 1) / G * G, (size_t)(M + Gt - 1) / Gt * Gt);
-  INQB_TRY(ctx->d_tmp.ensure(padded * (size_t)ctx->N * ctx->elem_bytes()));
-  if (ctx->proj.nproj > 0) INQB_TRY(ctx->d_projacc.ensure(sizeof(double2) * (size_t)ctx->proj.nproj * ctx->proj.L * M));
-  return INQB_OK;
+  return ctx->d_tmp.ensure(h_work(ctx, M, ctx->proj_mode == INQB_PROJECTION_FUSED ? ysplit_of(ctx, M) : 0).bytes);
 }
 
 // the projection kernels' coefficients at the current k + A (read in that form only)
@@ -136,7 +162,6 @@ int set_kA(inqb_ctx* ctx, const double kA[3], void* stream) {
 int apply(inqb_ctx* ctx, int mode, const void* in, long ld_in, void* out, long ld_out, int M, const void* base,
           long ld_base, const double alpha[2], const double beta[2], void* stream, void* fourier_out = nullptr,
           BatchCellDesc* batch_cell = nullptr, const void* minus = nullptr, long ld_minus = 0) {
-  INQB_TRY(reserve(ctx, M));
   if (!ctx->proj_phases_valid) {
     INQB_TRY(update_phases(ctx, stream));
     ctx->proj_phases_valid = true;
@@ -148,7 +173,6 @@ int apply(inqb_ctx* ctx, int mode, const void* in, long ld_in, void* out, long l
   a.out = out;
   a.ld_out = ld_out;
   a.M = M;
-  a.tmp = ctx->d_tmp.ptr;
   a.tw = ctx->d_tw.ptr;
   a.V = ctx->d_V.ptr;
   a.base = base;
@@ -167,18 +191,16 @@ int apply(inqb_ctx* ctx, int mode, const void* in, long ld_in, void* out, long l
     for (int j = 0; j < 3; j++) a.rlat[i][j] = ctx->cell.rlat[i][j];
   ctx->cell.cov_to_cart(ctx->kA_cov, a.kA_cart);
   const auto sched = ctx->schedules.find(M);
-  if (sched != ctx->schedules.end()) {
-    a.ysplit = sched->second[0];
+  if (sched != ctx->schedules.end())
     for (int k = 0; k < 3; k++) a.threads[k] = sched->second[1 + k];
-  }
-  if (a.ysplit <= 0) a.ysplit = ctx->plan->ysplit;
+  a.ysplit = ysplit_of(ctx, M);
   // the projection runs as its own kernel where that form is chosen and takes this block's
-  // rows; else it is fused into the first pass, with one [4][M] slot of partial sums per
-  // (plane, atom, CTA of the plane)
+  // rows; else it is fused into the first pass
   a.project_first = mode == LaunchArgs::H && ctx->proj.pc_chunks > 0 && ctx->proj_mode == INQB_PROJECTION_KERNEL &&
                     project_supported(ctx->precision, in, ld_in);
-  if (mode == LaunchArgs::H && ctx->proj.nproj > 0 && !a.project_first)
-    INQB_TRY(ctx->d_slots.ensure(sizeof(double2) * (size_t)ctx->proj.aslot.size() * a.ysplit * 4 * M));
+  const HWork w = h_work(ctx, M, mode == LaunchArgs::H && !a.project_first ? a.ysplit : 0);
+  INQB_TRY(ctx->d_tmp.ensure(w.bytes));
+  a.tmp = ctx->d_tmp.ptr;
   if (ctx->timing_on && mode == LaunchArgs::H && !batch_cell && ctx->timing_count < ctx->timing_capacity) {
     for (int i = 0; i < 6; i++) a.events[i] = ctx->timing_events[6 * ctx->timing_count + i];
     ctx->timing_count++;
@@ -186,10 +208,10 @@ int apply(inqb_ctx* ctx, int mode, const void* in, long ld_in, void* out, long l
   ProjView<double> v64;
   ProjView<float> v32;
   if (ctx->precision == INQB_FP64) {
-    v64 = proj_view<double>(ctx);
+    v64 = proj_view<double>(ctx, w);
     a.proj_view = &v64;
   } else {
-    v32 = proj_view<float>(ctx);
+    v32 = proj_view<float>(ctx, w);
     a.proj_view = &v32;
   }
   return ctx->plan->launch(a);
@@ -2024,7 +2046,7 @@ int inqb_autotune(inqb_ctx* ctx, int M, void* stream, int schedule[4]) {
   INQB_CHECK_CTX(ctx);
   if (M <= 0) return fail(INQB_ERR_INVALID, "M must be positive");
   INQB_GUARD(ctx);
-  INQB_TRY(reserve(ctx, M));
+  INQB_TRY(ctx->d_tmp.ensure(h_work(ctx, M, ctx->plan->y1).bytes));  // the largest of the candidates
   // the timings do not depend on the values: zeroed blocks
   DevBuf in, out;
   const size_t bytes = (size_t)ctx->N * M * ctx->elem_bytes();

@@ -209,8 +209,8 @@ struct inqb_ctx {
   inqb::ProjTables proj;
 
   // workspace (grown on demand)
-  inqb::DevBuf d_tmp;     // Fourier-space intermediate, [groups][N][G]
-  inqb::DevBuf d_projacc; // projection accumulators
+  inqb::DevBuf d_tmp;     // H applications: Fourier intermediate [groups][N][G], projections,
+                          // the fused projection's partial sums
   inqb::DevBuf d_work;    // one orbital block for propagators
   inqb::DevBuf d_work2;
   inqb::DevBuf d_red;     // small reduction buffers
@@ -230,7 +230,6 @@ struct inqb_ctx {
                                 // density [N], partial sums, sums
   inqb::DevBuf d_err;           // one int: set by a kernel whose bounded device-side wait gave up
   int proj_mode = 0;            // INQB_PROJECTION_FUSED (0) or INQB_PROJECTION_KERNEL (1)
-  inqb::DevBuf d_slots;         // the fused projection's per-(plane, half) partial sums
   inqb::DevBuf d_mix;           // Crank-Nicolson with self-consistency: Broyden ring df, dv [4][N],
                                 // f_old, vin_old, the new density [N], partial sums, dot products
   size_t elem_bytes() const { return precision == INQB_FP64 ? 16 : 8; }
