@@ -898,7 +898,13 @@ int inqb_ctx_reserve(inqb_ctx* ctx, int M) {
   INQB_CHECK_CTX(ctx);
   INQB_GUARD(ctx);
   if (M <= 0) return fail(INQB_ERR_INVALID, "M must be positive");
-  INQB_TRY(reserve(ctx, M));
+  // the partial sums too, of whichever count up to M runs the most CTAs per plane, and of the
+  // complex64 blocks that kernel mode leaves to the fused projection
+  int ysplit = ctx->plan->ysplit;
+  for (const auto& s : ctx->schedules)
+    if (s.first <= M) ysplit = std::max(ysplit, s.second[0]);
+  const bool fused = ctx->proj_mode == INQB_PROJECTION_FUSED || ctx->precision == INQB_MIXED;
+  INQB_TRY(ctx->d_tmp.ensure(h_work(ctx, M, fused ? ysplit : 0).bytes));
   INQB_TRY(ctx->d_work.ensure((size_t)ctx->N * M * ctx->elem_bytes()));
   return INQB_OK;
 }

@@ -156,3 +156,26 @@ def test_mode_switches_follow_the_vector_potential(pb, oracle_mod, sys70, precis
     h.device_status()
     assert _err(precision, y.cpu().numpy(), ref[2]) < TOL[precision]
     assert _err(precision, z.cpu().numpy(), ref[1]) < TOL[precision]
+
+
+@pytest.mark.parametrize("mode", ["fused", "kernel"])
+def test_reserve_covers_the_projection(pb, mode):
+    """After reserve(M), applies of M' <= M orbitals allocate nothing: the partial sums (10 MB
+    and more here) of smaller counts whose schedule has more CTAs per plane, and of odd
+    complex64 rows in kernel mode."""
+    M = 63
+    s = small_system(pb, n=32, M=M, seed=5, reps=2)
+    h = make_product(pb, s, "mixed")
+    h.set_projection_mode(mode)
+    h.set_schedule(M, (1, 256, 256, 256))
+    x = torch.as_tensor(s["psi"]).to("cuda", torch.complex64)
+    blocks = [x[:, :m].contiguous() for m in (M - 2, M - 1, M)]
+    outs = [torch.empty_like(b) for b in blocks]
+    h.reserve(M)
+    h.apply(blocks[0][:, :2].contiguous())  # the kernels are loaded
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    for b, o in zip(blocks, outs):
+        h.apply(b, o)
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] == free
