@@ -134,7 +134,9 @@ int inqb_fft_backward(inqb_ctx* ctx, const void* in, void* out, int M, int ld, v
  * counterpart (it batches ks_hamiltonian::operator(), ks_hamiltonian.hpp:132-152).
  * The first call with a given set of pointers and sizes captures and instantiates
  * the graph (it also runs each cell once, uncaptured, to set up workspace); later
- * calls with the same arguments only launch it.  The contexts must outlive the
+ * calls with the same arguments only launch it, as long as no cell's k + A, projectors,
+ * mask, projection form, schedule or workspace changed (the call then captures again; a
+ * potential set in place is followed as it is).  The contexts must outlive the
  * batch and must not be used concurrently with it. */
 typedef struct inqb_batch inqb_batch;
 int inqb_batch_create(inqb_ctx* const* cells, int ncells, inqb_batch** out);

@@ -152,6 +152,7 @@ int set_kA(inqb_ctx* ctx, const double kA[3], void* stream) {
   bool same = true;
   for (int d = 0; d < 3; d++) same = same && (ctx->kA_cov[d] == kA[d]);
   for (int d = 0; d < 3; d++) ctx->kA_cov[d] = kA[d];
+  if (!same) ctx->launch_version++;
   if (same && ctx->proj_phases_valid) return INQB_OK;
   INQB_TRY(update_phases(ctx, stream));
   ctx->proj_phases_valid = true;
@@ -552,10 +553,13 @@ struct inqb_batch {
   std::vector<cudaEvent_t> events;    // [0] fork, [1..n] joins
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  // arguments the instantiated graph or the persistent plan was built with
+  // what the instantiated graph or the persistent plan was built with: the arguments, and each
+  // cell's state and workspace
   std::vector<const void*> psis;
   std::vector<void*> hpsis;
   std::vector<int> Ms, lds;
+  std::vector<unsigned long> versions;
+  std::vector<const void*> works;
   // the persistent launch (batch.h)
   int mode = INQB_BATCH_AUTO;
   int tuned = INQB_BATCH_GRAPH;  // the form AUTO runs: GRAPH until inqb_batch_autotune picks
@@ -832,6 +836,7 @@ int inqb_set_projection_mode(inqb_ctx* ctx, int mode) {
     }
   }
   ctx->proj_mode = mode;
+  ctx->launch_version++;
   return INQB_OK;
 }
 
@@ -948,6 +953,7 @@ int inqb_set_vector_potential(inqb_ctx* ctx, const double kA_cov[3]) {
 int inqb_set_fourier_sphere_mask(inqb_ctx* ctx, int enable) {
   INQB_CHECK_CTX(ctx);
   ctx->fourier_mask = enable ? 1 : 0;
+  ctx->launch_version++;
   return INQB_OK;
 }
 
@@ -996,6 +1002,7 @@ int inqb_set_projectors(inqb_ctx* ctx, int nproj, int L, int smax, const int* co
   }
   INQB_CUDA_TRY(cudaDeviceSynchronize());
   ctx->proj = std::move(fresh);
+  ctx->launch_version++;
   {
     auto& src = ctx->proj_src;
     src.nproj = nproj;
@@ -1639,7 +1646,8 @@ int inqb_batch_apply_h(inqb_batch* b, const void* const* psis, void* const* hpsi
   if (guard.status != INQB_OK) return guard.status;
   bool same = b->ready;
   for (int i = 0; i < n && same; i++)
-    same = b->psis[i] == psis[i] && b->hpsis[i] == hpsis[i] && b->Ms[i] == Ms[i] && b->lds[i] == lds[i];
+    same = b->psis[i] == psis[i] && b->hpsis[i] == hpsis[i] && b->Ms[i] == Ms[i] && b->lds[i] == lds[i] &&
+           b->versions[i] == b->cells[i]->launch_version && b->works[i] == b->cells[i]->d_tmp.ptr;
   if (!same) {
     b->ready = false;
     b->persistent = false;
@@ -1669,6 +1677,12 @@ int inqb_batch_apply_h(inqb_batch* b, const void* const* psis, void* const* hpsi
     b->hpsis.assign(hpsis, hpsis + n);
     b->Ms.assign(Ms, Ms + n);
     b->lds.assign(lds, lds + n);
+    b->versions.clear();
+    b->works.clear();
+    for (const inqb_ctx* c : b->cells) {
+      b->versions.push_back(c->launch_version);
+      b->works.push_back(c->d_tmp.ptr);
+    }
     b->ready = true;
   }
   if (b->persistent)
@@ -2035,6 +2049,7 @@ int inqb_set_schedule(inqb_ctx* ctx, int M, const int schedule[4]) {
   if (M <= 0) return fail(INQB_ERR_INVALID, "M must be positive");
   if (!schedule) {
     ctx->schedules.erase(M);
+    ctx->launch_version++;
     return INQB_OK;
   }
   if (schedule[0] < 1 || ctx->plan->y1 % schedule[0] != 0)
@@ -2045,6 +2060,7 @@ int inqb_set_schedule(inqb_ctx* ctx, int M, const int schedule[4]) {
       return fail(INQB_ERR_INVALID, "schedule: threads per CTA must be a multiple of 32 in [64, 256]");
   }
   ctx->schedules[M] = {schedule[0], schedule[1], schedule[2], schedule[3]};
+  ctx->launch_version++;
   return INQB_OK;
 }
 
@@ -2113,6 +2129,7 @@ int inqb_autotune(inqb_ctx* ctx, int M, void* stream, int schedule[4]) {
     }
   for (auto& e : ev) cudaEventDestroy(e);
   ctx->timing_on = saved_timing;
+  ctx->launch_version++;
   if (status != INQB_OK) {
     ctx->schedules.erase(M);
     return status;

@@ -137,3 +137,33 @@ def test_unreachable_wait_times_out(pb):
     batch.status()
     for s, o in zip(single, outs):
         assert _rel(o, s) < 1e-6
+
+
+@pytest.mark.parametrize("mode", ["graph", "persistent"])
+def test_batch_follows_its_cells(pb, mode):
+    """The same blocks again after a cell's k + A, mask, projectors, schedule, potential or (an
+    apply of more orbitals) workspace changed: the batch gives each cell's own H psi."""
+    from pinq_b200 import systems
+
+    rng = np.random.default_rng(3)
+    cells = []
+    for n, M in ((24, 16), (32, 8)):
+        a = n * systems.SPACING
+        cells.append(_make(pb, "fp64", systems.cubic(a), (n, n, n), rng.uniform(0, a, (4, 3)), M, n))
+    h, x = cells[1]
+    lattice, nr = systems.cubic(32 * systems.SPACING), (32, 32, 32)
+    moved = rng.uniform(0, 32 * systems.SPACING, (6, 3))
+    changes = [lambda: h.set_vector_potential_cov([0.3, -0.1, 0.2]), lambda: h.set_fourier_sphere_mask(True),
+               lambda: h.set_gaussian_projectors(moved), lambda: h.set_schedule(8, (1, 128, 128, 128)),
+               lambda: h.set_scalar_potential(systems.gaussian_potential(lattice, nr, moved)),
+               lambda: h(x.repeat(1, 5)), lambda: h.etrs_step_(x.clone(), 0.01, [0.0, 0.0, 0.0], [0.1, 0.0, 0.0])]
+    batch = pb.CellBatch([c for c, _ in cells], mode=mode)
+    psis, outs = [p for _, p in cells], [torch.empty_like(p) for _, p in cells]
+    batch.apply(psis, outs)
+    for k, change in enumerate(changes):
+        change()
+        batch.apply(psis, outs)
+        batch.status()
+        assert batch.info()["form"] == mode
+        for (c, p), o in zip(cells, outs):
+            assert _rel(o, c(p)) < 1e-13, k
