@@ -1658,9 +1658,16 @@ int inqb_batch_apply_h(inqb_batch* b, const void* const* psis, void* const* hpsi
         INQB_TRY(update_phases(b->cells[i], nullptr));
         b->cells[i]->proj_phases_valid = true;
       }
+      // into scratch where the call is in place: the recorded launch below applies H too
       const double one[2] = {1.0, 0.0}, zero[2] = {0.0, 0.0};
-      INQB_TRY(apply(b->cells[i], LaunchArgs::H, psis[i], lds[i], hpsis[i], lds[i], Ms[i], nullptr, 0, one, zero,
-                     nullptr));
+      void* out = hpsis[i];
+      long ld_out = lds[i];
+      if (hpsis[i] == psis[i]) {
+        INQB_TRY(b->cells[i]->d_work.ensure((size_t)b->cells[i]->N * Ms[i] * b->cells[i]->elem_bytes()));
+        out = b->cells[i]->d_work.ptr;
+        ld_out = Ms[i];
+      }
+      INQB_TRY(apply(b->cells[i], LaunchArgs::H, psis[i], lds[i], out, ld_out, Ms[i], nullptr, 0, one, zero, nullptr));
     }
     INQB_CUDA_TRY(cudaDeviceSynchronize());
     batch_release_graph(b);

@@ -167,3 +167,23 @@ def test_batch_follows_its_cells(pb, mode):
         assert batch.info()["form"] == mode
         for (c, p), o in zip(cells, outs):
             assert _rel(o, c(p)) < 1e-13, k
+
+
+@pytest.mark.parametrize("mode", ["graph", "persistent"])
+def test_batch_in_place(pb, mode):
+    """Output blocks that are the input blocks: H once, in the first call too."""
+    from pinq_b200 import systems
+
+    rng = np.random.default_rng(4)
+    cells = []
+    for n, M in ((24, 9), (32, 8)):
+        a = n * systems.SPACING
+        cells.append(_make(pb, "fp64", systems.cubic(a), (n, n, n), rng.uniform(0, a, (4, 3)), M, n))
+    batch = pb.CellBatch([h for h, _ in cells], mode=mode)
+    blocks, ref = [x.clone() for _, x in cells], [x for _, x in cells]
+    for _ in range(2):
+        batch.apply(blocks, blocks)
+        batch.status()
+        ref = [h(x) for (h, _), x in zip(cells, ref)]
+        for a, b in zip(blocks, ref):
+            assert _rel(a, b) < 1e-13
