@@ -487,16 +487,21 @@ __global__ void k_jade_change(const double* __restrict__ delta, int nsteps, int 
 // jacobi3_top with its iteration in FP32 and the eigenvector then refined in FP64.  The
 // serial chain of FP64 roots and divisions made the Jacobi iteration the longest part of a
 // rotation step (5100 of 13200 cycles at 64 states).  The FP32 iteration makes the same
-// rotations, so it leaves the eigenvector in the same column with the same sign; three
-// steps of v += sum_i v_i (v_i . A v + lambda v_i . (v0 - v)) / (lambda - lambda_i) (the
-// column form of Ogita and Aishima's refinement, Japan J. Indust. Appl. Math. 35, 2018)
-// square its error each: 1e-4 -> 1e-8 -> 1e-16.  Where FP32 could choose differently (a
-// rotation near 45 degrees that involves a large eigenvalue) or the top eigenvalue is not
-// well separated, the FP64 iteration runs instead.
+// rotations, so it leaves the eigenvector in the same column with the same sign; then
+// v += sum_i v_i (v_i . (A - lambda) v) / (lambda - lambda_i) + v (1 - |v|^2) / 2, three times
+// (the column form of Ogita and Aishima's refinement, Japan J. Indust. Appl. Math. 35, 2018).
+// v_1, v_2 and the gaps keep their FP32 errors, up to 1e-5 with gaps of 2% and more, so a step
+// leaves about 1e-5 of v's error: 1e-5 -> 1e-10 -> 1e-15 -> rounding.  The last residual
+// subtracts lambda from the diagonal first, where the difference is exact for a close
+// eigenvalue; A v - lambda v rounds at |A| and ended 1.7 times as far off as the FP64
+// iteration at gaps of 2 to 4%, this form is nearer than that iteration at every gap.
+// Where FP32 could choose differently (a rotation near 45 degrees that involves a large
+// eigenvalue) or the top eigenvalue is not well separated, the FP64 iteration runs instead.
 __device__ void top3(const double G[3][3], double out[3]) {
   const double scale = fmax(G[0][0], fmax(G[1][1], G[2][2]));
   bool ok = scale > 0.0 && scale < 1e300;
-  const double inv = ok ? 1.0 / scale : 0.0;
+  // a power of two, so that A is G to the last bit (1 / scale rounded every entry)
+  const double inv = ok ? __longlong_as_double((2046LL - (__double_as_longlong(scale) >> 52)) << 52) : 0.0;
   double A[3][3];
 #pragma unroll
   for (int i = 0; i < 3; ++i)
@@ -575,7 +580,11 @@ __device__ void top3(const double G[3][3], double out[3]) {
     double e1 = 0.0, e2 = 0.0;
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-      const double res = fma(-lam, v[j], w[j]);
+      double res = fma(-lam, v[j], w[j]);
+      if (it == 2) {
+        const int p = (j + 1) % 3, q = (j + 2) % 3;
+        res = fma(A[j][j] - lam, v[j], fma(A[j][p], v[p], A[j][q] * v[q]));
+      }
       e1 = fma(v1[j], res, e1);
       e2 = fma(v2[j], res, e2);
     }
