@@ -751,11 +751,11 @@ __global__ void __launch_bounds__(GMAX * kJG)
         double v[3];
         top3(G, v);
         const double x = fabs(v[0]), y = v[0] < 0.0 ? -v[1] : v[1];
-        const double r = sqrt((x + 1.0) / 2.0), ir = 0.5 / r;
+        const double r = sqrt((x + 1.0) / 2.0);
         if (lane == 0) {
           q.rot[0] = r;
-          q.rot[1] = y * ir;
-          q.rot[2] = -v[2] * ir;
+          q.rot[1] = y / (2.0 * r);
+          q.rot[2] = -v[2] / (2.0 * r);
         }
       }
       __syncwarp();
