@@ -58,7 +58,7 @@ __global__ void k_lincomb(long N, int M, LinTerms<T> t, cplx<T>* __restrict__ y,
 // The same sums on blocks without padding (every ld = M, 16-byte aligned): one run of n
 // 16-byte pieces, so no row index is formed (its 64-bit division costs more than the sums
 // do: 32^3 x 16 orbitals, five terms, FP32) and the K loads of a piece go out together.
-// K is compiled in.
+// K is compiled in: 1 (a copy) and 5 (the Taylor sums) are the counts in use.
 template <typename T, int K>
 __global__ void __launch_bounds__(256) k_lincomb_flat(long n, LinTerms<T> t, cplx<T>* y) {
   constexpr int PV = 16 / (int)sizeof(cplx<T>);
@@ -782,17 +782,16 @@ static int lincomb_impl(long N, int M, int K, const double (*a)[2], const void* 
     t.a[k] = mk<T>((T)a[k][0], (T)a[k][1]);
   }
   constexpr int PV = 16 / (int)sizeof(cplx<T>);
-  bool flat = ldy == M && (uintptr_t)y % 16 == 0 && N * M % PV == 0;
+  bool flat = (K == 1 || K == 5) && ldy == M && (uintptr_t)y % 16 == 0 && N * M % PV == 0;
   for (int k = 0; k < K; k++) flat = flat && ldx[k] == M && (uintptr_t)x[k] % 16 == 0;
   if (flat) {
     const long n = N * M / PV;
     const int nb = grid_for(n, 256);
     cplx<T>* yt = (cplx<T>*)y;
-    if (K == 1) k_lincomb_flat<T, 1><<<nb, 256, 0, st>>>(n, t, yt);
-    if (K == 2) k_lincomb_flat<T, 2><<<nb, 256, 0, st>>>(n, t, yt);
-    if (K == 3) k_lincomb_flat<T, 3><<<nb, 256, 0, st>>>(n, t, yt);
-    if (K == 4) k_lincomb_flat<T, 4><<<nb, 256, 0, st>>>(n, t, yt);
-    if (K == 5) k_lincomb_flat<T, 5><<<nb, 256, 0, st>>>(n, t, yt);
+    if (K == 1)
+      k_lincomb_flat<T, 1><<<nb, 256, 0, st>>>(n, t, yt);
+    else
+      k_lincomb_flat<T, 5><<<nb, 256, 0, st>>>(n, t, yt);
   } else {
     k_lincomb<T><<<grid_for(N * M, 256), 256, 0, st>>>(N, M, t, (cplx<T>*)y, ldy);
   }
