@@ -625,7 +625,7 @@ __device__ __forceinline__ void cluster_wait() {
 // overwritten (arrived at after the reads, waited for after the eigenproblem), and all are
 // written before the next step reads.  Seven warps a slot: warp k sums and rotates matrix
 // k (warp 6: u); E elements of a row per lane (M <= 32 E); GMAX slots per CTA at most.
-constexpr int kJG = 7 * 32;
+constexpr int kJG = 7 * 32, kJadeCtas = 16;
 
 struct JadeShared {
   double red[6][6];   // warp k: Re, Im of the pair elements (pq, pp, qq) of matrix k
@@ -1031,41 +1031,34 @@ int launch_jade_step(double2* a, double2* u, int M, const int2* pairs, int np, d
 template <int E, int GMAX>
 static int jade_cluster_launch(double2* a, double2* u, int M, const int2* pairs, int np, int steps, int maxsweep,
                                double tol, double* delta, double* out, bool* done, cudaStream_t st) {
-  // sixteen CTAs (fewer slots each) where the GPU places such a cluster, else eight
-  for (const int cl : {16, 8}) {
-    const int slots = (np + cl - 1) / cl;
-    const size_t smem = (size_t)slots * 2 * 7 * M * sizeof(double2);
-    if (slots > GMAX || smem > 200 * 1024) continue;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(cl);
-    cfg.blockDim = dim3(slots * kJG);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cl;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    INQB_CUDA_TRY(cudaFuncSetAttribute(k_jade_cluster<E, GMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       200 * 1024));
-    if (cl > 8)
-      INQB_CUDA_TRY(cudaFuncSetAttribute(k_jade_cluster<E, GMAX>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    int fit = 0;
-    if (cudaOccupancyMaxActiveClusters(&fit, k_jade_cluster<E, GMAX>, &cfg) != cudaSuccess || fit < 1) {
-      cudaGetLastError();
-      continue;
-    }
-    INQB_CUDA_TRY(
-        cudaLaunchKernelEx(&cfg, k_jade_cluster<E, GMAX>, a, u, M, pairs, np, steps, maxsweep, tol, delta, out));
-    *done = true;
+  const int slots = (np + kJadeCtas - 1) / kJadeCtas;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kJadeCtas);
+  cfg.blockDim = dim3(slots * kJG);
+  cfg.dynamicSmemBytes = (size_t)slots * 2 * 7 * M * sizeof(double2);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kJadeCtas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  INQB_CUDA_TRY(cudaFuncSetAttribute(k_jade_cluster<E, GMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     GMAX * 2 * 7 * 32 * E * (int)sizeof(double2)));
+  INQB_CUDA_TRY(cudaFuncSetAttribute(k_jade_cluster<E, GMAX>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  int fit = 0;
+  if (cudaOccupancyMaxActiveClusters(&fit, k_jade_cluster<E, GMAX>, &cfg) != cudaSuccess || fit < 1) {
+    cudaGetLastError();  // no place for such a cluster: the step launches
     return INQB_OK;
   }
+  INQB_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_jade_cluster<E, GMAX>, a, u, M, pairs, np, steps, maxsweep, tol, delta, out));
+  *done = true;
   return INQB_OK;
 }
 
-// All sweeps in one launch (a and u on the device; u is set, not read); done: whether the
-// matrices fit a cluster.  out[0], out[1]: the last sweep's trace change, the sweeps.
+// All sweeps in one launch (a and u on the device; u is set, not read).  done: whether they ran
+// so, which takes at most 128 states and a GPU that places a cluster of 16 CTAs.  out[0], out[1]:
+// the last sweep's trace change, the sweeps.
 int launch_jade_cluster(double2* a, double2* u, int M, const int2* pairs, int np, int steps, int maxsweep, double tol,
                         double* delta, double* out, bool* done, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
