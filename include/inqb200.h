@@ -201,7 +201,8 @@ int inqb_dipole(inqb_ctx* ctx, const double* rho, double out[3], void* stream);
 int inqb_band_energies(inqb_ctx* ctx, const void* psi, const void* hpsi, int M, int ld, double* eps,
                        void* stream);
 /* operations::orthogonalize (src/operations/orthogonalize.hpp:25-32): FP64
- * overlap S = dV psi^H psi, Cholesky S = U^H U, psi <- psi U^-1; synchronous. */
+ * overlap S = dV psi^H psi, Cholesky S = U^H U, psi <- psi U^-1; synchronous.  The M x M
+ * scratch (32 M^2 bytes) grows with M and is kept in the context. */
 int inqb_orthonormalize(inqb_ctx* ctx, void* psi, int M, int ld, void* stream);
 /* Orbital-sharded orthonormalisation, the pieces of operations::orthogonalize when
  * the states are split over ranks (src/operations/orthogonalize.hpp:25-32).  Each rank
@@ -227,9 +228,10 @@ int inqb_cholesky_inverse(inqb_ctx* ctx, double* S, int M, int lds, void* stream
 int inqb_rotate_block(inqb_ctx* ctx, const void* a, int Ma, int lda, const double* R, int ldr, int Mo, void* out,
                       int ldo, void* stream);
 /* The same orthonormalisation without any device allocation (no counterpart in the
- * reference).  inqb_orthonormalize allocates its M x M scratch on every call; this
- * one uses a fixed array of 2 MiB compiled into the library, which every GPU that
- * loads the library holds until the process exits.  It is for callers that may not
+ * reference).  inqb_orthonormalize allocates its M x M scratch where M is larger than
+ * in any earlier call of the context; this one uses a fixed array of 2 MiB compiled
+ * into the library, which every GPU that loads the library holds until the process
+ * exits.  It is for callers that may not
  * call cudaMalloc: code running inside another framework's memory pool or allocator
  * hooks, or a service whose device memory budget is fixed after start-up.
  *   - M <= 256 orbitals; larger M returns INQB_ERR_UNSUPPORTED.
@@ -471,15 +473,18 @@ int inqb_timing_passes(inqb_ctx* ctx, double ms[4], int* napplies);
  * (src/hamiltonian/projector_all.hpp:98-216).  Both are deterministic: every partial
  * sum has one owner and the partials are added in a fixed order.
  *   INQB_PROJECTION_FUSED (default): summed inside the first tile pass while the tile
- *     is in shared memory (FP32 products, FP64 sums), one partial per (x-plane, half
- *     of its row classes, atom), added per atom by a small finish kernel.
+ *     is in shared memory (mixed: FP32 products and sums within an atom's entries of
+ *     one tile, FP64 sums beyond), one partial per (x-plane, CTA of the plane, atom),
+ *     added per atom by the second pass.
  *   INQB_PROJECTION_KERNEL: a kernel of its own before the tile passes, one CTA per
  *     (atom, block of orbitals) that gathers the orbitals at the atom's sphere points.
  *     In the mixed precision it is a tcgen05 tensor-core contraction (TF32 with a
  *     split-precision correction, FP64 sums per chunk of 32 points); in FP64 it runs
  *     on the CUDA cores.  It reads the sphere points' orbitals once more from memory,
  *     and measures slower than the fused form; orbital blocks whose complex64 rows are
- *     not 16-byte aligned (odd ld) take the fused form. */
+ *     not 16-byte aligned (odd ld) take the fused form.  Choosing it the first time
+ *     after inqb_set_projectors makes its tables (device allocations), and choosing it
+ *     after k + A changed synchronises the device and refills them. */
 enum inqb_projection_mode { INQB_PROJECTION_FUSED = 0, INQB_PROJECTION_KERNEL = 1 };
 int inqb_set_projection_mode(inqb_ctx* ctx, int mode);
 /* Kernels with a bounded device-side wait record a failed wait in a device word of

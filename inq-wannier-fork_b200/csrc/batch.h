@@ -2,7 +2,7 @@
 // stage, CTA coordinates) that CTAs take from a device ticket counter.
 //
 // Stages per (cell, orbital group g), a "unit":
-//   A       first tile pass, the (g, x-plane, half) CTAs                 -> signals cA[u]
+//   A       first tile pass, the (g, x-plane, share) CTAs                -> signals cA[u]
 //   finish  the fused projection's fixed-order finish for group g        waits cA, signals cB
 //   B       second tile pass, the (ka, kz) CTAs of group g                 waits cA, signals cB
 //   C       third tile pass, the (g, tile) CTAs                           waits cB

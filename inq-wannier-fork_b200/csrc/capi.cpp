@@ -480,9 +480,9 @@ std::vector<int2> jade_schedule(int np) {
   return sched;
 }
 
-// jade_complex on device arrays a [6][M][M] (rotated in place), u, adiag.  Where a cluster's
-// shared memory holds the matrices, all sweeps run in one launch; else one graph of
-// per-step launches a sweep, the sweep's trace change read back after each.
+// jade_complex on device arrays a [6][M][M] (rotated in place), u, adiag.  Up to 128 states all
+// sweeps run in one launch of a cluster; above, one graph of per-step launches a sweep, the
+// sweep's trace change read back after each.
 int jade_dev(int M, double2* a, double2* u, double2* adiag, int maxsweep, double tol, const MlwfWork& w, int* sweeps,
              void* stream) {
   const int np = (M + 1) / 2, steps = 2 * np - 1;

@@ -170,9 +170,9 @@ struct ProjView {
   const int* pc_pt;
   const void* pc_table;
   int* err;               // device error word (a device-side wait gave up)
-  // the fused projection's partial sums: slot (plane_ptr[ix] + local atom) * ysplit + half
-  // holds [LMAX][M]; aslot_ptr / aslot list each atom's slots in plane order
-  double2* slots;         // null: flush with atomics instead
+  // the fused projection's partial sums: slot (plane_ptr[ix] + local atom) * ysplit + share
+  // of the plane holds [LMAX][M]; aslot_ptr / aslot list each atom's slots in plane order
+  double2* slots;         // null: the projections come from their own kernel
   const int* aslot_ptr;
   const int* aslot;
 };

@@ -1,5 +1,5 @@
 // The launcher of the tile kernels (tiles.cuh) for one compiled grid: the shared
-// kernel parameters, the projection finish kernel and launch_h_impl<T, NX, NY, NZ>.
+// kernel parameters and launch_h_impl<T, NX, NY, NZ>.
 // Included by the grid translation units (grids_*.cu), each of which instantiates
 // the plans of a group of grids.
 //

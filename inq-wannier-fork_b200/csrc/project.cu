@@ -11,7 +11,7 @@
 //   mixed   k_project_tc: tcgen05 tensor-core MMAs, kind::tf32, FP32 accumulation in
 //           tensor memory, with a split-precision correction.  A chunk of 32 sphere
 //           points is gathered (cp.async, whole 512-byte orbital rows) into a
-//           staging buffer, four chunks in flight; a pass over shared memory
+//           staging buffer, six chunks in flight; a pass over shared memory
 //           transposes it into the K-major operand and splits each value x into
 //           hi = tf32(x) and lo = tf32(x - hi).  The coefficient table holds the same
 //           split, so hi*hi + hi*lo + lo*hi + lo*lo restores FP32 products.  Each chunk's

@@ -10,7 +10,7 @@
 // 144^3), so the orbital-fastest layout [point][orbital] is read and written in
 // full sectors.
 //
-//   pass A  k_tile_fwd  CTA (group, ix, half of the y1 classes), loops over y1: psi
+//   pass A  k_tile_fwd  CTA (group, ix, share of the y1 classes), loops over y1: psi
 //           rows -> KB projection (plane accumulators in shared memory, flushed
 //           once per CTA) ->
 //           z FFT -> inner y stage -> tmp[g][ka][kz][ix][y1][G]
@@ -18,7 +18,7 @@
 //           outer y stage -> x FFT -> 1/2 |G + k + A|^2 / N -> inverse x ->
 //           inverse outer y stage, in place
 //   pass C  k_tile_inv  CTA (group, ix, y1): inverse inner y stage -> inverse z
-//           -> nonlocal scatter -> alpha (K + V + V_nl) psi + beta base
+//           -> nonlocal scatter -> alpha (K + V + V_nl) psi + beta base - minus
 #pragma once
 
 #include "fft_tile.cuh"
@@ -466,8 +466,8 @@ __device__ __forceinline__ void outer_y_load(typename TG::V* X, const typename T
 // One contiguous block tmp[g][ka][kz] = [ix][y1][G]; in shared memory the x
 // index goes to padded slots of stride XS and (y1, j) stays contiguous.  With
 // fin.slots set, the first CTAs also finish the fused projection (pass C reads it):
-// thread t of CTA b handles item b * blockDim + t, so the few CTAs that carry the
-// finish run beside thousands that do not.
+// four items a warp (proj_finish_item), the warps of the launch in order, so the few CTAs
+// that carry the finish run beside thousands that do not.
 template <typename T, int NX, int NY, int NZ>
 __device__ __forceinline__ void tile_x_body(int bx, int by, typename TileGeom<T, NX, NY, NZ>::V* __restrict__ tmp,
                                             const cplx<T>* __restrict__ tw_x, KinParams<T> kp,
@@ -670,8 +670,9 @@ __global__ void __launch_bounds__(256, TileGeom<T, NX, NY, NZ>::X_MIN_CTAS)
 }
 
 // ---------------------------------------------------------------- pass C
-// The input orbitals of the tile (for V psi) are fetched into shared memory
-// with cp.async at the start, so that read overlaps the inverse transforms.
+// The (ka, kz) runs of the tile come by cp.async; the nonlocal term is added to the
+// transformed tile in shared memory, and the epilogue reads the input orbitals (for V psi)
+// straight from HBM, four lanes a thread in flight.
 // MODE_H = 1: the H epilogue; 0: out = alpha * (inverse transform), the second
 // half of to_real (alpha = 1/N), reading neither orbitals, V nor projectors.
 template <typename T, int NX, int NY, int NZ, int MODE_H>

@@ -7,7 +7,8 @@
 //            (FP64 slabs in FP64; FP32 slabs of 1024 points in the mixed precision)
 //   finish   sum of the slabs, normalisation 1/(|psi_m| |psi_n|), and the six matrices
 //            of tdmlwf_trans::update: cos = (Z + Z^H)/2, sin = (Z - Z^H)/(2i)
-//   jade     one CTA per pair and rotation step: the 18 pair elements, the 3 x 3
+//   jade     per pair and rotation step (up to 128 states: all of them in one cluster; else
+//            one CTA per pair, one launch per step): the 18 pair elements, the 3 x 3
 //            Jacobi eigenproblem, the plane rotation of the pair's rows of the six
 //            matrices and of u, and the step's change of the traces.  The reference
 //            multiplies dense M x M rotation matrices (7 GEMMs per step); the pairs are

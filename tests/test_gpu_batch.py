@@ -35,7 +35,7 @@ def test_batch_matches_cell_by_cell(pb, precision):
     for _ in range(3):  # capture once, replay twice
         batch.apply([c["x"] for c in cells], outs)
     torch.cuda.synchronize()
-    tol = 1e-5 if precision == "mixed" else 1e-12  # atomics in the projector sums reorder roundings
+    tol = 1e-5 if precision == "mixed" else 1e-12  # the graph runs the cells' own kernels
     for a, b in zip(single, outs):
         assert rel_max(b.cpu().numpy(), a.cpu().numpy()) < tol
 

@@ -1,6 +1,7 @@
 """The dense orbital kernels at the edges of their tiles: the overlap and rotation tiles
 (16, 32 and 64 wide), the blocks of 32 of the Cholesky factor and its inverse, and JADE in
-one cluster (rows spread over 16 CTAs, 2 to 6 elements a lane) against numpy and the oracle.
+one cluster (rows spread over 16 CTAs, 2 or 4 elements a lane) and, above 128 states, step by
+step, against numpy and the oracle.
 
 Tolerances: a sum of n rounded FP64 products is within about sqrt(n) 1.1e-16 of its
 2-norm; the factor's condition number (below 10 for these sets) multiplies it once."""
