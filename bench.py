@@ -599,7 +599,7 @@ def run_ours(args):
                                                           "tile_x": pms[2] / pn, "tile_inv": pms[3] / pn}}
         h.set_projection_mode("fused")
     proj_forms["engines"] = {"fused": "CUDA cores inside the first tile pass: FP32 products, FP64 sums per "
-                                      "(plane, half, atom), fixed-order finish in the second pass",
+                                      "(plane, CTA of the plane, atom), fixed-order finish in pass 2",
                              "kernel_mixed": "tcgen05.mma kind::tf32, M=128 N=16, 3xTF32 split, FP64 sums per "
                                              "32-point chunk",
                              "kernel_fp64": "CUDA cores, FP64"}
