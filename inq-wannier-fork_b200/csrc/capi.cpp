@@ -1651,11 +1651,12 @@ int inqb_batch_apply_h(inqb_batch* b, const void* const* psis, void* const* hpsi
   if (!same) {
     b->ready = false;
     b->persistent = false;
-    // workspace, attributes and phases are set up outside the capture
+    // workspace, attributes and phases are set up outside the capture, on the caller's stream:
+    // work queued there may still use the blocks
     for (int i = 0; i < n; i++) {
       INQB_TRY(reserve(b->cells[i], Ms[i]));
       if (!b->cells[i]->proj_phases_valid) {
-        INQB_TRY(update_phases(b->cells[i], nullptr));
+        INQB_TRY(update_phases(b->cells[i], stream));
         b->cells[i]->proj_phases_valid = true;
       }
       // into scratch where the call is in place: the recorded launch below applies H too
@@ -1667,7 +1668,7 @@ int inqb_batch_apply_h(inqb_batch* b, const void* const* psis, void* const* hpsi
         out = b->cells[i]->d_work.ptr;
         ld_out = Ms[i];
       }
-      INQB_TRY(apply(b->cells[i], LaunchArgs::H, psis[i], lds[i], out, ld_out, Ms[i], nullptr, 0, one, zero, nullptr));
+      INQB_TRY(apply(b->cells[i], LaunchArgs::H, psis[i], lds[i], out, ld_out, Ms[i], nullptr, 0, one, zero, stream));
     }
     INQB_CUDA_TRY(cudaDeviceSynchronize());
     batch_release_graph(b);

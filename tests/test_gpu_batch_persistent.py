@@ -187,3 +187,23 @@ def test_batch_in_place(pb, mode):
         ref = [h(x) for (h, _), x in zip(cells, ref)]
         for a, b in zip(blocks, ref):
             assert _rel(a, b) < 1e-13
+
+
+def test_first_call_follows_its_stream(pb):
+    """The first call's set-up applies wait for work that the caller's stream still has queued
+    on the output blocks."""
+    from pinq_b200 import systems
+
+    a = 24 * systems.SPACING
+    h, x = _make(pb, "fp64", systems.cubic(a), (24, 24, 24), np.array([[1.0, 2.0, 3.0]]), 8, 1)
+    ref, out = h(x), torch.full_like(x, 7.0)
+    batch = pb.CellBatch([h])
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(200_000_000)  # about 0.1 s
+        kept = out.clone()
+        batch.apply([x], [out])
+    torch.cuda.synchronize()
+    assert bool((kept == 7.0).all())
+    assert _rel(out, ref) < 1e-13
