@@ -152,7 +152,6 @@ int set_kA(inqb_ctx* ctx, const double kA[3], void* stream) {
   bool same = true;
   for (int d = 0; d < 3; d++) same = same && (ctx->kA_cov[d] == kA[d]);
   for (int d = 0; d < 3; d++) ctx->kA_cov[d] = kA[d];
-  if (!same) ctx->launch_version++;
   if (same && ctx->proj_phases_valid) return INQB_OK;
   INQB_TRY(update_phases(ctx, stream));
   ctx->proj_phases_valid = true;
@@ -544,6 +543,22 @@ void energies_from_sums(const inqb_ctx* ctx, const double s[4], double en[4]) {
 }  // namespace
 }  // namespace inqb
 
+namespace inqb {
+// The state of a cell that its recorded launches hold.
+struct CellState {
+  unsigned long version;
+  std::array<double, 3> kA;
+  int mask, proj_mode;
+  const void* work;
+  explicit CellState(const inqb_ctx* c)
+      : version(c->launch_version), kA{c->kA_cov[0], c->kA_cov[1], c->kA_cov[2]}, mask(c->fourier_mask),
+        proj_mode(c->proj_mode), work(c->d_tmp.ptr) {}
+  bool operator==(const CellState& o) const {
+    return version == o.version && kA == o.kA && mask == o.mask && proj_mode == o.proj_mode && work == o.work;
+  }
+};
+}  // namespace inqb
+
 // A set of independent cells whose H applications run as one CUDA graph: one
 // branch per cell (its three fused kernels), all branches concurrent.
 struct inqb_batch {
@@ -558,8 +573,7 @@ struct inqb_batch {
   std::vector<const void*> psis;
   std::vector<void*> hpsis;
   std::vector<int> Ms, lds;
-  std::vector<unsigned long> versions;
-  std::vector<const void*> works;
+  std::vector<inqb::CellState> states;
   // the persistent launch (batch.h)
   int mode = INQB_BATCH_AUTO;
   int tuned = INQB_BATCH_GRAPH;  // the form AUTO runs: GRAPH until inqb_batch_autotune picks
@@ -836,7 +850,6 @@ int inqb_set_projection_mode(inqb_ctx* ctx, int mode) {
     }
   }
   ctx->proj_mode = mode;
-  ctx->launch_version++;
   return INQB_OK;
 }
 
@@ -953,7 +966,6 @@ int inqb_set_vector_potential(inqb_ctx* ctx, const double kA_cov[3]) {
 int inqb_set_fourier_sphere_mask(inqb_ctx* ctx, int enable) {
   INQB_CHECK_CTX(ctx);
   ctx->fourier_mask = enable ? 1 : 0;
-  ctx->launch_version++;
   return INQB_OK;
 }
 
@@ -1647,7 +1659,7 @@ int inqb_batch_apply_h(inqb_batch* b, const void* const* psis, void* const* hpsi
   bool same = b->ready;
   for (int i = 0; i < n && same; i++)
     same = b->psis[i] == psis[i] && b->hpsis[i] == hpsis[i] && b->Ms[i] == Ms[i] && b->lds[i] == lds[i] &&
-           b->versions[i] == b->cells[i]->launch_version && b->works[i] == b->cells[i]->d_tmp.ptr;
+           b->states[i] == CellState(b->cells[i]);
   if (!same) {
     b->ready = false;
     b->persistent = false;
@@ -1685,12 +1697,8 @@ int inqb_batch_apply_h(inqb_batch* b, const void* const* psis, void* const* hpsi
     b->hpsis.assign(hpsis, hpsis + n);
     b->Ms.assign(Ms, Ms + n);
     b->lds.assign(lds, lds + n);
-    b->versions.clear();
-    b->works.clear();
-    for (const inqb_ctx* c : b->cells) {
-      b->versions.push_back(c->launch_version);
-      b->works.push_back(c->d_tmp.ptr);
-    }
+    b->states.clear();
+    for (const inqb_ctx* c : b->cells) b->states.emplace_back(c);
     b->ready = true;
   }
   if (b->persistent)

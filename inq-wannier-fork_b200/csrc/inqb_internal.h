@@ -192,8 +192,8 @@ struct inqb_ctx {
   double dV = 0.0;
   double kA_cov[3] = {0, 0, 0};
   const inqb::Plan* plan = nullptr;
-  // counts the changes that a recorded launch of this context (a batch's graph or persistent
-  // plan) does not see: k + A, projectors, mask, projection form, schedules
+  // counts the changes of the projector tables and the launch schedules, which a recorded
+  // launch of this context (a batch's graph or persistent plan) does not see
   unsigned long launch_version = 0;
   bool proj_phases_valid = false;  // device phases match kA_cov
   bool proj_table_valid = false;   // the projection kernels' table matches kA_cov
