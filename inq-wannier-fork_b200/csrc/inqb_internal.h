@@ -71,6 +71,13 @@ struct DevBuf {
   P* as() const { return reinterpret_cast<P*>(ptr); }
 };
 
+// A part of a DevBuf.
+struct DevSlice {
+  void* ptr = nullptr;
+  template <typename P>
+  P* as() const { return reinterpret_cast<P*>(ptr); }
+};
+
 // One sphere entry as the H tiles read it: exp(+i (k+A).r), the KB radial values
 // (zero past L) and the point's slot in the tile's shared-memory rows, padded to whole
 // 16-byte vectors so a tile's run of entries is copied with cp.async.
@@ -129,12 +136,13 @@ struct ProjTables {
   DevBuf d_pc_table;                // coefficient table beta exp(+i (k+A).r) for the current k + A
   // each atom's (plane, atom) slots of the fused projection, in plane order
   std::vector<int> aslot_ptr, aslot;
-  DevBuf d_aslot_ptr, d_aslot;
-  DevBuf d_adj_rec, d_atom_pos;     // [nent] AdjRec<T> in atom-major order
-  // device copies
-  DevBuf d_seg_ptr, d_seg_atom, d_seg_ent, d_seg_local, d_plane_ptr;
-  DevBuf d_ent_relpos;              // [nent][3] float
-  DevBuf d_ent_rec;                 // [nent] EntRec<T>, phases filled for each k + A
+  // device copies, in one allocation
+  DevBuf d_tables;
+  DevSlice d_aslot_ptr, d_aslot;
+  DevSlice d_adj_rec, d_atom_pos;   // [nent] AdjRec<T> in atom-major order
+  DevSlice d_seg_ptr, d_seg_atom, d_seg_ent, d_seg_local, d_plane_ptr;
+  DevSlice d_ent_relpos;            // [nent][3] float
+  DevSlice d_ent_rec;               // [nent] EntRec<T>, phases filled for each k + A
   // point order inside each tile: pt_pos[e] is the place of entry e, and
   // pt_ptr[tile * pt_stride + q] the first place of tile-local point q relative to the
   // tile's first entry
@@ -144,10 +152,10 @@ struct ProjTables {
   // that the entries of one rank touch different points.  rk_pos[e] is the place of entry
   // e; tile t's ranks are rk_start[k] .. rk_start[k + 1] for rk_ptr[t] <= k < rk_ptr[t + 1].
   std::vector<int> rk_pos, rk_ptr, rk_start;
-  DevBuf d_ent_rec_rk, d_rk_pos, d_rk_ptr, d_rk_start;
-  DevBuf d_scale;                   // [nproj][L] double
-  DevBuf d_atom_ptr, d_atom_ent, d_ent_pt, d_ent_xyz;
-  DevBuf d_chunk_atom, d_chunk_beg, d_atom_chunk_ptr;
+  DevSlice d_ent_rec_rk, d_rk_pos, d_rk_ptr, d_rk_start;
+  DevSlice d_scale;                 // [nproj][L] double
+  DevSlice d_atom_ptr;
+  DevSlice d_chunk_atom, d_chunk_beg, d_atom_chunk_ptr;
 };
 
 // Kernel view of the projector tables (T = float or double).
